@@ -16,6 +16,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 namespace hphc {
@@ -38,7 +39,11 @@ struct Layout {
 //              S_u = exp(cS d^2 + cW dt)   for dt > 0,
 // with cA = -a^2/2, cB = -b^2/2, cS = -sigma^2/2, cW = -omega.
 struct PairConsts {
-    double cA, cB, cS, cW;                 // natural-log units (FP64 path)
+    double cA, cB, cS, cW;                 // natural-log units (tile decisions, moved events)
+    // The same four in units of 1/32 octave (times 32 log2(e), each the correctly
+    // rounded product to within 2^-100), the argument of the FP64 sweep's
+    // table-driven exponential (exp2_32 in hphc_sweep.cuh).
+    double eA, eB, eS, eW;
     // FP32 path, on records scaled by sX = |a| sqrt(log2(e)/2), sT = |b| sqrt(log2(e)/2):
     // S exponent (log2 units) = kS |dx'|^2 + kW dt' with kS = -sigma^2 / a^2 and
     // kW = -omega log2(e) / sT, each split hi + lo.
@@ -129,7 +134,7 @@ constexpr double kFastTailLog2F64 = 60.0;
 // of the computed exponent (relative ~1e-6) cannot lift above -126.5.  FP64:
 // exp(x) is +0 for x < -745.14; -760 leaves a wide margin.
 constexpr double kSkipF32 = 88.0;
-constexpr double kSkipF64 = 760.0;
+constexpr double kSkipF64 = 710.0;
 
 // Background tail truncation.  Every event's background sum holds its own
 // term, B_ii = 1 unit, the largest of all its terms.  A tile pair whose
@@ -146,6 +151,20 @@ constexpr double kSkipF64 = 760.0;
 // skip only.
 constexpr double kNegligibleLog2 = 91.0;
 constexpr double kNegligibleLog2F32 = 60.0;
+
+// x y 32 log2(e), rounded once: two-product terms carry the rounding errors
+// of x y and of the constant, so the scaled coefficient is as accurate as the
+// unscaled one (its error shifts every pair term the same way).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline double times_32_log2e(double x, double y) {
+    const double kHi = 0x1.71547652b82fep+5, kLo = 0x1.777d0ffda0d24p-51;  // 32 log2(e)
+    const double p = x * y, pe = fma(x, y, -p);
+    const double r = p * kHi;
+    const double re = fma(p, kHi, -r) + (p * kLo + pe * kHi);
+    return r + re;
+}
 
 // The parameter-dependent constants of one problem: every PairConsts field
 // and every FinishConsts field except T and constant (which depend on the
@@ -165,6 +184,10 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     c.cB = -0.5 * b * b;
     c.cS = -0.5 * sigma * sigma;
     c.cW = -omega;
+    c.eA = -0.5 * times_32_log2e(a, a);
+    c.eB = -0.5 * times_32_log2e(b, b);
+    c.eS = -0.5 * times_32_log2e(sigma, sigma);
+    c.eW = -times_32_log2e(omega, 1.0);
     const double recScale = sqrt(0.5 * kLog2eC);  // record scale per unit precision
     const double sX = fabs(a) * recScale, sT = fabs(b) * recScale;
     if (fp32) {
