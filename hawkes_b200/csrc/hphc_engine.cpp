@@ -186,6 +186,46 @@ struct EventSet {
     DevBuf<int32_t> dRanks;
     DevBuf<int> dTileChanges;  // FP32 mode, sorted times: ranks computed on the device
     DevBuf<int32_t> dOrder2, dOrder4;  // FP32 mode: spatial row order of R = 2 and 4 strips
+    bool haveBox = false;              // bounds of the coordinates
+    double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
+
+    // Bounds of the coordinates hLoc, once after each new block of locations;
+    // a moved event only widens them.
+    void update_box(const double* hLoc) {
+        if (haveBox) return;
+        constexpr int W = 8;  // independent running bounds: the loop vectorises
+        double lo[W], hi[W];
+        const size_t n = (size_t)N * D;
+        size_t i = 0;
+        for (int k = 0; k < W; ++k) lo[k] = hi[k] = hLoc[k % D];
+        if (W % D == 0) {
+            for (; i + W <= n; i += W)
+                for (int k = 0; k < W; ++k) {
+                    lo[k] = hLoc[i + k] < lo[k] ? hLoc[i + k] : lo[k];
+                    hi[k] = hLoc[i + k] > hi[k] ? hLoc[i + k] : hi[k];
+                }
+            for (int k = D; k < W; ++k) {
+                lo[k % D] = std::min(lo[k % D], lo[k]);
+                hi[k % D] = std::max(hi[k % D], hi[k]);
+            }
+        }
+        for (; i < n; i += D)
+            for (int k = 0; k < D; ++k) {
+                lo[k] = std::min(lo[k], hLoc[i + k]);
+                hi[k] = std::max(hi[k], hLoc[i + k]);
+            }
+        for (int k = 0; k < D; ++k) {
+            locMin[k] = lo[k];
+            locMax[k] = hi[k];
+        }
+        haveBox = true;
+    }
+    void widen_box(const double* row) {
+        for (int k = 0; k < D; ++k) {
+            locMin[k] = std::min(locMin[k], row[k]);
+            locMax[k] = std::max(locMax[k], row[k]);
+        }
+    }
 
     cudaError_t alloc(int dim, int n, int precision) {
         D = dim;
@@ -318,6 +358,11 @@ struct EventSet {
         v.hTileMin = hTileMin.data();
         v.hTileMax = hTileMax.data();
         v.sorted = sorted;
+        v.haveBox = haveBox;
+        for (int k = 0; k < D; ++k) {
+            v.locMin[k] = locMin[k];
+            v.locMax[k] = locMax[k];
+        }
         return v;
     }
 };
@@ -368,6 +413,11 @@ struct Runtime {
         ex.symmetric = mode.symmetric;
         ex.fastTail = mode.fastTail;
         ex.truncateTail = mode.truncateTail;
+        const bool plainSums = mode.fastTail && mode.truncateTail && mode.underflowSkip &&
+                               (mode.precision == HPHC_PRECISION_FP64 ||
+                                (mode.precision == HPHC_PRECISION_FP32_COMP && mode.variant == 2));
+        ex.gridSums = plainSums && mode.symmetric && mode.precision == HPHC_PRECISION_FP64;
+        ex.selfWindow = plainSums;
         if (st) err = ex.error;
         return st;
     }
@@ -618,6 +668,7 @@ struct hphc_engine {
         if (!moved.empty() || recStale) dirty = true;
         int st = upload_if_dirty();
         if (st) return st;
+        if (rt.ex.selfWindow) set.update_box(hLoc[curLoc].p);
         std::vector<SetView> sets{set.view()};
         std::vector<int> setOf(K, 0);
         // the evaluation keeps problem 0's sums (a self-excitation-only sweep
@@ -672,7 +723,7 @@ struct hphc_engine {
         int st = upload_if_dirty();
         if (st) return st;
         cudaStream_t s = rt.stream;
-        const PairConsts c = rt.ex.pair_consts(p);
+        const PairConsts c = rt.ex.pair_consts(p, set.view());
         cudaError_t e = cudaSuccess;
         for (size_t m = 0; m < moved.size(); ++m) {
             MovedEvent mv{};
@@ -725,12 +776,15 @@ struct hphc_engine {
         rt.ex.sumsOut = dPart;
         rt.ex.shardRank = rank;
         rt.ex.shardWorld = world;
+        const bool gridSums = rt.ex.gridSums;
+        rt.ex.gridSums = false;  // a rank sweeps its share of the pairs
         st = rt.ex.enqueue(sets, &setOf, params, 1, nullptr);
         if (st == HPHC_OK) {
             lastLaunches += rt.ex.lastLaunches;
             hOut.resize(8);
             st = rt.ex.wait(hOut.data());  // its log-likelihood is of a share: not used
         }
+        rt.ex.gridSums = gridSums;
         rt.ex.sumsOut = nullptr;
         rt.ex.shardRank = 0;
         rt.ex.shardWorld = 1;
@@ -840,6 +894,7 @@ int hphc::engine_loop_setup(hphc_engine* e, const double* params, int K, EngineL
     if (!e->moved.empty() || e->recStale) e->dirty = true;
     int st = e->upload_if_dirty();
     if (st) return fmt(*err, st, "%s", e->lastError.c_str());
+    if (e->rt.ex.selfWindow) e->set.update_box(e->hLoc[e->curLoc].p);
     std::vector<SetView> sets{e->set.view()};
     std::vector<int> setOf(K, 0);
     // Chains that all have the kept sums' tauX and tauT (the loop keeps them
@@ -847,7 +902,7 @@ int hphc::engine_loop_setup(hphc_engine* e, const double* params, int K, EngineL
     // the self-excitation terms.  The loop does not write the kept sums.
     e->rt.ex.keptB = e->kept_background_serves(params, K) ? e->dSums.p : nullptr;
     st = e->rt.ex.setup_device_loop(sets, setOf.data(), params, K);
-    out->spec = e->rt.ex.consts_spec();
+    out->spec = e->rt.ex.consts_spec(sets[0], 0.0);
     e->rt.ex.keptB = nullptr;
     if (st) return fmt(*err, st, "%s", e->rt.ex.error.c_str());
     out->device = e->rt.device;
@@ -945,6 +1000,7 @@ int hphc_update_locations(hphc_engine* e, int locationIndex, const double* locat
         if (!copy_checked<false>(location, e->hLocSpare.p, length, &bad, nullptr))
             return e->fail(HPHC_ERR_NONFINITE, "locations: entry %zu is not finite", bad);
         e->hLoc[e->curLoc].swap(e->hLocSpare);
+        e->set.haveBox = false;
         e->invalidate_sums();
         e->dirty = true;
         return HPHC_OK;
@@ -969,6 +1025,7 @@ int hphc_update_locations(hphc_engine* e, int locationIndex, const double* locat
         e->dirty = true;
     }
     std::memcpy(row, location, length * sizeof(double));
+    e->set.widen_box(row);
     return HPHC_OK;
 }
 
@@ -1042,6 +1099,7 @@ int hphc_restore_state(hphc_engine* e) {
     e->sumOfLikContribs = e->storedSumOfLikContribs;
     std::memcpy(e->params, e->storedParams, sizeof e->params);
     e->curLoc = 1 - e->curLoc;
+    e->set.haveBox = false;
     e->dirty = true;
     e->clear_moved();
     if (e->storedSumsValid) {
@@ -1356,6 +1414,8 @@ int hphc_multiset_set_data(hphc_multiset* m, int set, const double* locations, s
         std::memcpy(es.hTimes.p, times, timesLength * sizeof(double));
     }
     es.derive_times(ascending);
+    es.haveBox = false;
+    if (m->rt.ex.selfWindow) es.update_box(m->hLoc[set].p);
     m->ready[set] = 1;
     m->dirty[set] = 1;
     // upload now, overlapping the host work on the next sets

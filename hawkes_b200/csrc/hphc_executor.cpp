@@ -37,6 +37,39 @@ void tile_needs(double tminI, double tmaxI, double tminJ, double tmaxJ, const Pa
     *doS = (dtHi > 0.0) && !(c.skipS >= 0.0 && allCausal && -c.cW * dtLo >= c.skipS);
 }
 
+// The first tile at or after `from` (and before `end`) whose latest time is
+// above v / whose earliest time is at least v, starting from an earlier answer
+// `at`: strips come in time order, so over a plan each edge moves through the
+// tiles once.
+int first_max_above(const SetView& s, double v, int end, int at) {
+    while (at < end && s.hTileMax[at] <= v) ++at;
+    return std::min(at, end);
+}
+int first_min_from(const SetView& s, double v, int from, int end, int at) {
+    at = std::max(at, from);
+    while (at < end && s.hTileMin[at] < v) ++at;
+    return at;
+}
+
+// Time gaps beyond which every background or self-excitation term is left out
+// (+inf: none is, -inf: there are none) and from which background terms take the
+// far tail's exponential.
+struct StripGaps {
+    double b, s, far;
+    explicit StripGaps(const PairConsts& c) {
+        const double kInf = INFINITY;
+        const bool falls = c.cB < 0.0 && c.cA <= 0.0;
+        b = c.noB ? -kInf : c.skipB >= 0.0 && falls ? std::sqrt(c.skipB / -c.cB) : kInf;
+        s = c.skipS >= 0.0 && c.cW < 0.0 && c.cS <= 0.0 ? c.skipS / -c.cW : kInf;
+        far = c.fastB > 0.0 && falls ? std::sqrt(c.fastB / -c.cB) : kInf;
+    }
+};
+
+// Where the edges of the previous strip lay.
+struct StripCursor {
+    int lo = 0, hi = 0, nearLo = 0, nearHi = 0, selfLo = 0;
+};
+
 // Band [*lo, *hi) of j tiles that strip st (r tiles of targets) must visit:
 // every tile that may hold a non-zero term for constants c, plus one tile of
 // margin each side; wide: for any sigma and omega (the device-resident
@@ -44,32 +77,28 @@ void tile_needs(double tminI, double tmaxI, double tminJ, double tmaxJ, const Pa
 // before the strip can hold a background term only if its time gap is below
 // dB = sqrt(skipB / -cB), a self-excitation term only below
 // dS = skipS / -cW (tile_mode's underflow tests solved for the gap), so each
-// edge is one binary search on the bounds.  The band may keep a few tiles
+// edge is a search on the bounds, which moves on from the previous strip's
+// answer: host planning of an N = 100k
+// self-excitation step 90 -> 35 us.  The band may keep a few tiles
 // those tests would drop (tile_mode also tests causality and the space
 // coefficient); the sweep decides every tile itself, and chunks sit on a
 // fixed grid, so a wider band never changes a bit of the result.
-void strip_band(const SetView& s, const PairConsts& c, bool symmetric, bool wide, int r,
-                int nTiles, int st, int* loOut, int* hiOut) {
+void strip_band(const SetView& s, const StripGaps& gap, bool symmetric, bool wide, int r,
+                int nTiles, int st, StripCursor& at, int* loOut, int* hiOut) {
     const int ts0 = st * r, ts1 = std::min(ts0 + r, nTiles);
     *loOut = 0;
     *hiOut = nTiles;
     if (!s.sorted) return;
     const double tminI = s.hTileMin[ts0], tmaxI = s.hTileMax[ts1 - 1];
-    // gap beyond which every term of the kind is exactly zero (+inf: none)
-    const double kInf = INFINITY;
-    const bool anyB = !c.noB;
-    const double dB = !anyB ? -kInf
-                    : (c.skipB >= 0.0 && c.cB < 0.0 && c.cA <= 0.0) ? std::sqrt(c.skipB / -c.cB)
-                                                                      : kInf;
-    const double dS = (c.skipS >= 0.0 && c.cW < 0.0 && c.cS <= 0.0) ? c.skipS / -c.cW : kInf;
+    const double kInf = INFINITY, dB = gap.b, dS = gap.s;
     // left edge: the first tile before the strip whose gap tminI - tmaxJ is
     // below the larger distance (wide: any sigma, omega, so every tile)
     int lo = 0;
     if (!wide) {
         const double d = std::max(dB, dS);
         if (d < kInf) {
-            const double* first = std::upper_bound(s.hTileMax, s.hTileMax + ts0, tminI - d);
-            lo = std::max(0, (int)(first - s.hTileMax) - 1);
+            at.lo = first_max_above(s, tminI - d, ts0, at.lo);
+            lo = std::max(0, at.lo - 1);
         }
     }
     // right edge: with the symmetric sweep, later tiles add this strip's
@@ -81,9 +110,8 @@ void strip_band(const SetView& s, const PairConsts& c, bool symmetric, bool wide
         if (dB == kInf) {
             hi = nTiles;
         } else {
-            const double* first = std::lower_bound(s.hTileMin + ts1, s.hTileMin + nTiles,
-                                                   tmaxI + dB);
-            hi = std::min(nTiles, (int)(first - s.hTileMin) + 1);
+            at.hi = first_min_from(s, tmaxI + dB, ts1, nTiles, at.hi);
+            hi = std::min(nTiles, at.hi + 1);
         }
     } else if (!symmetric && ts1 < nTiles) {
         hi = std::min(nTiles, ts1 + 1);
@@ -118,8 +146,8 @@ struct StripCost {
     double self = kSelfTileCostF32;  // added weight of a tile with self-excitation terms
 };
 
-StripCost strip_cost(const SetView& s, const PairConsts& c, bool fp32, int r, int nTiles,
-                     int st) {
+StripCost strip_cost(const SetView& s, const StripGaps& gap, bool fp32, int r, int nTiles,
+                     int st, StripCursor& at) {
     StripCost k;
     k.self = fp32 ? kSelfTileCostF32 : kSelfTileCostF64;
     const int ts0 = st * r, ts1 = std::min(ts0 + r, nTiles);
@@ -129,16 +157,15 @@ StripCost strip_cost(const SetView& s, const PairConsts& c, bool fp32, int r, in
     k.selfHi = ts1;
     if (!s.sorted) return k;
     const double tminI = s.hTileMin[ts0], tmaxI = s.hTileMax[ts1 - 1];
-    if (c.fastB > 0.0 && c.cB < 0.0 && c.cA <= 0.0) {
-        const double dF = std::sqrt(c.fastB / -c.cB);
-        k.nearLo = (int)(std::upper_bound(s.hTileMax, s.hTileMax + ts0, tminI - dF) - s.hTileMax);
-        k.nearHi = (int)(std::lower_bound(s.hTileMin + ts1, s.hTileMin + nTiles, tmaxI + dF) -
-                         s.hTileMin);
+    if (gap.far < INFINITY) {
+        const double dF = gap.far;
+        k.nearLo = at.nearLo = first_max_above(s, tminI - dF, ts0, at.nearLo);
+        k.nearHi = at.nearHi = first_min_from(s, tmaxI + dF, ts1, nTiles, at.nearHi);
         k.far = fp32 ? kFarTileCostF32 : kFarTileCostF64;
     }
-    if (c.skipS >= 0.0 && c.cW < 0.0 && c.cS <= 0.0) {
-        const double dS = c.skipS / -c.cW;
-        k.selfLo = (int)(std::upper_bound(s.hTileMax, s.hTileMax + ts0, tminI - dS) - s.hTileMax);
+    if (gap.s < INFINITY) {
+        const double dS = gap.s;
+        k.selfLo = at.selfLo = first_max_above(s, tminI - dS, ts0, at.selfLo);
     }
     return k;
 }
@@ -148,6 +175,25 @@ double item_cost(const StripCost& k, bool noB, int jt0, int jt1) {
     const int near = overlap(k.nearLo, k.nearHi);
     const double b = noB ? 0.0 : near + k.far * (jt1 - jt0 - near);
     return b + k.self * overlap(k.selfLo, k.selfHi);
+}
+
+// Writes the items to out (the staged table) largest first, so that the
+// persistent CTAs end on small items; equal costs keep their order.  Costs are
+// sums of whole tiles times weights in tenths, so one counting pass over
+// cost * 10 sorts them.
+void stage_items(const std::vector<WorkItem>& items, const std::vector<double>& cost,
+                 WorkItem* out) {
+    const size_t n = items.size();
+    int top = 0;
+    std::vector<int> key(n);
+    for (size_t k = 0; k < n; ++k) {
+        key[k] = (int)(cost[k] * 10.0 + 0.5);
+        top = std::max(top, key[k]);
+    }
+    std::vector<int> at(top + 2, 0);
+    for (size_t k = 0; k < n; ++k) ++at[top - key[k] + 1];
+    for (int v = 0; v <= top; ++v) at[v + 1] += at[v];
+    for (size_t k = 0; k < n; ++k) out[at[top - key[k]]++] = items[k];
 }
 
 int f32_stride(int D) {
@@ -262,6 +308,18 @@ void append_tune_file(const std::string& device, int sms, const TuneKey& key, in
     std::fclose(f);
 }
 
+// Gridded background sums: cost estimates (plan_grid) and limits.  Microseconds
+// from measured times (one B200): the FP64 sweep's background terms took 6.86 ms
+// for 3.38e9 pairs at N = 100k and 0.25 ms for 1.13e8 at N = 20k; the grid
+// kernels 0.20, 0.28 and 0.56 ms at N = 1,500, 20k and 100k with 1.24e6 nodes,
+// and 0.12 and 0.21 ms at N = 3,000 and 20k with 2.3e5 nodes.
+constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 0.83e-6;  // a pair
+constexpr double kGridCostFixed = 105.0, kGridCostEvent = 3.6e-3, kGridCostNode = 7.0e-5;
+constexpr int kGridMinEvents = 1000;
+constexpr double kGridMaxNodes = 4e8;
+constexpr size_t kGridMaxWork = size_t(8) << 30;    // one problem's workspace
+constexpr size_t kGridGroupWork = size_t(1) << 30;  // of problems that run together
+
 int log2_bucket(double x) {
     int b = 0;
     while (x > 1.0 && b < 80) {
@@ -314,6 +372,11 @@ void Executor::release() {
     if (dOut_) cudaFree(dOut_);
     if (hOut_) cudaFreeHost(hOut_);
     if (dCounter_) cudaFree(dCounter_);
+    if (dGridSums_) cudaFree(dGridSums_);
+    if (dGridWork_) cudaFree(dGridWork_);
+    dGridSums_ = nullptr;
+    dGridWork_ = nullptr;
+    gridSumsCap_ = gridWorkCap_ = 0;
     for (auto& ev : ev_)
         if (ev) cudaEventDestroy(ev);
     dTables_ = hStaging_ = nullptr;
@@ -338,17 +401,52 @@ ConstsSpec Executor::consts_spec() const {
     return s;
 }
 
-PairConsts Executor::pair_consts(const double* p) const {
+// A bound on sum_k e^(-omega (dt_k - d)) over the events k at least d before any
+// one time: at most M events lie in an interval of length 1 / omega (whole
+// tiles), so the sum is at most M (1 + e^-1 + e^-2 + ...) = 1.59 M; 1.7 M
+// also bounds the sum weighted by omega dt / (omega d) for omega d >= 20.
+// omega 0: any omega.
+double decayed_events(const SetView& set, double omega) {
+    if (!set.sorted || !(omega > 0.0)) return set.N;
+    const int nTiles = (set.N + kTile - 1) / kTile;
+    int most = 1;
+    for (int k = 0, j = 0; k < nTiles; ++k) {
+        const double end = set.hTileMax[k] + 1.0 / omega;
+        while (j < nTiles && set.hTileMin[j] <= end) ++j;
+        most = std::max(most, j - k);
+    }
+    return std::min((double)set.N, 1.7 * kTile * most);
+}
+
+// With the event set's self-excitation window, where the sweep has one (omega
+// 0: for any omega).
+ConstsSpec Executor::consts_spec(const SetView& set, double omega) const {
+    ConstsSpec s = consts_spec();
+    if (!selfWindow || fixedR || fixedItems || shardWorld > 1 || !set.haveBox) return s;
+    const int nTiles = (set.N + kTile - 1) / kTile;
+    double volume = set.sorted ? set.hTileMax[nTiles - 1] - set.hTileMin[0]
+                               : *std::max_element(set.hTileMax, set.hTileMax + nTiles) -
+                                     *std::min_element(set.hTileMin, set.hTileMin + nTiles);
+    double ball = 1.0;  // V_D = V_{D-2} 2 pi / D
+    for (int d = D_; d > 1; d -= 2) ball *= 2.0 * M_PI / d;
+    if (D_ % 2) ball *= 2.0;
+    for (int k = 0; k < D_; ++k) volume *= set.locMax[k] - set.locMin[k];
+    s.selfCount = decayed_events(set, omega);
+    s.selfDensity = volume > 0.0 ? set.N / volume * ball / (0.5 * D_ + 1.0) : 1e300;
+    return s;
+}
+
+PairConsts Executor::pair_consts(const double* p, const SetView& set) const {
     PairConsts c{};
     FinishConsts f{};
-    param_consts(p, consts_spec(), c, f);
+    param_consts(p, consts_spec(set, p[3]), c, f);
     return c;
 }
 
 FinishConsts Executor::finish_consts(const double* p, const SetView& set) const {
     PairConsts c{};
     FinishConsts f{};
-    param_consts(p, consts_spec(), c, f);
+    param_consts(p, consts_spec(set, p[3]), c, f);
     f.T = set.hTimes[set.N - 1];
     // src/NewHawkes.hpp:659: locationCount * (embeddingDimension - 1) * log(M_1_SQRT_2PI)
     f.constant = (double)(set.N * (D_ - 1)) * std::log(kInvSqrt2Pi);
@@ -357,8 +455,143 @@ FinishConsts Executor::finish_consts(const double* p, const SetView& set) const 
 
 int Executor::sweep_grid(int r) const {
     const int perSM = sweep_list_blocks_per_sm(precision_ == HPHC_PRECISION_FP64 ? 0 : 1, D_, r,
-                                               variant_);
+                                               sweep_variant());
     return numSMs_ * std::max(1, perSM);
+}
+
+bool Executor::self_only(int P) const {
+    if (keptB) return true;
+    if (gridOf_.empty()) return false;
+    for (int p = 0; p < P; ++p)
+        if (!gridOf_[p]) return false;
+    return true;
+}
+
+// Problem p's gridded background sums: the kept sums' own rows for problem 0
+// where they are kept.
+double* Executor::grid_sums(int p) const {
+    return p == 0 && sumsOut ? sumsOut : dGridSums_ + gridSumsOff_[p];
+}
+
+// Which problems take their background sums from a grid.  The choice depends
+// on the problem alone (not on the others of its batch), so that a batch and
+// single evaluations take the same path: the estimated time of the grid kernels
+// (fixed, per event and per node) against that of the pairs the sweep would
+// evaluate, counted from sampled tiles of sorted times.  A wide grid (sharp
+// kernels over a long span) has too many nodes and stays with the sweep.
+void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                         int P) {
+    gridOf_.clear();
+    if (!gridSums || keptB || fixedR || fixedItems || shardWorld > 1 || D_ > 2) return;
+    const bool fp32 = precision_ != HPHC_PRECISION_FP64;
+    std::vector<char> of(P, 0);
+    std::vector<GridShape> shapes(P);
+    std::vector<size_t> off(P, 0);
+    size_t sums = 0, work = 0;
+    bool any = false;
+    for (int p = 0; p < P; ++p) {
+        const SetView& s = sets[setOf[p]];
+        const double* prm = params + (size_t)6 * p;
+        if (!s.haveBox || s.N < kGridMinEvents || s.N >= (1 << 28)) continue;
+        const PairConsts c = pair_consts(prm, s);
+        const int nTiles = (s.N + kTile - 1) / kTile;
+        // pairs the sweep would evaluate (each once)
+        double pairs = 0.5 * s.N * (double)s.N;
+        double tMin = s.hTileMin[0], tMax = s.hTileMax[nTiles - 1];
+        if (s.sorted && c.skipB >= 0.0 && c.cB < 0.0) {
+            const double d = std::sqrt(c.skipB / -c.cB);
+            const int step = std::max(1, nTiles / 32);
+            double tiles = 0.0;
+            int n = 0;
+            for (int k = 0; k < nTiles; k += step, ++n)
+                tiles += k + 1 - (std::upper_bound(s.hTileMax, s.hTileMax + k + 1,
+                                                   s.hTileMin[k] - d) - s.hTileMax);
+            pairs = std::min(pairs, tiles / n * kTile * s.N);
+        }
+        if (!s.sorted)
+            for (int k = 0; k < nTiles; ++k) {
+                tMin = std::min(tMin, s.hTileMin[k]);
+                tMax = std::max(tMax, s.hTileMax[k]);
+            }
+        const double direct = pairs * (fp32 ? kPairCostF32 : kPairCostF64);
+        const double maxNodes = (direct - kGridCostFixed - s.N * kGridCostEvent) / kGridCostNode;
+        if (!(maxNodes > 0.0)) continue;
+        const double lo[3] = {tMin, D_ == 2 ? s.locMin[1] : 0.0, s.locMin[0]};
+        const double hi[3] = {tMax, D_ == 2 ? s.locMax[1] : 0.0, s.locMax[0]};
+        const GridShape g = grid_shape(prm[1], prm[2], lo, hi, std::min(maxNodes, kGridMaxNodes));
+        if (!g.ok) continue;
+        const size_t need = grid_workspace(g, s.N);
+        if (need > kGridMaxWork) continue;
+        of[p] = 1;
+        shapes[p] = g;
+        off[p] = sums;
+        if (p > 0 || !sumsOut) sums += (size_t)3 * s.N;
+        work = std::max(work, need);
+        any = true;
+    }
+    if (!any) return;
+    // workspace: room for several jobs at once where that is cheap
+    size_t total = 0;
+    for (int p = 0; p < P; ++p)
+        if (of[p]) total += grid_workspace(shapes[p], sets[setOf[p]].N);
+    work = std::max(work, std::min(total, kGridGroupWork));
+    const auto grow = [&](void** ptr, size_t& cap, size_t bytes) {
+        if (bytes <= cap) return true;
+        if (*ptr) cudaFree(*ptr);
+        *ptr = nullptr;
+        cap = 0;
+        if (cudaMalloc(ptr, bytes + bytes / 4) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        cap = bytes + bytes / 4;
+        return true;
+    };
+    // without the memory the pair sweep takes every problem
+    if (!grow(&dGridWork_, gridWorkCap_, work) ||
+        !grow(reinterpret_cast<void**>(&dGridSums_), gridSumsCap_,
+              std::max<size_t>(sums, 1) * sizeof(double)))
+        return;
+    gridOf_.swap(of);
+    gridShape_.swap(shapes);
+    gridSumsOff_.swap(off);
+}
+
+// Enqueue the gridded sums of the planned problems, in groups that fit the
+// workspace.
+int Executor::launch_grid(const std::vector<SetView>& sets, const int* setOf,
+                          const double* params, int P) {
+    if (gridOf_.empty()) return HPHC_OK;
+    cudaError_t e;
+    if (kernelTiming && (e = cudaEventRecord(ev_[4], stream_))) return cuda_fail(e, "timing event");
+    std::vector<GridJob> jobs;
+    size_t used = 0;
+    const auto flush = [&]() {
+        if (jobs.empty()) return cudaSuccess;
+        const cudaError_t err = launch_grid_sums(jobs.data(), (int)jobs.size(), stream_,
+                                                 &gridLaunches_);
+        jobs.clear();
+        used = 0;
+        return err;
+    };
+    for (int p = 0; p < P; ++p) {
+        if (!gridOf_[p]) continue;
+        const SetView& s = sets[setOf[p]];
+        const double* prm = params + (size_t)6 * p;
+        const size_t need = grid_workspace(gridShape_[p], s.N);
+        if (((int)jobs.size() == kGridMaxJobs || used + need > gridWorkCap_) && (e = flush()))
+            return cuda_fail(e, "gridded sums");
+        GridJob j{};
+        j.loc = s.dLoc;
+        j.times = s.dTimes;
+        j.sums = grid_sums(p);
+        grid_job(gridShape_[p], prm[1], prm[2], s.N, D_, static_cast<char*>(dGridWork_) + used, &j);
+        used += need;
+        jobs.push_back(j);
+    }
+    if ((e = flush())) return cuda_fail(e, "gridded sums");
+    if (kernelTiming && (e = cudaEventRecord(ev_[5], stream_))) return cuda_fail(e, "timing event");
+    return HPHC_OK;
 }
 
 int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, const double* params,
@@ -395,19 +628,27 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // strips a problem, for about four items per resident CTA (never coarser
     // than the general grid).  With more strips each band stays one item.
     int selfCT = 0;
-    if (keptB && !wideBands_ && totalStrips < 2.0 * sweep_grid(r)) {
+    selfOnly_ = self_only(P);
+    const auto gridded = [&](int p) { return !gridOf_.empty() && gridOf_[p] != 0; };
+    const auto problem_consts = [&](int p) {
+        PairConsts c = pair_consts(params + (size_t)6 * p, sets[setOf[p]]);
+        if (gridded(p)) c.noB = 1;
+        return c;
+    };
+    if (selfOnly_ && !wideBands_ && totalStrips < 2.0 * sweep_grid(r)) {
         double bandTiles = 0.0;
         for (int p = 0; p < P; ++p) {
             const SetView& s = sets[setOf[p]];
-            const PairConsts c = pair_consts(params + (size_t)6 * p);
+            const StripGaps gap(problem_consts(p));
             const int nTiles = (s.N + kTile - 1) / kTile;
             const int nStrips = (s.N + stripEvents - 1) / stripEvents;
             const int step = std::max(1, nStrips / 16);
             double sampled = 0.0;
             int n = 0;
+            StripCursor at;
             for (int st = 0; st < nStrips; st += step, ++n) {
                 int lo = 0, hi = nTiles;
-                strip_band(s, c, false, false, r, nTiles, st, &lo, &hi);
+                strip_band(s, gap, false, false, r, nTiles, st, at, &lo, &hi);
                 sampled += hi - lo;
             }
             bandTiles += sampled * nStrips / std::max(1, n);
@@ -446,14 +687,14 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         int maxSlots = 1;  // partial-sum slots the widest strip band uses
         pl.maxN = std::max(pl.maxN, N);
         SweepProblem& sp = pl.sp[p];
-        sp.c = pair_consts(prm);
+        sp.c = problem_consts(p);
         sp.N = N;
         sp.nTiles = nTiles;
         sp.Npad = Npad;
         sp.tileMin = s.dTileMin;
         sp.tileMax = s.dTileMax;
         // a self-excitation-only sweep has no background, so no column sums
-        sp.symmetric = (symmetric && !keptB && N <= kMaxSymmetricEvents) ? 1 : 0;
+        sp.symmetric = (symmetric && !sp.c.noB && N <= kMaxSymmetricEvents) ? 1 : 0;
         if (!fp32 && sp.symmetric) {
             // FP64 column sums are fixed point: bound each column total by N
             // times the largest term, B_u <= 1, B_u d^2 <= 1/(e |cA|),
@@ -510,10 +751,12 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
 
         // work items: each strip's band of tiles that may hold a non-zero term
         chunkBase[p] = pl.stripChunks.size();
+        StripCursor at;
+        const StripGaps gap(sp.c);
         for (int st = 0; st < nStrips; ++st) {
             int lo = 0, hi = nTiles;
-            strip_band(s, sp.c, sp.symmetric != 0, wideBands_, r, nTiles, st, &lo, &hi);
-            const StripCost sc = strip_cost(s, sp.c, fp32, r, nTiles, st);
+            strip_band(s, gap, sp.symmetric != 0, wideBands_, r, nTiles, st, at, &lo, &hi);
+            const StripCost sc = strip_cost(s, gap, fp32, r, nTiles, st, at);
             // Chunks sit on a fixed grid of CT tiles per problem, so a tile
             // always lands in the same chunk whatever the band: skipping a
             // band's outside only drops chunks whose sums are exactly zero,
@@ -542,9 +785,14 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         fp.colAcc = nullptr;
         fp.stripChunks = nullptr;
         fp.times = s.dTimes;
+        fp.loc = s.dLoc;
+        fp.tileMin = s.dTileMin;
+        fp.tileMax = s.dTileMax;
+        fp.nTiles = nTiles;
+        fp.sorted = s.sorted ? 1 : 0;
         fp.probs = (p == 0) ? dProbs : nullptr;
         fp.sums = (p == 0) ? sumsOut : nullptr;
-        fp.keptB = keptB;
+        fp.keptB = gridded(p) ? grid_sums(p) : keptB;
         fp.N = N;
         fp.Npad = Npad;
         fp.stripEvents = stripEvents;
@@ -589,17 +837,6 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         for (size_t k = 0; k < nS; ++k)
             if (!owned[k]) pl.stripChunks[k] = 0;
     }
-    // largest first, so that the persistent CTAs end on small items
-    {
-        std::vector<int> order(pl.items.size());
-        for (size_t k = 0; k < order.size(); ++k) order[k] = (int)k;
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int x, int y) { return itemCost[x] > itemCost[y]; });
-        std::vector<WorkItem> sorted(order.size());
-        for (size_t k = 0; k < order.size(); ++k) sorted[k] = pl.items[order[k]];
-        pl.items.swap(sorted);
-    }
-
     // table layout and buffer capacities
     offSP_ = 0;
     offItems_ = align16(offSP_ + sizeof(SweepProblem) * P);
@@ -634,7 +871,7 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     }
     for (auto& j : pl.pj) j.rec = dRecPool_ + reinterpret_cast<size_t>(j.rec);
     std::memcpy(h + offSP_, pl.sp.data(), sizeof(SweepProblem) * P);
-    std::memcpy(h + offItems_, pl.items.data(), sizeof(WorkItem) * nItems);
+    stage_items(pl.items, itemCost, reinterpret_cast<WorkItem*>(h + offItems_));
     const int n = (int)nItems;
     std::memcpy(h + offNItems_, &n, sizeof(int));
     std::memcpy(h + offChunks_, pl.stripChunks.data(), sizeof(int) * pl.stripChunks.size());
@@ -729,7 +966,8 @@ int Executor::launch_sequence(int grid) {
                                          stream_)))
         return cuda_fail(e, "reset column sums");
     if (kernelTiming && (e = record(ev_[1]))) return cuda_fail(e, "timing event");
-    if ((e = launch_sweep_list(prec, D_, R, variant_, grid, sp, items, nItems, dCounter_, stream_)))
+    if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), grid, sp, items, nItems, dCounter_,
+                               stream_)))
         return cuda_fail(e, "sweep kernel");
     if (kernelTiming && (e = record(ev_[2]))) return cuda_fail(e, "timing event");
     if ((e = launch_finish_list(pl.nBlocks, fp, fb, dBlockSums_, stream_)))
@@ -751,7 +989,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
     for (int p = 0; p < P; ++p) pairs += (double)sets[setOf[p]].N * sets[setOf[p]].N;
     pairs /= std::max(1, shardWorld);  // work of this rank
     const int mode = variant_ | (symmetric ? 16 : 0) | (fastTail ? 32 : 0) | (skip_ ? 64 : 0) |
-                     (truncateTail ? 128 : 0);
+                     (truncateTail ? 128 : 0) | (selfOnly_ ? 256 : 0);
     const TuneKey key = std::make_tuple(D_, precision_, mode, log2_bucket(pairs), log2_bucket(P));
     if (deviceName_.empty()) {
         cudaDeviceProp prop{};
@@ -771,7 +1009,6 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
         if (it != gTuneCache.end()) {
             R = fixedR ? fixedR : it->second.first;
             itemsPerSM = fixedItems ? fixedItems : it->second.second;
-            tuned_ = true;
             return HPHC_OK;
         }
     }
@@ -780,6 +1017,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
     else if (precision_ == HPHC_PRECISION_FP64) rs = {1, 2};
     else rs = {2, 4};
     if (fixedItems) its = {fixedItems};
+    else if (selfOnly_) its = {8, 16, 32};  // short sweeps: fewer items to plan and upload
     else its = {8, 16, 32, 64};
     const bool timing = kernelTiming;
     kernelTiming = true;
@@ -831,7 +1069,31 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
     }
     R = bestR;
     itemsPerSM = bestI;
-    tuned_ = true;
+    return HPHC_OK;
+}
+
+// R and itemsPerSM for the current kind of plan: fixed by the caller, or tuned
+// the first time the kind runs.  A self-excitation-only sweep of an engine
+// whose full sweeps are tuned keeps their shape.
+int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
+                           const double* params, int P, double* dProbs) {
+    selfOnly_ = self_only(P);
+    Shape& s = shape_[selfOnly_ ? 1 : 0];
+    if (fixedR && fixedItems) {
+        s.R = fixedR;
+        s.items = fixedItems;
+        s.tuned = true;
+    }
+    if (!s.tuned && shape_[0].tuned) s = shape_[0];
+    if (!s.tuned) {
+        const int st = autotune(sets, setOf, params, P, dProbs);
+        if (st) return st;
+        s.R = R;
+        s.items = itemsPerSM;
+        s.tuned = true;
+    }
+    R = s.R;
+    itemsPerSM = s.items;
     return HPHC_OK;
 }
 
@@ -841,21 +1103,20 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
         error = "no problems to evaluate";
         return HPHC_ERR_BAD_ARGUMENT;
     }
-    if (fixedR && fixedItems) {
-        R = fixedR;
-        itemsPerSM = fixedItems;
-        tuned_ = true;
-    }
-    if (!tuned_) {
-        const int st = autotune(sets, setOf, params, P, dProbs);
-        if (st) return st;
-    }
-    int st = build_plan(sets, setOf, params, P, dProbs, R, itemsPerSM);
+    plan_grid(sets, setOf, params, P);
+    int st = choose_shape(sets, setOf, params, P, dProbs);
+    if (st) return st;
+    // the gridded sums need no plan: the device forms them while the host plans
+    gridLaunches_ = 0;
+    const bool faulty = faultStage == HPHC_FAULT_LAUNCH && faultCount > 0;
+    if (!faulty && (st = launch_grid(sets, setOf, params, P))) return st;
+    st = build_plan(sets, setOf, params, P, dProbs, R, itemsPerSM);
     if (st) return st;
     const int grid = sweep_grid(R);
     timedValid = false;
     if (!useGraph) {
         st = launch_sequence(grid);
+        lastLaunches += gridLaunches_;
         timedValid = kernelTiming && st == HPHC_OK;
         return st;
     }
@@ -870,12 +1131,14 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     key.colNeed = colNeed_;
     key.tables = dTables_;
     key.timing = kernelTiming;
+    key.variant = sweep_variant();
     const bool same = graphExec_ && key.P == graphKey_.P && key.nJobs == graphKey_.nJobs &&
                       key.nBlocks == graphKey_.nBlocks &&
                       key.maxN == graphKey_.maxN && key.R == graphKey_.R &&
                       key.grid == graphKey_.grid && key.tablesBytes == graphKey_.tablesBytes &&
                       key.colNeed == graphKey_.colNeed &&
-                      key.tables == graphKey_.tables && key.timing == graphKey_.timing;
+                      key.tables == graphKey_.tables && key.timing == graphKey_.timing &&
+                      key.variant == graphKey_.variant;
     cudaError_t e;
     if (!same) {
         drop_graph();
@@ -902,7 +1165,7 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     if (take_fault(HPHC_FAULT_LAUNCH))
         return cuda_fail(cudaErrorLaunchOutOfResources, "launch graph (injected)");
     if ((e = cudaGraphLaunch(graphExec_, stream_))) return cuda_fail(e, "launch graph");
-    lastLaunches = (precision_ == HPHC_PRECISION_FP64 ? 3 : 4);
+    lastLaunches = (precision_ == HPHC_PRECISION_FP64 ? 3 : 4) + gridLaunches_;
     timedValid = kernelTiming;
     return HPHC_OK;
 }
@@ -923,6 +1186,15 @@ int Executor::wait(double* hostOut) {
             timedValid = false;
             return cuda_fail(t, "kernel timing");
         }
+        if (!gridOf_.empty()) {  // the gridded sums are part of the sweep and of the step
+            float grid = 0.f;
+            if ((t = cudaEventElapsedTime(&grid, ev_[4], ev_[5])) != cudaSuccess ||
+                (t = cudaEventElapsedTime(&lastStepMs, ev_[4], ev_[3])) != cudaSuccess) {
+                timedValid = false;
+                return cuda_fail(t, "kernel timing");
+            }
+            lastSweepMs += grid;
+        }
     }
     return HPHC_OK;
 }
@@ -933,17 +1205,11 @@ int Executor::setup_device_loop(const std::vector<SetView>& sets, const int* set
         error = "no problems to evaluate";
         return HPHC_ERR_BAD_ARGUMENT;
     }
-    if (fixedR && fixedItems) {
-        R = fixedR;
-        itemsPerSM = fixedItems;
-        tuned_ = true;
-    }
-    if (!tuned_) {
-        const int st = autotune(sets, setOf, params, P, nullptr);
-        if (st) return st;
-    }
+    gridOf_.clear();  // the loop sweeps every term that is not kept
+    int st = choose_shape(sets, setOf, params, P, nullptr);
+    if (st) return st;
     wideBands_ = true;
-    int st = build_plan(sets, setOf, params, P, nullptr, R, itemsPerSM);
+    st = build_plan(sets, setOf, params, P, nullptr, R, itemsPerSM);
     wideBands_ = false;
     if (st) return st;
     drop_graph();  // the tables' layout changed under any captured graph
@@ -979,8 +1245,8 @@ int Executor::enqueue_device_body() {
     if (colNeed_ && (e = cudaMemsetAsync(dColAcc_, 0, colNeed_ * sizeof(unsigned long long),
                                          stream_)))
         return cuda_fail(e, "reset column sums");
-    if ((e = launch_sweep_list(prec, D_, R, variant_, loopGrid_, sp, items, nItems, dCounter_,
-                               stream_)))
+    if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), loopGrid_, sp, items, nItems,
+                               dCounter_, stream_)))
         return cuda_fail(e, "sweep kernel");
     if ((e = launch_finish_list(plan_.nBlocks, fp, fb, dBlockSums_, stream_)))
         return cuda_fail(e, "finish kernel");
@@ -1027,6 +1293,9 @@ void Executor::count_terms(const std::vector<SetView>& sets, double* bTerms, dou
             if (se) ns += ni * nj;
         }
     }
+    // a gridded problem's sums account for every ordered pair, none evaluated
+    for (size_t p = 0; p < gridOf_.size(); ++p)
+        if (gridOf_[p]) nb += (double)plan_.sp[p].N * plan_.sp[p].N;
     *bTerms = nb;
     *sTerms = ns;
     if (bEvals) *bEvals = ne;

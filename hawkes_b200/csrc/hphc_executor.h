@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "hphc_grid.h"
 #include "hphc_kernels.cuh"
 
 namespace hphc {
@@ -41,6 +42,8 @@ struct SetView {
     const double* hTileMin = nullptr;
     const double* hTileMax = nullptr;
     bool sorted = false;               // times ascending (bands are contiguous)
+    bool haveBox = false;              // bounds of the coordinates
+    double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 };
 
 struct RunStats {
@@ -98,6 +101,13 @@ public:
     bool symmetric = false;  // symmetric background sweep (set before the first enqueue)
     bool fastTail = true;    // FP32 polynomial mode: far-tail tile pairs use ex2.approx
     bool truncateTail = true;  // skip background tile pairs below 2^-91 of B_ii (with the skip)
+    // Background sums on a grid (hphc_grid.h) for the problems where that is
+    // estimated to be faster than the pair sweep; the sweep then evaluates only
+    // their self-excitation terms.  Set for the modes whose background terms
+    // need no particular pair arithmetic; a fixed sweep shape or a shard asks
+    // for the pair sweep.
+    bool gridSums = false;
+    bool selfWindow = false;  // self-excitation window (kSelfMisses), checked by the finish
     // Sharded sweep: with shardWorld > 1 the plan keeps only the target
     // strips assigned to shardRank (whole strips, balanced by their tile
     // counts; every rank computes the same assignment), and the finish takes
@@ -129,10 +139,17 @@ private:
     bool skip_ = true;
     bool wideBands_ = false;  // build_plan: bands for any sampled parameters
     int loopGrid_ = 0;        // sweep grid of the device loop
+    bool selfOnly_ = false;   // the current plan's sweep is self-excitation-only
+    int sweep_variant() const { return variant_ | (selfOnly_ ? kSelfOnly : 0); }
     double ex2Bias_ = 0.0;
     std::string deviceName_;  // for the persistent tune cache
     cudaStream_t stream_ = nullptr;
-    bool tuned_ = false;
+    // shapes in use, of sweeps with background terms [0] and of
+    // self-excitation-only sweeps [1]
+    struct Shape {
+        bool tuned = false;
+        int R = 0, items = 0;
+    } shape_[2];
 
     // plan of the last enqueue
     struct Plan {
@@ -163,7 +180,18 @@ private:
     double* hOut_ = nullptr;
     size_t outCap_ = 0;
     int* dCounter_ = nullptr;
-    cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev_[6] = {};  // step start, sweep start and end, step end; grid start and end
+
+    // gridded background sums: which problems of the plan take them, their
+    // grids, the [3][N] sums of those whose sums are not kept, and a workspace
+    std::vector<char> gridOf_;
+    std::vector<GridShape> gridShape_;
+    std::vector<size_t> gridSumsOff_;
+    double* dGridSums_ = nullptr;
+    size_t gridSumsCap_ = 0;
+    void* dGridWork_ = nullptr;
+    size_t gridWorkCap_ = 0;
+    int gridLaunches_ = 0;
 
     // table layout inside dTables_ / hStaging_ (byte offsets)
     size_t offSP_ = 0, offItems_ = 0, offNItems_ = 0, offChunks_ = 0, offFP_ = 0, offFB_ = 0,
@@ -178,12 +206,22 @@ private:
         int P = -1, nJobs = -1, nBlocks = -1, maxN = -1, R = -1, grid = -1;
         size_t tablesBytes = 0, colNeed = 0;
         void* tables = nullptr;
+        int variant = 0;
         bool timing = false;
     } graphKey_;
 
+    ConstsSpec consts_spec() const;
     int build_plan(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,
                    double* dProbs, int r, int items);
     int ensure_buffers();
+    void plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                   int P);
+    double* grid_sums(int p) const;
+    bool self_only(int P) const;  // no problem of the plan has background terms to sweep
+    int choose_shape(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                     int P, double* dProbs);
+    int launch_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                    int P);
     int launch_sequence(int grid);
     int sweep_grid(int r) const;
     int autotune(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,
@@ -194,8 +232,8 @@ private:
     bool capturing_ = false;
 
 public:
-    ConstsSpec consts_spec() const;
-    PairConsts pair_consts(const double* p) const;
+    ConstsSpec consts_spec(const SetView& set, double omega) const;
+    PairConsts pair_consts(const double* p, const SetView& set) const;
     FinishConsts finish_consts(const double* p, const SetView& set) const;
 };
 

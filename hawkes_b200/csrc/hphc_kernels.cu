@@ -464,6 +464,73 @@ final_kernel(int nBlocks, const double* __restrict__ blockSums, FinishConsts f,
     }
 }
 
+// The self-excitation terms of event i that the window left out of its strip's
+// sweep (FinishConsts::skipS instead of fullS), by a whole warp: the tiles are
+// tested as the sweep tests them, and the terms of the tiles between the two
+// thresholds added in tile order.  All of those tiles' events are earlier.
+__device__ __forceinline__ void add_left_out(const FinishProblem& P, const FinishConsts& f, int i,
+                                             double (&s)[kNumAcc]) {
+    const int lane = threadIdx.x & 31;
+    const int t0 = i / P.stripEvents * (P.stripEvents / kTile);
+    const int t1 = min(t0 + P.stripEvents / kTile, P.nTiles);
+    double tmin = INFINITY;
+    for (int t = t0; t < t1; ++t) tmin = fmin(tmin, P.tileMin[t]);
+    const double* xi = P.loc + (size_t)i * f.D;
+    const double ti = P.times[i];
+    double v[3] = {0.0, 0.0, 0.0};
+    // sorted times: the gap falls with the tile number, so the tiles left out
+    // are [first below fullS, first below skipS), each edge by a 32-way search
+    int g0 = 0, g1 = P.nTiles;
+    if (P.sorted) {
+        const auto first_below = [&](double threshold) {
+            int lo = 0, hi = t0;  // gap 0 or less from the strip's own tiles on
+            while (lo < hi) {
+                const int step = (hi - lo + 31) / 32;
+                const int t = lo + lane * step;
+                const bool below = t >= hi || !(-f.cW * (tmin - P.tileMax[t]) >= threshold);
+                const int k = __ffs(__ballot_sync(0xffffffffu, below)) - 1;  // -1: none
+                if (k == 0) break;
+                const int end = k < 0 ? hi : min(hi, lo + k * step);
+                lo += ((k < 0 ? 32 : k) - 1) * step + 1;
+                hi = max(lo, end);
+            }
+            return lo;
+        };
+        g0 = first_below(f.fullS) & ~31;
+        g1 = first_below(f.skipS);
+    }
+    for (int g = g0; g < g1; g += 32) {
+        const double gap = g + lane < P.nTiles ? tmin - P.tileMax[g + lane] : -1.0;
+        const double decay = -f.cW * gap;
+        unsigned left = __ballot_sync(0xffffffffu, gap > 0.0 && decay >= f.skipS &&
+                                                       !(decay >= f.fullS));
+        while (left) {
+            const int t = g + __ffs(left) - 1;
+            left &= left - 1;
+#pragma unroll
+            for (int u = 0; u < kTile; u += 32) {
+                const bool live = t * kTile + u + lane < P.N;
+                const int j = live ? t * kTile + u + lane : i;
+                double d2 = 0.0;
+                for (int k = 0; k < f.D; ++k) {
+                    const double d = xi[k] - P.loc[(size_t)j * f.D + k];
+                    d2 = fma(d, d, d2);
+                }
+                const double dt = ti - P.times[j];
+                const double S = live ? exp(fma(f.cS, d2, f.cW * dt)) : 0.0;
+                v[0] += S;
+                v[1] = fma(S, d2, v[1]);
+                v[2] = fma(S, dt, v[2]);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        for (int d = 16; d > 0; d >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], d);
+        s[3 + q] += v[q];
+    }
+}
+
 // Finish over many problems: CTA b handles events [i0, i0 + kFinishThreads)
 // of problem blocks[b].problem; each event sums its strip's slots in order.
 __global__ void __launch_bounds__(kFinishThreads)
@@ -477,9 +544,11 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
     double v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    double s[kNumAcc];
+#pragma unroll
+    for (int q = 0; q < kNumAcc; ++q) s[q] = 0.0;
     if (i < N) {
         const int nc = P.stripChunks[i / P.stripEvents];
-        double s[kNumAcc];
 #pragma unroll
         for (int q = 0; q < kNumAcc; ++q) {
             if (q < 3 && P.keptB) {
@@ -498,8 +567,24 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
                     acc += (double)P.colAcc[(size_t)q * P.Npad + i] * kColInv;
             }
             s[q] = acc * f.accScale[q];
-            if (P.sums) P.sums[(size_t)q * N + i] = s[q];
         }
+    }
+    // events whose sum does not bound the terms left out (few, see kSelfMisses)
+    unsigned low = __ballot_sync(0xffffffffu, i < N && f.selfLeast > 0.0 && !(s[3] >= f.selfLeast));
+    while (low) {
+        const int src = __ffs(low) - 1;
+        low &= low - 1;
+        double w[kNumAcc] = {};
+        add_left_out(P, f, i - (int)(threadIdx.x & 31) + src, w);
+        if ((int)(threadIdx.x & 31) == src)
+#pragma unroll
+            for (int q = 3; q < kNumAcc; ++q) s[q] += w[q];
+    }
+    if (i < N) {
+        if (P.sums)
+#pragma unroll
+            for (int q = 0; q < kNumAcc; ++q)
+                if (q >= 3 || !P.keptB) P.sums[(size_t)q * N + i] = s[q];
         event_contributions(f, s, P.times[i], v, P.probs ? P.probs + i : nullptr);
     }
     block_sum<8, kFinishThreads>(v);

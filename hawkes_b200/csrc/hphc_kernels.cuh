@@ -87,6 +87,10 @@ struct FinishConsts {
                          // relative error (1 + beta, measured on the device)
     double T;         // t[N-1]
     double constant;  // N (D-1) log(1/sqrt(2 pi))
+    // Self-excitation window (see kSelfWindow...): constants of the sums, the skip
+    // thresholds the sweep applied and applies without the window, and the least
+    // sum that makes the terms left out negligible (0: no window).
+    double cS, cW, skipS, fullS, selfLeast;
     int D;
     int plain32;      // FP32 throughout: the per-event finish in float (the reference's
                       // single precision, src/factory.cpp:45)
@@ -106,6 +110,11 @@ struct ConstsSpec {
     int fastTail;     // far-tail tile pairs use the hardware exponential (FP32 software-
                       // exponential variant, and FP64)
     int noB;          // self-excitation-only sweep (PairConsts::noB)
+    // Self-excitation window, per event set and omega: a bound on
+    // sum_k e^x e^(-omega dt_k) over events k at least x / omega before a time
+    // (0: no window), and the events expected within scaled distance 1 of an
+    // event, N / (T extent) V_D / (D/2 + 1), V_D the unit ball's volume.
+    double selfCount, selfDensity;
 };
 
 // Far background tail of the FP32 software-exponential mode.  A tile pair
@@ -147,10 +156,31 @@ constexpr double kSkipF64 = 710.0;
 // 8760 h span).  FP32 modes: T = 60, so N 2^-60 <= 2^-33 = 1.2e-10 for any
 // N the symmetric sweep holds (2^27), far below their own rounding; the cut
 // falls at |dt| = 9.1 / b = 3070 h, against 13.3 / b for FP32 underflow.
-// The self-excitation sums have no such lower bound and keep the underflow
-// skip only.
 constexpr double kNegligibleLog2 = 91.0;
 constexpr double kNegligibleLog2F32 = 60.0;
+
+// Self-excitation window.  A term decays as exp(-omega dt), and all but a few
+// events have a close earlier neighbour, so of the earlier events within the
+// underflow distance (710 / omega in FP64, 88 / omega in FP32) nearly all add
+// nothing to an event's sum.  There is no term that bounds the sum from below
+// in advance, as B_ii does for the background, so the bound is checked
+// afterwards: the sweep leaves out tile pairs more than x / omega apart, and
+// the finish compares each event's sum with what they could hold, at most
+// M e^-x (M x e^-x for the sum weighted by omega dt), M = selfCount.  If that is
+// not below 2^-60 (FP64) or 2^-36 (FP32-compensated) of the event's own sum, the
+// finish adds the event's terms of those tile pairs one by one, up to the
+// underflow distance.  Every sum thus holds all its terms to 2^-60 or 2^-36
+// of itself, below the rounding of the mode.
+//
+// x = ln M + ln x + 60 ln 2 + E, where E is the exponent of an event's closest
+// earlier neighbour that all but about exp(-kSelfMisses) of the events stay
+// under: the expected number of neighbours with exponent below E, from the mean
+// density of the events, is C(E) = density (2/sigma^2)^(D/2) E^(D/2 + 1) / omega.
+// Without a window (unknown density, a fixed sweep shape, a shard's partial
+// sums, the full-sum flags, the plain FP32 mode) only the underflow skip is
+// left.  Measured at N = 100k (omega = 1 / h): 8.1e8 -> 9.9e7 terms and 1.24 -> 0.18 ms
+// in FP64, 1.30e8 -> 9.0e7 terms and 0.177 -> 0.128 ms in the FP32-compensated mode.
+constexpr double kSelfMisses = 16.0;
 
 // x y 32 log2(e), rounded once: two-product terms carry the rounding errors
 // of x y and of the constant, so the scaled coefficient is as accurate as the
@@ -205,6 +235,28 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
         s.truncate ? fmin(thr, (fp32 ? kNegligibleLog2F32 : kNegligibleLog2) * kLn2) : thr;
     c.skipB = (s.skip && c.cB < 0.0 && c.cA <= 0.0) ? thrB : -1.0;
     c.skipS = (s.skip && c.cW < 0.0 && c.cS <= 0.0) ? thr : -1.0;
+    f.cS = c.cS;
+    f.cW = c.cW;
+    f.skipS = f.fullS = c.skipS;
+    f.selfLeast = 0.0;
+    if (s.selfCount > 0.0 && c.skipS > 0.0 && c.cS < 0.0) {
+        const double root = sqrt(2.0) / fabs(sigma);
+        double perE = s.selfDensity / omega;
+        for (int k = 0; k < s.D; ++k) perE *= root;
+        double E = 1.0;  // in steps of 1/8: products and square roots only
+        for (; E < thr; E *= 1.125) {
+            double count = perE * E;
+            const double r = sqrt(E);
+            for (int k = 0; k < s.D; ++k) count *= r;
+            if (count >= kSelfMisses) break;
+        }
+        // 41.6 = 60 ln 2, 25.0 = 36 ln 2; 6.6 = ln 710
+        const double x = log(s.selfCount) + 6.6 + (fp32 ? 25.0 : 41.6) + E;
+        if (x < 0.7 * thr) {
+            c.skipS = f.skipS = x;
+            f.selfLeast = s.selfCount * x * exp(-x) * (fp32 ? 0x1p36 : 0x1p60);
+        }
+    }
     c.fastB = (s.fastTail && (!fp32 || (s.variant & 2)) && c.cB < 0.0 && c.cA <= 0.0)
                   ? (fp32 ? kFastTailLog2 : kFastTailLog2F64) * kLn2
                   : -1.0;
@@ -392,11 +444,15 @@ struct FinishProblem {
     const double* times;      // the set's raw times
     double* probs;            // P_i output (may be null)
     double* sums;             // [6][N] unit pair sums out, natural units (may be null)
+    // the events, for the terms the self-excitation window left out
+    const double* loc;        // N x D
+    const double* tileMin;
+    const double* tileMax;
     const double* keptB;      // [3][N] background unit sums (natural units) of an earlier
                               // sweep on the same events and tauX, tauT, used instead of
                               // this sweep's (which then has no background terms), or null
     int N, Npad, stripEvents, blockBase;  // blockBase: first finish CTA of this problem
-    int nBlocks, colWords, pad0, pad1;    // colWords: 1 = FP32 column format, 2 = FP64
+    int nBlocks, colWords, nTiles, sorted;  // colWords: 1 = FP32 column format, 2 = FP64
     int colShift[4];
     FinishConsts f;
 };
@@ -417,9 +473,13 @@ struct PackJob {
 
 cudaError_t launch_pack_f32_jobs(int D, int nJobs, int maxN, const PackJob* jobs, cudaStream_t s);
 
+// Variant bit of the sweeps below: every problem of the list has noB set.
+constexpr int kSelfOnly = 32;
+
 // Persistent sweep over a work list: `grid` CTAs take items from *counter
 // (which must be 0 at launch) until *nItems are taken.  precision: 0 = FP64,
-// 1 = FP32-compensated with variant V.
+// 1 = FP32-compensated with variant V; kSelfOnly in V: the
+// self-excitation-only kernels.
 cudaError_t launch_sweep_list(int precision, int D, int R, int V, int grid,
                               const SweepProblem* problems, const WorkItem* items,
                               const int* nItems, int* counter, cudaStream_t s);

@@ -131,7 +131,8 @@ __device__ __forceinline__ double exp_table_lane() { return kExpTable[threadIdx.
 // Results below 2^-1021 are +0 (the smallest normal numbers and the
 // subnormals: at most 4.5e-308), above 2^1024 +inf.  s = -inf gives 0; a NaN
 // exponent comes only from NaN parameters, which make every rate NaN in the
-// finish.
+// finish.  OVER = false: s is known to be below 1024 * 32.
+template <bool OVER>
 __device__ __forceinline__ double exp2_32(double s, double table) {
     constexpr double kRound = 0x1.8p52;  // s + kRound rounds s to an integer in the low word
     const double m = s + kRound;
@@ -144,9 +145,10 @@ __device__ __forceinline__ double exp2_32(double s, double table) {
     q = fma(q, f, kE1);
     const double r = fma(T, q * f, T);
     const int top = __double2hiint(s);
-    int hi = __double2hiint(r) + ((n >> 5) << 20), lo = __double2loint(r);
+    // n >> 5 into the exponent field, which starts at bit 20
+    int hi = __double2hiint(r) + (n & ~31) * (1 << 15), lo = __double2loint(r);
     // s <= -1021 * 32 (as its top word; -inf too), s >= 1024 * 32
-    const bool under = (unsigned)top >= 0xC0DFE800u, over = top >= 0x40E00000;
+    const bool under = (unsigned)top >= 0xC0DFE800u, over = OVER && top >= 0x40E00000;
     hi = under ? 0 : over ? 0x7ff00000 : hi;
     lo = under || over ? 0 : lo;
     return __hiloint2double(hi, lo);
@@ -158,10 +160,10 @@ __device__ __forceinline__ double exp2_32(double s, double table) {
 template <bool FAST>
 __device__ __forceinline__ double background_f64(double s, double table) {
     if (FAST) return (double)ex2_ftz((float)s * 0.03125f);
-    return exp2_32(s, table);
+    return exp2_32<false>(s, table);
 }
 
-template <int D, int R, bool DO_B, bool DO_S, bool MASK, bool FAST = false>
+template <int D, int R, bool DO_B, bool DO_S, bool MASK, bool FAST = false, bool OVER = true>
 __device__ __forceinline__ void body_f64(const double* __restrict__ sRec, int nj,
                                          const double (&xi)[R][D], const double (&ti)[R],
                                          const PairConsts& c, double (&acc)[R][kNumAcc],
@@ -193,7 +195,7 @@ __device__ __forceinline__ void body_f64(const double* __restrict__ sRec, int nj
                 acc[r][2] = fma(B, t2, acc[r][2]);
             }
             if (DO_S) {
-                double Sv = exp2_32(fma(c.eS, d2, c.eW * dt), table);
+                double Sv = exp2_32<OVER>(fma(c.eS, d2, c.eW * dt), table);
                 if (MASK) Sv = dt > 0.0 ? Sv : 0.0;
                 acc[r][3] += Sv;
                 acc[r][4] = fma(Sv, d2, acc[r][4]);
@@ -280,7 +282,7 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
                     cp[2][m] += Bt;
                 }
                 if (DO_S) {
-                    double Sv = exp2_32(fma(c.eS, d2, c.eW * dt), table);
+                    double Sv = exp2_32<true>(fma(c.eS, d2, c.eW * dt), table);
                     if (MASK) Sv = dt > 0.0 ? Sv : 0.0;
                     acc[r][3] += Sv;
                     acc[r][4] = fma(Sv, d2, acc[r][4]);
@@ -345,7 +347,9 @@ __device__ __forceinline__ int first_tile_with_terms(const SweepProblem& P, int 
 // One work item of the FP64 sweep: target strip `strip` (kSweepThreads * R
 // events) against j tiles [jt0, jt1); unit pair sums to partial slot `slot`.
 // sym: tiles before the strip are evaluated once per pair (rows + columns).
-template <int D, int R>
+// SELF: a self-excitation-only sweep (every problem has noB), with the
+// background's code and sums compiled out.
+template <int D, int R, bool SELF = false>
 __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
                                          const double* __restrict__ tileMin,
                                          const double* __restrict__ tileMax,
@@ -389,7 +393,7 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
 
     for (int jt = jt0; jt < jt1; ++jt) {
         TileMode m = tile_mode(tminI, tmaxI, tileMin[jt], tileMax[jt], c);
-        if (sym && jt >= ts1) m.doB = false;  // covered as columns by later strips
+        if (SELF || (sym && jt >= ts1)) m.doB = false;  // sym: as columns by later strips
         if (!m.doB && !m.doS) continue;
         const int j0 = jt * kTile;
         const int nj = min(kTile, N - j0);
@@ -407,7 +411,16 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         // Far-tail tile pairs (every background term at most 2^-60) take them
         // from the FP32 hardware exponential; the choice depends on the
         // background bound alone, and such a pair needs no causality mask.
-        if (sym && m.doB && jt < ts0 && m.fastB) {
+        if (SELF) {
+            // growing kernels (omega < 0) may overflow; terms of pairs that are
+            // not causal may too, but the mask drops them
+            if (c.eW > 0.0)
+                body_f64<D, R, false, true, true>(sRec, nj, xi, ti, c, acc, table);
+            else if (m.allCausal)
+                body_f64<D, R, false, true, false, false, false>(sRec, nj, xi, ti, c, acc, table);
+            else
+                body_f64<D, R, false, true, true, false, false>(sRec, nj, xi, ti, c, acc, table);
+        } else if (sym && m.doB && jt < ts0 && m.fastB) {
             if (!m.doS)
                 tile_sym_f64<D, R, false, false, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad,
                                                        j0, shift, table);
@@ -452,7 +465,7 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
             for (int q = 0; q < kNumAcc; ++q)
                 // a self-excitation-only sweep leaves the background rows to
                 // the kept sums: they are neither written nor read
-                if (q >= 3 || !c.noB) partials[((size_t)slot * kNumAcc + q) * Npad + i] = acc[r][q];
+                if (q >= 3 || (!SELF && !c.noB)) partials[((size_t)slot * kNumAcc + q) * Npad + i] = acc[r][q];
         }
     }
 }
@@ -482,13 +495,16 @@ __device__ __forceinline__ int next_item(int* counter, int* sNext) {
 }
 
 // Work-list form: persistent CTAs take items until the list is exhausted.
-template <int D, int R>
-__global__ void __launch_bounds__(kSweepThreads)
+// The self-excitation-only form needs 96 registers instead of 168 at R = 2, so five
+// CTAs share an SM instead of three: N = 100k self-excitation sweep 1.37 -> 1.24 ms
+// (with the full underflow distance).
+template <int D, int R, bool SELF>
+__global__ void __launch_bounds__(kSweepThreads, (R == 1 ? 4 : 3) + (SELF ? R : 0))
 sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
                       const WorkItem* __restrict__ items, const int* __restrict__ nItems,
                       int* __restrict__ counter) {
     __shared__ __align__(16) double sRec[kTile * Layout<D>::kF64Stride];
-    __shared__ __align__(16) double sCol[(kSweepThreads / 32) * 3 * kTile];
+    __shared__ __align__(16) double sCol[SELF ? 2 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ int sNext;
     const int n = *nItems;
     for (;;) {
@@ -498,7 +514,7 @@ sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         const int shift[3] = {P.colShift[0], P.colShift[1], P.colShift[2]};
-        f64_item<D, R>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
+        f64_item<D, R, SELF>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
                        P.nTiles, P.Npad, c, w.strip, w.start, w.jt1, w.slot, sRec,
                        P.symmetric != 0, P.colAcc, shift, sCol);
     }
@@ -961,7 +977,7 @@ __device__ __forceinline__ void load_record_f32(const float* __restrict__ rec, i
 }
 
 // One work item of the FP32-compensated sweep (see f64_item).
-template <int D, int R, int V>
+template <int D, int R, int V, bool SELF>
 __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
                                           const double* __restrict__ tileMin,
                                           const double* __restrict__ tileMax,
@@ -1018,7 +1034,7 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
         // plain FP32: causal only where the FP32-rounded times differ, so a
         // tile pair with equal rounded bounds keeps the rank mask
         if (V & kPlain) m.allCausal = m.allCausal && (float)tminI > (float)tileMax[jt];
-        if (sym && jt >= ts1) m.doB = false;  // covered as columns by later strips
+        if (SELF || (sym && jt >= ts1)) m.doB = false;  // sym: as columns by later strips
         if (!m.doB && !m.doS) continue;
         const int j0 = jt * kTile;
         const int nj = min(kTile, N - j0);
@@ -1060,7 +1076,12 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
         // no causality mask.
         constexpr int VF = V & ~kPolyExp;         // background exponential of far tiles
         constexpr int VG = V | kTimeHiOnly;        // their geometry: hi parts of the times
-        if (sym && m.doB && jt < ts0) {
+        if (SELF) {
+            if (m.allCausal)
+                tile_f32<D, R, V, V, false, false, true, false>(st, nj, w, c, acc);
+            else
+                tile_f32<D, R, V, V, false, false, true, true>(st, nj, w, c, acc);
+        } else if (sym && m.doB && jt < ts0) {
             // jt < ts0 <= nTiles - 1: a full tile
             if (m.fastB && !m.doS)
                 tile_sym_f32<D, R, VG, VF, true, false, false>(st, w, c, acc, sCol, colAcc, Npad,
@@ -1094,7 +1115,7 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
             else
                 tile_f32<D, R, V, V, false, false, true, true>(st, nj, w, c, acc);
         }
-        if (m.doB && m.fastB) fold_far<R>(acc, c.farScale);
+        if (!SELF && m.doB && m.fastB) fold_far<R>(acc, c.farScale);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -1105,7 +1126,7 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
             for (int q = 0; q < kNumAcc; ++q)
                 // a self-excitation-only sweep leaves the background rows to
                 // the kept sums: they are neither written nor read
-                if (q >= 3 || !c.noB)
+                if (q >= 3 || (!SELF && !c.noB))
                     partials[((size_t)slot * kNumAcc + q) * Npad + i] =
                         (((double)acc.hi[r][q].x - (double)c.rowOffset[q]) +
                          ((double)acc.hi[r][q].y - (double)c.rowOffset[q])) +
@@ -1115,14 +1136,16 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
 }
 
 // R = 2 fits 128 registers (4 CTAs per SM); R = 4 holds twice the rows and
-// column partials and runs 2 CTAs per SM.
-template <int D, int R, int V>
-__global__ void __launch_bounds__(kSweepThreads, (R <= 2 ? 4 : 2))
+// column partials and runs 2 CTAs per SM.  The self-excitation-only form holds
+// half the sums: 96 registers, 5 CTAs per SM at R = 2; N = 100k self-excitation sweep
+// 0.206 -> 0.177 ms (with the full underflow distance).
+template <int D, int R, int V, bool SELF>
+__global__ void __launch_bounds__(kSweepThreads, SELF ? (R <= 2 ? 5 : 3) : (R <= 2 ? 4 : 2))
 sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
                        const WorkItem* __restrict__ items, const int* __restrict__ nItems,
                        int* __restrict__ counter) {
     __shared__ __align__(16) StagedTile<D> sTile;
-    __shared__ __align__(16) float sCol[(kSweepThreads / 32) * 3 * kTile];
+    __shared__ __align__(16) float sCol[SELF ? 4 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ int sNext;
     const int n = *nItems;
     for (;;) {
@@ -1131,9 +1154,40 @@ sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
         const WorkItem w = items[it];
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
-        f32c_item<D, R, V>(static_cast<const float*>(P.rec), P.tileMin, P.tileMax, P.partials,
+        f32c_item<D, R, V, SELF>(static_cast<const float*>(P.rec), P.tileMin, P.tileMax, P.partials,
                            P.colAcc, P.N, P.nTiles, P.Npad, P.symmetric != 0, c, w.strip, w.start,
                            w.jt1, w.slot, P.rowOrder, sTile, sCol);
+    }
+}
+
+template <int D, int R>
+const void* sweep_list_function(int precision, int V) {
+    constexpr int R64 = R > 2 ? 2 : R, R32 = R < 2 ? 2 : R;
+    const bool self = (V & kSelfOnly) != 0;
+    V &= ~kSelfOnly;
+    if (precision == 0) {
+        if (R > 2) return nullptr;
+        return self ? reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, true>)
+                    : reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, false>);
+    }
+    if (R < 2) return nullptr;
+    if (self) {
+        // the self-excitation terms take hi + lo coordinates in every variant
+        // but the plain one
+        if (V & kPlain)
+            return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, kPlain, true>);
+        if (V & kPolyExp)
+            return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, kPolyExp, true>);
+        return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, 0, true>);
+    }
+    switch (V) {
+        case 0: return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, 0, false>);
+        case 1: return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, 1, false>);
+        case 2: return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, 2, false>);
+        case 3: return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, 3, false>);
+        case kPlain:
+            return reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, R32, kPlain, false>);
+        default: return nullptr;
     }
 }
 
@@ -1141,21 +1195,8 @@ template <int D, int R>
 cudaError_t sweep_list_dispatch_v(int precision, int V, int grid, const SweepProblem* problems,
                                   const WorkItem* items, const int* nItems, int* counter,
                                   cudaStream_t s, int* blocksPerSM) {
-    const void* fn = nullptr;
-    if (precision == 0) {
-        if (R > 2) return cudaErrorInvalidValue;
-        fn = reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, (R > 2 ? 2 : R)>);
-    } else {
-        if (R < 2) return cudaErrorInvalidValue;
-        switch (V) {
-            case 0: fn = reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, (R < 2 ? 2 : R), 0>); break;
-            case 1: fn = reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, (R < 2 ? 2 : R), 1>); break;
-            case 2: fn = reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, (R < 2 ? 2 : R), 2>); break;
-            case 3: fn = reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, (R < 2 ? 2 : R), 3>); break;
-            case kPlain: fn = reinterpret_cast<const void*>(&sweep_f32c_list_kernel<D, (R < 2 ? 2 : R), kPlain>); break;
-            default: return cudaErrorInvalidValue;
-        }
-    }
+    const void* fn = sweep_list_function<D, R>(precision, V);
+    if (!fn) return cudaErrorInvalidValue;
     if (blocksPerSM) {
         *blocksPerSM = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, kSweepThreads, 0);
