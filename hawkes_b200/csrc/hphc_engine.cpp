@@ -536,7 +536,8 @@ struct hphc_engine {
     // re-runs only the O(N) finish, instead of the O(N^2) sweep.  storeState
     // keeps a device copy of the sums, which restoreState brings back.
     bool incremental = true;
-    DevBuf<double> dSums, dStoredSums, dRowPartials, dIncBlockSums, dIncOut;
+    DevBuf<double> dSums, dStoredSums, dRowPartials, dIncBlockSums;
+    DevBuf<int> dIncArrived;
     HostBuf<double> hIncOut;
     bool sumsValid = false, storedSumsValid = false, recStale = false;
     double sumsParams[6] = {0, 0, 0, 0, 0, 0}, storedSumsParams[6] = {0, 0, 0, 0, 0, 0};
@@ -598,7 +599,8 @@ struct hphc_engine {
                 (e = dStoredSums.reserve((size_t)kNumAcc * N)) ||
                 (e = dRowPartials.reserve((size_t)kNumAcc * move_event_blocks(N))) ||
                 (e = dIncBlockSums.reserve((size_t)8 * finish_blocks(N))) ||
-                (e = dIncOut.reserve(8)) || (e = hIncOut.reserve(8)))
+                (e = dIncArrived.reserve(1)) || (e = hIncOut.reserve(8)) ||
+                (e = cudaMemset(dIncArrived.p, 0, sizeof(int))))
                 return cuda_status(lastError, e, "device allocation");
             movedSlot.assign(N, -1);
             const int nTiles = (N + kTile - 1) / kTile;
@@ -622,7 +624,7 @@ struct hphc_engine {
         dStoredSums.release();
         dRowPartials.release();
         dIncBlockSums.release();
-        dIncOut.release();
+        dIncArrived.release();
         hIncOut.release();
     }
 
@@ -744,12 +746,10 @@ struct hphc_engine {
         lastIncTerms = (double)moved.size() * (3.0 * N - 2.0);
         clear_moved();
         const FinishConsts f = rt.ex.finish_consts(p, set.view());
-        if ((e = launch_finish_sums(N, dSums.p, set.dTimes.p, f, dIncBlockSums.p,
-                                    probs ? dProbs.p : nullptr, dIncOut.p, s)) ||
-            (e = cudaMemcpyAsync(hIncOut.p, dIncOut.p, 8 * sizeof(double),
-                                 cudaMemcpyDeviceToHost, s)))
+        if ((e = launch_finish_sums(N, dSums.p, set.dTimes.p, f, dIncBlockSums.p, dIncArrived.p,
+                                    probs ? dProbs.p : nullptr, hIncOut.p, s)))
             return cuda_status(lastError, e, "finish from kept sums");
-        lastLaunches += 2;
+        lastLaunches += 1;
         if ((e = cudaStreamSynchronize(s))) return cuda_status(lastError, e, "evaluation");
         if (probs &&
             (e = cudaMemcpy(probs, dProbs.p, (size_t)N * sizeof(double), cudaMemcpyDeviceToHost)))

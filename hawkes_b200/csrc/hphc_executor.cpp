@@ -332,6 +332,7 @@ int log2_bucket(double x) {
 }  // namespace
 
 int Executor::cuda_fail(cudaError_t e, const char* what) {
+    stale_ = true;
     error = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? HPHC_ERR_OUT_OF_MEMORY : HPHC_ERR_CUDA;
 }
@@ -350,6 +351,7 @@ int Executor::init(int D, int precision, int variant, bool underflowSkip, int de
     itemsPerSM = 32;
     cudaError_t e = cudaMalloc(&dCounter_, sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e, "device allocation");
+    stale_ = true;
     for (auto& ev : ev_)
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cuda_fail(e, "create events");
     return HPHC_OK;
@@ -372,6 +374,9 @@ void Executor::release() {
     if (dOut_) cudaFree(dOut_);
     if (hOut_) cudaFreeHost(hOut_);
     if (dCounter_) cudaFree(dCounter_);
+    if (dArrived_) cudaFree(dArrived_);
+    dArrived_ = nullptr;
+    arrivedCap_ = 0;
     if (dGridSums_) cudaFree(dGridSums_);
     if (dGridWork_) cudaFree(dGridWork_);
     dGridSums_ = nullptr;
@@ -903,6 +908,8 @@ int Executor::ensure_buffers() {
         (e = grow_dev(reinterpret_cast<void**>(&dColAcc_), colCap_,
                       std::max<size_t>(colNeed_, 1) * sizeof(unsigned long long))) !=
             cudaSuccess ||
+        (e = grow_dev(reinterpret_cast<void**>(&dArrived_), arrivedCap_,
+                      (size_t)(1 + pl.P) * sizeof(int))) != cudaSuccess ||
         (e = grow_dev(reinterpret_cast<void**>(&dBlockSums_), blockCap_,
                       (size_t)std::max(pl.nBlocks, 1) * 8 * sizeof(double))) != cudaSuccess ||
         (e = grow_dev(&dTables_, tablesCap_, tablesBytes_)) != cudaSuccess)
@@ -928,7 +935,19 @@ int Executor::ensure_buffers() {
         outCap_ = n;
         grew = true;
     }
-    if (grew) drop_graph();
+    if (grew) {
+        drop_graph();
+        stale_ = true;
+    }
+    // the counters and column sums every run leaves at zero: set here when they
+    // are new or an earlier run may not have ended
+    if (stale_) {
+        if ((e = cudaMemsetAsync(dCounter_, 0, sizeof(int), stream_)) ||
+            (e = cudaMemsetAsync(dArrived_, 0, arrivedCap_, stream_)) ||
+            (e = cudaMemsetAsync(dColAcc_, 0, colCap_, stream_)))
+            return cuda_fail(e, "reset counters");
+        stale_ = false;
+    }
     return HPHC_OK;
 }
 
@@ -960,24 +979,16 @@ int Executor::launch_sequence(int grid) {
             return cuda_fail(e, "pack kernel");
         ++launches;
     }
-    if ((e = cudaMemsetAsync(dCounter_, 0, sizeof(int), stream_)))
-        return cuda_fail(e, "reset work counter");
-    if (colNeed_ && (e = cudaMemsetAsync(dColAcc_, 0, colNeed_ * sizeof(unsigned long long),
-                                         stream_)))
-        return cuda_fail(e, "reset column sums");
     if (kernelTiming && (e = record(ev_[1]))) return cuda_fail(e, "timing event");
     if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), grid, sp, items, nItems, dCounter_,
                                stream_)))
         return cuda_fail(e, "sweep kernel");
     if (kernelTiming && (e = record(ev_[2]))) return cuda_fail(e, "timing event");
-    if ((e = launch_finish_list(pl.nBlocks, fp, fb, dBlockSums_, stream_)))
+    // the results go straight to the pinned host buffer
+    if ((e = launch_finish_list(pl.nBlocks, fp, fb, pl.P, dBlockSums_, dArrived_, dCounter_, hOut_,
+                                stream_)))
         return cuda_fail(e, "finish kernel");
-    if ((e = launch_final_list(pl.P, fp, dBlockSums_, dOut_, stream_)))
-        return cuda_fail(e, "final kernel");
-    launches += 3;
-    if ((e = cudaMemcpyAsync(hOut_, dOut_, (size_t)pl.P * 8 * sizeof(double),
-                             cudaMemcpyDeviceToHost, stream_)))
-        return cuda_fail(e, "read results");
+    launches += 2;
     if (kernelTiming && (e = record(ev_[3]))) return cuda_fail(e, "timing event");
     lastLaunches = launches;
     return HPHC_OK;
@@ -1165,7 +1176,7 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     if (take_fault(HPHC_FAULT_LAUNCH))
         return cuda_fail(cudaErrorLaunchOutOfResources, "launch graph (injected)");
     if ((e = cudaGraphLaunch(graphExec_, stream_))) return cuda_fail(e, "launch graph");
-    lastLaunches = (precision_ == HPHC_PRECISION_FP64 ? 3 : 4) + gridLaunches_;
+    lastLaunches = (precision_ == HPHC_PRECISION_FP64 ? 2 : 3) + gridLaunches_;
     timedValid = kernelTiming;
     return HPHC_OK;
 }
@@ -1236,23 +1247,17 @@ int Executor::enqueue_device_body() {
     const auto* fp = reinterpret_cast<const FinishProblem*>(d + offFP_);
     const auto* fb = reinterpret_cast<const FinishBlock*>(d + offFB_);
     cudaError_t e;
-    if ((e = cudaMemsetAsync(dCounter_, 0, sizeof(int), stream_)))
-        return cuda_fail(e, "reset work counter");
     // the plan lists every earlier tile for any sigma and omega: start each
     // item where the current constants allow a term
     if ((e = launch_band_starts((int)plan_.items.size(), sp, items, nItems, R, stream_)))
         return cuda_fail(e, "band kernel");
-    if (colNeed_ && (e = cudaMemsetAsync(dColAcc_, 0, colNeed_ * sizeof(unsigned long long),
-                                         stream_)))
-        return cuda_fail(e, "reset column sums");
     if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), loopGrid_, sp, items, nItems,
                                dCounter_, stream_)))
         return cuda_fail(e, "sweep kernel");
-    if ((e = launch_finish_list(plan_.nBlocks, fp, fb, dBlockSums_, stream_)))
+    if ((e = launch_finish_list(plan_.nBlocks, fp, fb, plan_.P, dBlockSums_, dArrived_, dCounter_,
+                                dOut_, stream_)))
         return cuda_fail(e, "finish kernel");
-    if ((e = launch_final_list(plan_.P, fp, dBlockSums_, dOut_, stream_)))
-        return cuda_fail(e, "final kernel");
-    lastLaunches = 4;
+    lastLaunches = 3;
     return HPHC_OK;
 }
 

@@ -5,10 +5,10 @@
 //   H2D     problem tables, work items, finish tables    one cudaMemcpyAsync from pinned staging
 //   pack    FP32 records scaled per problem (FP32 mode;   pack_f32_jobs_kernel, grid (N, jobs)
 //           one copy per distinct set, tauX, tauT)
+//   grid    background sums of gridded problems           launch_grid_sums (not in the graph)
 //   sweep   persistent CTAs over the work list            sweep_*_list_kernel
-//   finish  per-event contributions, per-CTA sums        finish_list_kernel
-//   final   per-problem fixed-order totals               final_list_kernel
-//   D2H     P x 8 results                                 one cudaMemcpyAsync to pinned memory
+//   finish  per-event contributions, per-CTA sums, and    finish_list_kernel
+//           per-problem totals to pinned host memory
 //
 // The sequence is captured once into a CUDA graph and replayed while buffer
 // capacities and the sweep shape stay the same; only the staged tables change
@@ -180,6 +180,9 @@ private:
     double* hOut_ = nullptr;
     size_t outCap_ = 0;
     int* dCounter_ = nullptr;
+    int* dArrived_ = nullptr;  // finish CTAs arrived: all problems, then each problem
+    size_t arrivedCap_ = 0;
+    bool stale_ = false;  // counters and column sums may not be at zero
     cudaEvent_t ev_[6] = {};  // step start, sweep start and end, step end; grid start and end
 
     // gridded background sums: which problems of the plan take them, their

@@ -467,9 +467,10 @@ final_kernel(int nBlocks, const double* __restrict__ blockSums, FinishConsts f,
 // The self-excitation terms of event i that the window left out of its strip's
 // sweep (FinishConsts::skipS instead of fullS), by a whole warp: the tiles are
 // tested as the sweep tests them, and the terms of the tiles between the two
-// thresholds added in tile order.  All of those tiles' events are earlier.
+// thresholds added in tile order; of those tiles, warp `part` of `parts` takes
+// every parts-th.  All of those tiles' events are earlier.
 __device__ __forceinline__ void add_left_out(const FinishProblem& P, const FinishConsts& f, int i,
-                                             double (&s)[kNumAcc]) {
+                                             int part, int parts, double (&v)[3]) {
     const int lane = threadIdx.x & 31;
     const int t0 = i / P.stripEvents * (P.stripEvents / kTile);
     const int t1 = min(t0 + P.stripEvents / kTile, P.nTiles);
@@ -477,7 +478,7 @@ __device__ __forceinline__ void add_left_out(const FinishProblem& P, const Finis
     for (int t = t0; t < t1; ++t) tmin = fmin(tmin, P.tileMin[t]);
     const double* xi = P.loc + (size_t)i * f.D;
     const double ti = P.times[i];
-    double v[3] = {0.0, 0.0, 0.0};
+    v[0] = v[1] = v[2] = 0.0;
     // sorted times: the gap falls with the tile number, so the tiles left out
     // are [first below fullS, first below skipS), each edge by a 32-way search
     int g0 = 0, g1 = P.nTiles;
@@ -499,6 +500,7 @@ __device__ __forceinline__ void add_left_out(const FinishProblem& P, const Finis
         g0 = first_below(f.fullS) & ~31;
         g1 = first_below(f.skipS);
     }
+    int n = 0;
     for (int g = g0; g < g1; g += 32) {
         const double gap = g + lane < P.nTiles ? tmin - P.tileMax[g + lane] : -1.0;
         const double decay = -f.cW * gap;
@@ -507,6 +509,7 @@ __device__ __forceinline__ void add_left_out(const FinishProblem& P, const Finis
         while (left) {
             const int t = g + __ffs(left) - 1;
             left &= left - 1;
+            if (n++ % parts != part) continue;
 #pragma unroll
             for (int u = 0; u < kTile; u += 32) {
                 const bool live = t * kTile + u + lane < P.N;
@@ -525,17 +528,53 @@ __device__ __forceinline__ void add_left_out(const FinishProblem& P, const Finis
         }
     }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
+    for (int q = 0; q < 3; ++q)
         for (int d = 16; d > 0; d >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], d);
-        s[3 + q] += v[q];
+}
+
+// End of a finish CTA: its sums (thread 0's v) to blockSums[block], and if it is
+// the last of its problem's CTAs [first, first + count) to arrive, the problem's
+// total in CTA order to out[0..7] (which may be pinned host memory), so that no
+// launch and no copy follow.  Returns true on the problem's last CTA's thread 0.
+// *arrived is zero before and after.
+__device__ __forceinline__ bool finish_total(double (&v)[8], double* __restrict__ blockSums,
+                                             int block, int first, int count, int* arrived,
+                                             double constant, double* __restrict__ out) {
+    static_assert(kFinishThreads == kFinalThreads, "the total's order");
+    __shared__ bool sLast;
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) blockSums[(size_t)block * 8 + q] = v[q];
+        __threadfence();
+        sLast = atomicAdd(arrived, 1) == count - 1;
     }
+    __syncthreads();
+    if (!sLast) return false;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    for (int b = threadIdx.x; b < count; b += kFinishThreads)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] += __ldcg(blockSums + (size_t)(first + b) * 8 + q);
+    block_sum<8, kFinishThreads>(v);
+    if (threadIdx.x != 0) return false;
+    out[0] = v[0] + constant;
+#pragma unroll
+    for (int q = 1; q < 7; ++q) out[q] = v[q];
+    out[7] = 0.0;
+    *arrived = 0;
+    return true;
 }
 
 // Finish over many problems: CTA b handles events [i0, i0 + kFinishThreads)
 // of problem blocks[b].problem; each event sums its strip's slots in order.
+// The last problem to end resets the sweep's work counter, and the column sums
+// are zeroed as they are read: the next run's launches find both at zero.
 __global__ void __launch_bounds__(kFinishThreads)
 finish_list_kernel(const FinishProblem* __restrict__ problems,
-                   const FinishBlock* __restrict__ blocks, double* __restrict__ blockSums) {
+                   const FinishBlock* __restrict__ blocks, int nProblems,
+                   double* __restrict__ blockSums, int* __restrict__ arrived,
+                   int* __restrict__ counter, double* __restrict__ out) {
     const FinishBlock fb = blocks[blockIdx.x];
     const FinishProblem& P = problems[fb.problem];
     const FinishConsts f = P.f;
@@ -559,26 +598,60 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
             for (int ch = 0; ch < nc; ++ch)
                 acc += P.partials[((size_t)ch * kNumAcc + q) * P.Npad + i];
             if (q < 3 && P.colAcc) {
-                if (P.colWords == 2)  // FP64 sweep: two-word fixed point
-                    acc += ldexp((double)P.colAcc[(size_t)(2 * q) * P.Npad + i], -P.colShift[q]) +
-                           ldexp((double)P.colAcc[(size_t)(2 * q + 1) * P.Npad + i],
-                                 -(P.colShift[q] + kColLoBits));
-                else
-                    acc += (double)P.colAcc[(size_t)q * P.Npad + i] * kColInv;
+                if (P.colWords == 2) {  // FP64 sweep: two-word fixed point
+                    unsigned long long* hi = P.colAcc + (size_t)(2 * q) * P.Npad + i;
+                    unsigned long long* lo = hi + P.Npad;
+                    acc += ldexp((double)*hi, -P.colShift[q]) +
+                           ldexp((double)*lo, -(P.colShift[q] + kColLoBits));
+                    *hi = *lo = 0;
+                } else {
+                    unsigned long long* w = P.colAcc + (size_t)q * P.Npad + i;
+                    acc += (double)*w * kColInv;
+                    *w = 0;
+                }
             }
             s[q] = acc * f.accScale[q];
         }
     }
-    // events whose sum does not bound the terms left out (few, see kSelfMisses)
-    unsigned low = __ballot_sync(0xffffffffu, i < N && f.selfLeast > 0.0 && !(s[3] >= f.selfLeast));
-    while (low) {
-        const int src = __ffs(low) - 1;
-        low &= low - 1;
-        double w[kNumAcc] = {};
-        add_left_out(P, f, i - (int)(threadIdx.x & 31) + src, w);
-        if ((int)(threadIdx.x & 31) == src)
-#pragma unroll
-            for (int q = 3; q < kNumAcc; ++q) s[q] += w[q];
+    // Events whose sum does not bound the terms left out of it (few, see
+    // kSelfMisses) are listed; the CTA's warps take one each, or share the
+    // tiles of each where there are fewer events than warps.
+    constexpr int kWarps = kFinishThreads / 32;
+    __shared__ int sLow[kFinishThreads], sLows;
+    __shared__ double sAdd[kFinishThreads][3];
+    if (f.selfLeast > 0.0) {
+        bool low = i < N && !(s[3] >= f.selfLeast);
+        if (low && P.sorted)  // sorted times: nothing is left out if the first tile is not
+            low = -f.cW * (P.tileMin[i / P.stripEvents * (P.stripEvents / kTile)] -
+                           P.tileMax[0]) >= f.skipS;
+        if (threadIdx.x == 0) sLows = 0;
+        __syncthreads();
+        if (low) sLow[atomicAdd(&sLows, 1)] = threadIdx.x;
+        __syncthreads();
+        const int warp = threadIdx.x >> 5, lows = sLows;
+        const int parts = lows < kWarps ? kWarps : 1;
+        for (int k = parts == 1 ? warp : 0; k < lows; k += parts == 1 ? kWarps : 1) {
+            double w[3];
+            add_left_out(P, f, fb.i0 + sLow[k], parts == 1 ? 0 : warp, parts, w);
+            if (parts == 1) {
+                if ((threadIdx.x & 31) == 0)
+                    for (int q = 0; q < 3; ++q) sAdd[sLow[k]][q] = w[q];
+                continue;
+            }
+            __shared__ double sPart[kWarps][3];
+            if ((threadIdx.x & 31) == 0)
+                for (int q = 0; q < 3; ++q) sPart[warp][q] = w[q];
+            __syncthreads();
+            if (threadIdx.x < 3) {
+                double sum = 0.0;
+                for (int u = 0; u < kWarps; ++u) sum += sPart[u][threadIdx.x];
+                sAdd[sLow[k]][threadIdx.x] = sum;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        if (low)
+            for (int q = 0; q < 3; ++q) s[3 + q] += sAdd[threadIdx.x][q];
     }
     if (i < N) {
         if (P.sums)
@@ -588,30 +661,13 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
         event_contributions(f, s, P.times[i], v, P.probs ? P.probs + i : nullptr);
     }
     block_sum<8, kFinishThreads>(v);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) blockSums[(size_t)blockIdx.x * 8 + q] = v[q];
-    }
-}
-
-// One CTA per problem: fixed-order sum of its finish CTAs' sums.
-__global__ void __launch_bounds__(kFinalThreads)
-final_list_kernel(const FinishProblem* __restrict__ problems, const double* __restrict__ blockSums,
-                  double* __restrict__ out) {
-    const FinishProblem& P = problems[blockIdx.x];
-    double v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = 0.0;
-    for (int b = threadIdx.x; b < P.nBlocks; b += kFinalThreads)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] += blockSums[(size_t)(P.blockBase + b) * 8 + q];
-    block_sum<8, kFinalThreads>(v);
-    if (threadIdx.x == 0) {
-        double* o = out + (size_t)blockIdx.x * 8;
-        o[0] = v[0] + P.f.constant;
-#pragma unroll
-        for (int q = 1; q < 7; ++q) o[q] = v[q];
-        o[7] = 0.0;
+    if (finish_total(v, blockSums, blockIdx.x, P.blockBase, P.nBlocks, arrived + 1 + fb.problem,
+                     f.constant, out + (size_t)fb.problem * 8)) {
+        __threadfence();
+        if (atomicAdd(arrived, 1) == nProblems - 1) {
+            *arrived = 0;
+            *counter = 0;
+        }
     }
 }
 
@@ -693,7 +749,8 @@ move_event_row_kernel(int N, int k, int nBlocks, const double* __restrict__ rowP
 
 __global__ void __launch_bounds__(kFinishThreads)
 finish_sums_kernel(int N, const double* __restrict__ sums, const double* __restrict__ times,
-                   FinishConsts f, double* __restrict__ blockSums, double* __restrict__ probs) {
+                   FinishConsts f, double* __restrict__ blockSums, int* __restrict__ arrived,
+                   double* __restrict__ probs, double* __restrict__ out) {
     const int i = blockIdx.x * kFinishThreads + threadIdx.x;
     double v[8];
 #pragma unroll
@@ -705,10 +762,7 @@ finish_sums_kernel(int N, const double* __restrict__ sums, const double* __restr
         event_contributions(f, s, times[i], v, probs ? probs + i : nullptr);
     }
     block_sum<8, kFinishThreads>(v);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) blockSums[(size_t)blockIdx.x * 8 + q] = v[q];
-    }
+    finish_total(v, blockSums, blockIdx.x, 0, gridDim.x, arrived, f.constant, out);
 }
 
 }  // namespace
@@ -830,17 +884,12 @@ cudaError_t launch_band_starts(int maxItems, const SweepProblem* problems, WorkI
 }
 
 cudaError_t launch_finish_list(int nBlocks, const FinishProblem* problems,
-                               const FinishBlock* blocks, double* blockSums, cudaStream_t s) {
-    finish_list_kernel<<<nBlocks, kFinishThreads, 0, s>>>(problems, blocks, blockSums);
+                               const FinishBlock* blocks, int nProblems, double* blockSums,
+                               int* arrived, int* counter, double* out, cudaStream_t s) {
+    finish_list_kernel<<<nBlocks, kFinishThreads, 0, s>>>(problems, blocks, nProblems, blockSums,
+                                                          arrived, counter, out);
     return cudaGetLastError();
 }
-
-cudaError_t launch_final_list(int nProblems, const FinishProblem* problems,
-                              const double* blockSums, double* out, cudaStream_t s) {
-    final_list_kernel<<<nProblems, kFinalThreads, 0, s>>>(problems, blockSums, out);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_finish(const SweepGeometry& g, const double* partials, const double* times,
                           const FinishConsts& f, double* blockSums, double* probs,
                           cudaStream_t s) {
@@ -895,11 +944,10 @@ cudaError_t launch_move_event_row(int N, int k, const double* rowPartials, doubl
 }
 
 cudaError_t launch_finish_sums(int N, const double* sums, const double* times,
-                               const FinishConsts& f, double* blockSums, double* probs,
-                               double* out, cudaStream_t s) {
+                               const FinishConsts& f, double* blockSums, int* arrived,
+                               double* probs, double* out, cudaStream_t s) {
     finish_sums_kernel<<<finish_blocks(N), kFinishThreads, 0, s>>>(N, sums, times, f, blockSums,
-                                                                   probs);
-    final_kernel<<<1, kFinalThreads, 0, s>>>(finish_blocks(N), blockSums, f, out);
+                                                                   arrived, probs, out);
     return cudaGetLastError();
 }
 

@@ -439,7 +439,8 @@ cudaError_t launch_band_starts(int maxItems, const SweepProblem* problems, WorkI
 // Finish view of a problem.
 struct FinishProblem {
     const double* partials;   // [slot][6][Npad]
-    const unsigned long long* colAcc;  // [3][Npad] symmetric-sweep column sums, or null
+    unsigned long long* colAcc;  // [3][Npad] symmetric-sweep column sums, or null; zeroed once
+                                 // read
     const int* stripChunks;   // slots used by each strip
     const double* times;      // the set's raw times
     double* probs;            // P_i output (may be null)
@@ -487,12 +488,12 @@ cudaError_t launch_sweep_list(int precision, int D, int R, int V, int grid,
 // Resident CTAs per SM of that sweep kernel (0 if the configuration is invalid).
 int sweep_list_blocks_per_sm(int precision, int D, int R, int V);
 
+// arrived: 1 + nProblems counters, zero between runs; counter: the sweep's work
+// counter, reset; out[8p .. 8p+7] for every problem p: log-likelihood, gradient, 0
+// (device or pinned host memory).
 cudaError_t launch_finish_list(int nBlocks, const FinishProblem* problems,
-                               const FinishBlock* blocks, double* blockSums, cudaStream_t s);
-
-// out[8p .. 8p+7] for every problem p: log-likelihood, gradient, 0.
-cudaError_t launch_final_list(int nProblems, const FinishProblem* problems,
-                              const double* blockSums, double* out, cudaStream_t s);
+                               const FinishBlock* blocks, int nProblems, double* blockSums,
+                               int* arrived, int* counter, double* out, cudaStream_t s);
 
 // ---- incremental evaluation ------------------------------------------------
 //
@@ -519,10 +520,11 @@ cudaError_t launch_move_event(int D, int N, const MovedEvent& m, const double* l
 cudaError_t launch_move_event_row(int N, int k, const double* rowPartials, double* sums,
                                   cudaStream_t s);
 // Per-event finish from kept sums (natural units) and the fixed-order total:
-// out[0] = log-likelihood, out[1..6] = gradient, out[7] = 0; probs may be null.
+// out[0] = log-likelihood, out[1..6] = gradient, out[7] = 0 (device or pinned
+// host memory); probs may be null.  *arrived is zero between runs.
 cudaError_t launch_finish_sums(int N, const double* sums, const double* times,
-                               const FinishConsts& f, double* blockSums, double* probs,
-                               double* out, cudaStream_t s);
+                               const FinishConsts& f, double* blockSums, int* arrived,
+                               double* probs, double* out, cudaStream_t s);
 // CTAs of launch_move_event for N events.
 int move_event_blocks(int N);
 
