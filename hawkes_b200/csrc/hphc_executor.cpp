@@ -432,6 +432,7 @@ ConstsSpec Executor::consts_spec(const SetView& set, double omega) const {
     double volume = set.sorted ? set.hTileMax[nTiles - 1] - set.hTileMin[0]
                                : *std::max_element(set.hTileMax, set.hTileMax + nTiles) -
                                      *std::min_element(set.hTileMin, set.hTileMin + nTiles);
+    s.selfTile = volume / nTiles;
     double ball = 1.0;  // V_D = V_{D-2} 2 pi / D
     for (int d = D_; d > 1; d -= 2) ball *= 2.0 * M_PI / d;
     if (D_ % 2) ball *= 2.0;
@@ -625,44 +626,47 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     const int target = numSMs_ * items * std::max(1, shardWorld);
     const int nChunksTarget = std::max(1, (int)std::ceil(target / std::max(1.0, totalStrips)));
 
-    // A self-excitation-only sweep (kept background sums, host-planned bands)
-    // visits a few tiles near each strip.  With fewer strips than two per
-    // resident CTA (one problem, say), the general grid leaves about one wave
-    // of items, where the few left over double the sweep's time: the bands
-    // are then cut on a grid set from their total, estimated from up to 16
-    // strips a problem, for about four items per resident CTA (never coarser
-    // than the general grid).  With more strips each band stays one item.
-    int selfCT = 0;
-    selfOnly_ = self_only(P);
     const auto gridded = [&](int p) { return !gridOf_.empty() && gridOf_[p] != 0; };
     const auto problem_consts = [&](int p) {
         PairConsts c = pair_consts(params + (size_t)6 * p, sets[setOf[p]]);
         if (gridded(p)) c.noB = 1;
         return c;
     };
-    if (selfOnly_ && !wideBands_ && totalStrips < 2.0 * sweep_grid(r)) {
-        double bandTiles = 0.0;
-        for (int p = 0; p < P; ++p) {
+    // A self-excitation-only sweep (kept or gridded background sums) visits a few
+    // tiles before each strip.  Problems of one size with sorted times need no
+    // work list for that: every strip gets the same number of slots, enough for
+    // the widest band (the device loop: for every earlier tile), and an item's
+    // tiles follow from its number (SweepProblem::itemsPerProblem).  A slot holds
+    // the tiles that make about four items per resident CTA, at most a whole band.
+    selfOnly_ = self_only(P);
+    int selfSlots = 0, selfTiles = 1;
+    // A device loop over more than kLoopTiles tiles keeps its list: its bands may
+    // come to hold every earlier tile, and then largest first counts (16 chains
+    // at N = 10,000: 0.86 ms an iteration without, 0.64 with).
+    constexpr int kLoopTiles = 32;
+    bool listless = selfOnly_ && shardWorld == 1 &&
+                    !(wideBands_ && sets[setOf[0]].N > kLoopTiles * kTile);
+    for (int p = 0; p < P && listless; ++p)
+        listless = sets[setOf[p]].sorted && sets[setOf[p]].N == sets[setOf[0]].N;
+    if (listless) {
+        const int nTiles = (sets[setOf[0]].N + kTile - 1) / kTile;
+        const int nStrips = (sets[setOf[0]].N + stripEvents - 1) / stripEvents;
+        int widest = wideBands_ ? nTiles : 1;
+        double bandTiles = wideBands_ ? (double)P * nStrips * nTiles : 0.0;
+        for (int p = 0; p < P && !wideBands_; ++p) {
             const SetView& s = sets[setOf[p]];
             const StripGaps gap(problem_consts(p));
-            const int nTiles = (s.N + kTile - 1) / kTile;
-            const int nStrips = (s.N + stripEvents - 1) / stripEvents;
-            const int step = std::max(1, nStrips / 16);
-            double sampled = 0.0;
-            int n = 0;
             StripCursor at;
-            for (int st = 0; st < nStrips; st += step, ++n) {
+            for (int st = 0; st < nStrips; ++st) {
                 int lo = 0, hi = nTiles;
-                strip_band(s, gap, false, false, r, nTiles, st, at, &lo, &hi);
-                sampled += hi - lo;
+                strip_band(s, gap, true, false, r, nTiles, st, at, &lo, &hi);
+                widest = std::max(widest, hi - lo);
+                bandTiles += hi - lo;
             }
-            bandTiles += sampled * nStrips / std::max(1, n);
         }
-        // a power of two near it, so that small changes of the bands (a
-        // sampler's steps in omega) keep the grid, the list's capacity and
-        // the captured graph
-        const double want = std::max(1.0, bandTiles / (4.0 * sweep_grid(r)));
-        selfCT = 1 << (int)std::lround(std::log2(want));
+        selfTiles = std::min(widest, std::max(1, (int)std::lround(bandTiles /
+                                                                  (4.0 * sweep_grid(r)))));
+        selfSlots = (widest + selfTiles - 1) / selfTiles;
     }
 
     size_t recOff = 0, partOff = 0, colOff = 0;
@@ -685,10 +689,9 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         const int nTiles = (N + kTile - 1) / kTile;
         const int nStrips = (N + stripEvents - 1) / stripEvents;
         const int Npad = nStrips * stripEvents;
-        // tiles a chunk (a self-excitation-only grid never coarser than the
-        // general one, which follows the tuned items per SM)
+        // tiles a chunk, from the tuned items per SM
         const int generalCT = std::max(1, (nTiles + nChunksTarget - 1) / nChunksTarget);
-        const int CT = selfCT > 0 ? std::min(selfCT, generalCT) : generalCT;
+        const int CT = generalCT;
         int maxSlots = 1;  // partial-sum slots the widest strip band uses
         pl.maxN = std::max(pl.maxN, N);
         SweepProblem& sp = pl.sp[p];
@@ -756,9 +759,15 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
 
         // work items: each strip's band of tiles that may hold a non-zero term
         chunkBase[p] = pl.stripChunks.size();
+        if (listless) {
+            maxSlots = selfSlots;
+            sp.itemsPerProblem = nStrips * selfSlots;
+            sp.slots = selfSlots;
+            sp.chunkTiles = selfTiles;
+        }
         StripCursor at;
         const StripGaps gap(sp.c);
-        for (int st = 0; st < nStrips; ++st) {
+        for (int st = 0; st < nStrips && !listless; ++st) {
             int lo = 0, hi = nTiles;
             strip_band(s, gap, sp.symmetric != 0, wideBands_, r, nTiles, st, at, &lo, &hi);
             const StripCost sc = strip_cost(s, gap, fp32, r, nTiles, st, at);
@@ -845,8 +854,8 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // table layout and buffer capacities
     offSP_ = 0;
     offItems_ = align16(offSP_ + sizeof(SweepProblem) * P);
-    const size_t nItems = pl.items.size();
-    itemsCap_ = std::max(itemsCap_, nItems);
+    const size_t nItems = listless ? (size_t)P * pl.sp[0].itemsPerProblem : pl.items.size();
+    itemsCap_ = std::max(itemsCap_, pl.items.size());
     offNItems_ = align16(offItems_ + sizeof(WorkItem) * itemsCap_);
     offChunks_ = align16(offNItems_ + sizeof(int));
     offFP_ = align16(offChunks_ + sizeof(int) * pl.stripChunks.size());
@@ -872,14 +881,17 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         FinishProblem& fp = pl.fp[p];
         fp.partials = sp.partials;
         fp.colAcc = sp.colAcc;
-        fp.stripChunks = reinterpret_cast<const int*>(d + offChunks_) + chunkBase[p];
+        fp.stripChunks =
+            listless ? nullptr : reinterpret_cast<const int*>(d + offChunks_) + chunkBase[p];
+        fp.slots = selfSlots;
     }
     for (auto& j : pl.pj) j.rec = dRecPool_ + reinterpret_cast<size_t>(j.rec);
     std::memcpy(h + offSP_, pl.sp.data(), sizeof(SweepProblem) * P);
     stage_items(pl.items, itemCost, reinterpret_cast<WorkItem*>(h + offItems_));
     const int n = (int)nItems;
     std::memcpy(h + offNItems_, &n, sizeof(int));
-    std::memcpy(h + offChunks_, pl.stripChunks.data(), sizeof(int) * pl.stripChunks.size());
+    if (!pl.stripChunks.empty())
+        std::memcpy(h + offChunks_, pl.stripChunks.data(), sizeof(int) * pl.stripChunks.size());
     std::memcpy(h + offFP_, pl.fp.data(), sizeof(FinishProblem) * P);
     std::memcpy(h + offFB_, pl.fb.data(), sizeof(FinishBlock) * pl.fb.size());
     if (!pl.pj.empty()) std::memcpy(h + offPJ_, pl.pj.data(), sizeof(PackJob) * pl.pj.size());
@@ -1040,6 +1052,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
             R = r;
             itemsPerSM = it;
             if ((st = build_plan(sets, setOf, params, P, dProbs, r, it))) break;
+            if (plan_.sp[0].itemsPerProblem > 0 && it != its[0]) continue;  // no list: no choice
             const int grid = sweep_grid(r);
             // median of four sweeps after one that warms the caches: the
             // shapes' typical times differ by ~1 %, about as much as the
@@ -1095,7 +1108,11 @@ int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
         s.items = fixedItems;
         s.tuned = true;
     }
-    if (!s.tuned && shape_[0].tuned) s = shape_[0];
+    if (!s.tuned && shape_[0].tuned) {
+        s = shape_[0];
+        // a few thousand events: more, smaller strips fill the SMs
+        if (selfOnly_ && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
+    }
     if (!s.tuned) {
         const int st = autotune(sets, setOf, params, P, dProbs);
         if (st) return st;
@@ -1247,9 +1264,11 @@ int Executor::enqueue_device_body() {
     const auto* fp = reinterpret_cast<const FinishProblem*>(d + offFP_);
     const auto* fb = reinterpret_cast<const FinishBlock*>(d + offFB_);
     cudaError_t e;
-    // the plan lists every earlier tile for any sigma and omega: start each
-    // item where the current constants allow a term
-    if ((e = launch_band_starts((int)plan_.items.size(), sp, items, nItems, R, stream_)))
+    // a listed plan holds every earlier tile for any sigma and omega: start each
+    // item where the current constants allow a term (the sweep of a plan without
+    // a list finds that itself)
+    if (!plan_.items.empty() &&
+        (e = launch_band_starts((int)plan_.items.size(), sp, items, nItems, R, stream_)))
         return cuda_fail(e, "band kernel");
     if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), loopGrid_, sp, items, nItems,
                                dCounter_, stream_)))
@@ -1273,7 +1292,20 @@ void Executor::count_terms(const std::vector<SetView>& sets, double* bTerms, dou
                            double* bEvals) const {
     double nb = 0.0, ns = 0.0, ne = 0.0;
     const int stripEvents = kSweepThreads * R;
-    for (const WorkItem& w : plan_.items) {
+    std::vector<WorkItem> listless;  // the items of a plan without a list (see work_item)
+    for (int p = 0; p < plan_.P && plan_.sp[p].itemsPerProblem > 0; ++p) {
+        const SweepProblem& sp = plan_.sp[p];
+        for (int k = 0; k < sp.itemsPerProblem; ++k) {
+            WorkItem w{};
+            w.problem = p;
+            w.strip = k / sp.slots;
+            w.jt1 = std::max(0, std::min((w.strip + 1) * R, sp.nTiles) -
+                                    k % sp.slots * sp.chunkTiles);
+            w.jt0 = std::max(0, w.jt1 - sp.chunkTiles);
+            listless.push_back(w);
+        }
+    }
+    for (const WorkItem& w : listless.empty() ? plan_.items : listless) {
         const SetView& s = sets[plan_.setOf[w.problem]];
         const PairConsts& c = plan_.sp[w.problem].c;
         const int nTiles = plan_.sp[w.problem].nTiles;

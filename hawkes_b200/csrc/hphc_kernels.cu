@@ -587,7 +587,7 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
 #pragma unroll
     for (int q = 0; q < kNumAcc; ++q) s[q] = 0.0;
     if (i < N) {
-        const int nc = P.stripChunks[i / P.stripEvents];
+        const int nc = P.stripChunks ? P.stripChunks[i / P.stripEvents] : P.slots;
 #pragma unroll
         for (int q = 0; q < kNumAcc; ++q) {
             if (q < 3 && P.keptB) {

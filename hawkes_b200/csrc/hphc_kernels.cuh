@@ -115,6 +115,7 @@ struct ConstsSpec {
     // (0: no window), and the events expected within scaled distance 1 of an
     // event, N / (T extent) V_D / (D/2 + 1), V_D the unit ball's volume.
     double selfCount, selfDensity;
+    double selfTile;  // mean time between a tile's ends
 };
 
 // Far background tail of the FP32 software-exponential mode.  A tile pair
@@ -240,19 +241,13 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     f.skipS = f.fullS = c.skipS;
     f.selfLeast = 0.0;
     if (s.selfCount > 0.0 && c.skipS > 0.0 && c.cS < 0.0) {
-        const double root = sqrt(2.0) / fabs(sigma);
         double perE = s.selfDensity / omega;
-        for (int k = 0; k < s.D; ++k) perE *= root;
-        double E = 1.0;  // in steps of 1/8: products and square roots only
-        for (; E < thr; E *= 1.125) {
-            double count = perE * E;
-            const double r = sqrt(E);
-            for (int k = 0; k < s.D; ++k) count *= r;
-            if (count >= kSelfMisses) break;
-        }
+        for (int k = 0; k < s.D; ++k) perE *= sqrt(2.0) / fabs(sigma);
+        const double E = pow(kSelfMisses / perE, 1.0 / (0.5 * s.D + 1.0));
         // 41.6 = 60 ln 2, 25.0 = 36 ln 2; 6.6 = ln 710
         const double x = log(s.selfCount) + 6.6 + (fp32 ? 25.0 : 41.6) + E;
-        if (x < 0.7 * thr) {
+        // worth it where it leaves out whole tiles
+        if (x < 0.7 * thr && thr - x > 3.0 * omega * s.selfTile) {
             c.skipS = f.skipS = x;
             f.selfLeast = s.selfCount * x * exp(-x) * (fp32 ? 0x1p36 : 0x1p60);
         }
@@ -409,7 +404,12 @@ struct SweepProblem {
     // Items may start far before the first tile holding a term (plans built
     // for any sigma and omega, sorted times): the sweep finds that tile by
     // bisection on the tile time bounds instead of scanning to it.
-    int searchBand, pad[3];
+    int searchBand;
+    // Self-excitation-only plans of problems with sorted times and one size
+    // carry no work list: item k of the launch is problem k / itemsPerProblem,
+    // there strip (k % itemsPerProblem) / slots, and of that strip's tiles, counted
+    // back from its own last one, the chunkTiles of slot k % slots.
+    int itemsPerProblem, slots, chunkTiles;
     // FP32 sweep: event of row r of thread t of a full strip, at
     // [stripBase + r * 128 + t] (launch_strip_order for the sweep's R), or
     // null for the identity order.
@@ -441,7 +441,7 @@ struct FinishProblem {
     const double* partials;   // [slot][6][Npad]
     unsigned long long* colAcc;  // [3][Npad] symmetric-sweep column sums, or null; zeroed once
                                  // read
-    const int* stripChunks;   // slots used by each strip
+    const int* stripChunks;   // slots used by each strip, or null: `slots` by every strip
     const double* times;      // the set's raw times
     double* probs;            // P_i output (may be null)
     double* sums;             // [6][N] unit pair sums out, natural units (may be null)
@@ -455,6 +455,7 @@ struct FinishProblem {
     int N, Npad, stripEvents, blockBase;  // blockBase: first finish CTA of this problem
     int nBlocks, colWords, nTiles, sorted;  // colWords: 1 = FP32 column format, 2 = FP64
     int colShift[4];
+    int slots, pad0;
     FinishConsts f;
 };
 

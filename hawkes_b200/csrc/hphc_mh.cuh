@@ -91,11 +91,16 @@ HPHC_HD inline double log_truncated_normal(double x, double mean, double sd) {
     return -0.5 * z * z - log(sd) - kLogSqrt2Pi - log(tail);
 }
 
-// Log prior of the reference's Potential (R/Untitled.R:226-227).
+// Log prior density of parameter q in the reference's Potential
+// (R/Untitled.R:226-227).
+HPHC_HD inline double log_prior_term(const double* p, int q) {
+    return log_truncated_normal(p[q], 0.0, q < 5 ? 10.0 : 1.0);
+}
+
 HPHC_HD inline double log_prior(const double* p) {
     double s = 0.0;
-    for (int k = 0; k < 5; ++k) s += log_truncated_normal(p[k], 0.0, 10.0);
-    return s + log_truncated_normal(p[5], 0.0, 1.0);
+    for (int k = 0; k < 5; ++k) s += log_prior_term(p, k);
+    return s + log_prior_term(p, 5);
 }
 
 struct Chain {
@@ -138,13 +143,27 @@ HPHC_HD inline void propose(Chain& c, const int* sampled, int nSampled, double* 
     prop[idx] = truncated_normal(c.rng, c.former, c.radii[idx]);
 }
 
-// Accept or reject the proposal given its log-likelihood, then adapt.
-HPHC_HD inline void accept(Chain& c, const double* prop, double loglik) {
+// The densities an acceptance test needs, one at a time (the device driver forms
+// them in parallel): the prior of each parameter, the proposal's density from
+// the current value and the other way round.
+constexpr int kAcceptTerms = kParams + 2;
+
+HPHC_HD inline double accept_term(const Chain& c, const double* prop, int q) {
+    if (q < kParams) return log_prior_term(prop, q);
+    const double r = c.radii[c.index];
+    return q == kParams ? log_truncated_normal(prop[c.index], c.former, r)
+                        : log_truncated_normal(c.former, prop[c.index], r);
+}
+
+// Accept or reject the proposal given its log-likelihood and accept_term's
+// densities, then adapt.
+HPHC_HD inline void accept(Chain& c, const double* prop, double loglik, const double* terms) {
     const int idx = c.index;
-    const double r = c.radii[idx];
-    const double propU = -loglik - log_prior(prop);
-    const double curH = c.potential - log_truncated_normal(prop[idx], c.former, r);
-    const double propH = propU - log_truncated_normal(c.former, prop[idx], r);
+    double prior = 0.0;
+    for (int k = 0; k < kParams; ++k) prior += terms[k];
+    const double propU = -loglik - prior;
+    const double curH = c.potential - terms[kParams];
+    const double propH = propU - terms[kParams + 1];
     const double ratio = -propH + curH;
     const double logU = log(c.rng.uniform());
     ++c.proposed;
@@ -162,6 +181,12 @@ HPHC_HD inline void accept(Chain& c, const double* prop, double loglik) {
         c.sampBound[idx] = (int)ceil(pow((double)c.sampBound[idx], 1.1));
         c.acceptances[idx] = 0;
     }
+}
+
+HPHC_HD inline void accept(Chain& c, const double* prop, double loglik) {
+    double terms[kAcceptTerms];
+    for (int q = 0; q < kAcceptTerms; ++q) terms[q] = accept_term(c, prop, q);
+    accept(c, prop, loglik, terms);
 }
 
 }  // namespace mh

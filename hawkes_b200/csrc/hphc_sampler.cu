@@ -12,12 +12,11 @@
 //                  CUDA graph) or by a caller-supplied evaluator, and accepts
 //                  on the host;
 //   device driver  hphc_sampler_run_device: the chains live in device memory
-//                  and one iteration -- a proposal kernel that also rewrites
-//                  each problem's parameter constants in the engine's device
-//                  tables, the pair sweep, finish and final kernels, and an
-//                  acceptance kernel -- is captured once into a CUDA graph and
-//                  replayed for every iteration, with no host work or
-//                  transfer in between.
+//                  and one iteration -- the pair sweep, the finish and a step
+//                  kernel that accepts, proposes and rewrites each problem's
+//                  parameter constants in the engine's device tables -- is
+//                  captured once into a CUDA graph and replayed for every
+//                  iteration, with no host work or transfer in between.
 //
 // Both drivers draw the same random numbers (one splitmix64 stream per chain)
 // and evaluate with the same kernels; their chains differ only where the host
@@ -48,47 +47,69 @@ struct SampledSet {
     int n;
 };
 
-constexpr int kChainThreads = 128;
+// One step of every chain between two evaluations: the acceptance of the
+// proposal just evaluated (accepting; results: K x 8, [0] = log-likelihood) with
+// the chain's state into samples (K x saved x 6) and targets (K x saved) after
+// burn-in, then, but for the last iteration, the next proposal with problem k's
+// constants in the engine's device tables rewritten for it (the fields that
+// depend on the event set only, T and constant, are kept).
+//
+// A step is one long chain of FP64 functions, so its latency is what counts: a
+// warp per chain (chains of one warp would take each other's branches and
+// rejection loops in turn), the eight densities of an acceptance on eight
+// lanes, the chain's state in shared memory, and one launch for both halves.
+// N = 1000, 16 chains, an iteration with separate one-thread-per-chain kernels
+// (26 us of it) and listed plans: 74 us in the FP32-compensated mode and 69 in
+// FP64; now 54 and 48.
+constexpr int kStepThreads = 32;
 
-// Proposal of every chain; the problem k constants in the engine's device
-// tables are rewritten for the proposal (the fields that depend on the event
-// set only, T and constant, are kept).  Thread 0 also advances the
-// iteration counter.
-__global__ void __launch_bounds__(kChainThreads)
-mh_propose_kernel(Chain* __restrict__ chains, int K, SampledSet sampled,
-                  double* __restrict__ prop, hphc::SweepProblem* __restrict__ sp,
-                  hphc::FinishProblem* __restrict__ fp, hphc::ConstsSpec spec,
-                  int* __restrict__ iteration) {
-    const int k = blockIdx.x * kChainThreads + threadIdx.x;
-    if (k == 0) ++*iteration;
-    if (k >= K) return;
-    double* p = prop + (size_t)k * kParams;
-    hphc::mh::propose(chains[k], sampled.idx, sampled.n, p);
-    hphc::PairConsts c = sp[k].c;
-    hphc::FinishConsts f = fp[k].f;
-    hphc::param_consts(p, spec, c, f);
-    sp[k].c = c;
-    fp[k].f = f;
-}
-
-// Acceptance of every chain from its proposal's log-likelihood (results:
-// K x 8, [0] = log-likelihood) and, after burn-in, the chain's state into
-// samples (K x saved x 6) and targets (K x saved).
-__global__ void __launch_bounds__(kChainThreads)
-mh_accept_kernel(Chain* __restrict__ chains, int K, const double* __restrict__ prop,
-                 const double* __restrict__ results, const int* __restrict__ iteration,
-                 int burnIn, int saved, double* __restrict__ samples,
-                 double* __restrict__ targets) {
-    const int k = blockIdx.x * kChainThreads + threadIdx.x;
-    if (k >= K) return;
-    Chain& c = chains[k];
-    hphc::mh::accept(c, prop + (size_t)k * kParams, results[(size_t)8 * k]);
-    const int it = *iteration;  // 1-based, advanced by this iteration's proposal kernel
-    if (it > burnIn && it - burnIn <= saved) {
-        const size_t s = (size_t)k * saved + (it - burnIn - 1);
-        for (int q = 0; q < kParams; ++q) samples[s * kParams + q] = c.params[q];
-        targets[s] = c.potential;
+__global__ void __launch_bounds__(kStepThreads)
+mh_step_kernel(Chain* __restrict__ chains, SampledSet sampled, double* __restrict__ prop,
+               hphc::SweepProblem* __restrict__ sp, hphc::FinishProblem* __restrict__ fp,
+               hphc::ConstsSpec spec, const double* __restrict__ results,
+               int* __restrict__ iteration, bool accepting, int iterations, int burnIn, int saved,
+               double* __restrict__ samples, double* __restrict__ targets) {
+    const int k = blockIdx.x, lane = threadIdx.x;
+    __shared__ Chain c;
+    __shared__ double p[kParams];
+    static_assert(sizeof(Chain) % sizeof(int) == 0, "copied as words");
+    constexpr int kWords = sizeof(Chain) / sizeof(int);
+    int* words = reinterpret_cast<int*>(&c);
+    int* stored = reinterpret_cast<int*>(chains + k);
+    for (int w = lane; w < kWords; w += kStepThreads) words[w] = stored[w];
+    if (lane < kParams) p[lane] = prop[(size_t)k * kParams + lane];
+    int done = iteration[k];
+    __syncwarp();
+    if (accepting) {
+        const double term = lane < hphc::mh::kAcceptTerms ? hphc::mh::accept_term(c, p, lane) : 0.0;
+        double terms[hphc::mh::kAcceptTerms];
+#pragma unroll
+        for (int q = 0; q < hphc::mh::kAcceptTerms; ++q)
+            terms[q] = __shfl_sync(0xffffffffu, term, q);
+        ++done;
+        __syncwarp();
+        if (lane == 0) {
+            hphc::mh::accept(c, p, results[(size_t)8 * k], terms);
+            iteration[k] = done;
+        }
+        __syncwarp();
+        if (done > burnIn && done - burnIn <= saved) {
+            const size_t s = (size_t)k * saved + (done - burnIn - 1);
+            if (lane < kParams) samples[s * kParams + lane] = c.params[lane];
+            if (lane == 0) targets[s] = c.potential;
+        }
     }
+    if (done < iterations && lane == 0) {
+        hphc::PairConsts pc = sp[k].c;
+        hphc::FinishConsts f = fp[k].f;
+        hphc::mh::propose(c, sampled.idx, sampled.n, p);
+        hphc::param_consts(p, spec, pc, f);
+        sp[k].c = pc;
+        fp[k].f = f;
+    }
+    __syncwarp();
+    for (int w = lane; w < kWords; w += kStepThreads) stored[w] = words[w];
+    if (lane < kParams) prop[(size_t)k * kParams + lane] = p[lane];
 }
 
 }  // namespace
@@ -293,25 +314,28 @@ int hphc_sampler_run_device(hphc_sampler* s, hphc_engine* engine, int iterations
         (e = cudaMalloc(&run.prop, sizeof(double) * kParams * K)) ||
         (e = cudaMalloc(&run.samples, sizeof(double) * kParams * nSaved)) ||
         (e = cudaMalloc(&run.targets, sizeof(double) * nSaved)) ||
-        (e = cudaMalloc(&run.iteration, sizeof(int))))
+        (e = cudaMalloc(&run.iteration, sizeof(int) * K)))
         return cuda_fail("device allocation");
     cudaStream_t stream = loop.stream;
     if ((e = cudaMemcpyAsync(run.chains, s->chains.data(), sizeof(Chain) * K,
                              cudaMemcpyHostToDevice, stream)) ||
-        (e = cudaMemsetAsync(run.iteration, 0, sizeof(int), stream)))
+        (e = cudaMemsetAsync(run.iteration, 0, sizeof(int) * K, stream)))
         return cuda_fail("upload chains");
 
-    // one iteration, captured once
-    const int blocks = (K + kChainThreads - 1) / kChainThreads;
+    const auto step = [&](bool accepting) {
+        mh_step_kernel<<<K, kStepThreads, 0, stream>>>(
+            run.chains, sampled, run.prop, loop.ex->device_sweep_problems(),
+            loop.ex->device_finish_problems(), loop.spec, loop.ex->device_results(),
+            run.iteration, accepting, iterations, burnIn, saved, run.samples, run.targets);
+    };
+    // the first proposals, then one iteration, captured once: evaluation,
+    // acceptance and the next proposals
+    step(false);
+    if ((e = cudaGetLastError())) return cuda_fail("first proposals");
     if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal)))
         return cuda_fail("begin graph capture");
-    mh_propose_kernel<<<blocks, kChainThreads, 0, stream>>>(
-        run.chains, K, sampled, run.prop, loop.ex->device_sweep_problems(),
-        loop.ex->device_finish_problems(), loop.spec, run.iteration);
     st = loop.ex->enqueue_device_body();
-    mh_accept_kernel<<<blocks, kChainThreads, 0, stream>>>(
-        run.chains, K, run.prop, loop.ex->device_results(), run.iteration, burnIn, saved,
-        run.samples, run.targets);
+    step(true);
     cudaError_t launchErr = cudaGetLastError();
     e = cudaStreamEndCapture(stream, &run.graph);
     if (st) return s->fail(st, "device loop: %s", loop.ex->error.c_str());

@@ -494,6 +494,27 @@ __device__ __forceinline__ int next_item(int* counter, int* sNext) {
     return *sNext;
 }
 
+// Item `it` of a launch: from the list, or (SELF) from its number where the
+// problems carry no list.  A slot before the first tile is empty: its sums are
+// written as zeros.
+template <bool SELF, int R>
+__device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ problems,
+                                              const WorkItem* __restrict__ items, int it) {
+    if (!SELF || problems[0].itemsPerProblem == 0) return items[it];
+    const int per = problems[0].itemsPerProblem;
+    WorkItem w;
+    w.problem = it / per;
+    const SweepProblem& P = problems[w.problem];
+    const int k = it - w.problem * per;
+    w.strip = k / P.slots;
+    w.slot = k - w.strip * P.slots;
+    w.jt1 = max(0, min((w.strip + 1) * R, P.nTiles) - w.slot * P.chunkTiles);
+    w.start = w.jt0 = max(0, w.jt1 - P.chunkTiles);
+    if (P.searchBand && w.jt1 - w.jt0 > 2)
+        w.start = first_tile_with_terms(P, R, w.strip, w.jt0, w.jt1);
+    return w;
+}
+
 // Work-list form: persistent CTAs take items until the list is exhausted.
 // The self-excitation-only form needs 96 registers instead of 168 at R = 2, so five
 // CTAs share an SM instead of three: N = 100k self-excitation sweep 1.37 -> 1.24 ms
@@ -510,7 +531,7 @@ sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
     for (;;) {
         const int it = next_item(counter, &sNext);
         if (it >= n) break;
-        const WorkItem w = items[it];
+        const WorkItem w = work_item<SELF, R>(problems, items, it);
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         const int shift[3] = {P.colShift[0], P.colShift[1], P.colShift[2]};
@@ -1151,7 +1172,7 @@ sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
     for (;;) {
         const int it = next_item(counter, &sNext);
         if (it >= n) break;
-        const WorkItem w = items[it];
+        const WorkItem w = work_item<SELF, R>(problems, items, it);
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         f32c_item<D, R, V, SELF>(static_cast<const float*>(P.rec), P.tileMin, P.tileMax, P.partials,
