@@ -416,7 +416,7 @@ struct Runtime {
         const bool plainSums = mode.fastTail && mode.truncateTail && mode.underflowSkip &&
                                (mode.precision == HPHC_PRECISION_FP64 ||
                                 (mode.precision == HPHC_PRECISION_FP32_COMP && mode.variant == 2));
-        ex.gridSums = plainSums && mode.symmetric && mode.precision == HPHC_PRECISION_FP64;
+        ex.gridSums = plainSums && mode.symmetric;
         ex.selfWindow = plainSums;
         if (st) err = ex.error;
         return st;
