@@ -181,11 +181,14 @@ struct EventSet {
     HostBuf<int32_t> hRanks;
     std::vector<double> hTileMin, hTileMax;
     bool sorted = false;
+    bool precision64 = false;  // FP64 mode: the records are packed at each upload
     bool floatTimes = false;  // plain FP32 mode: causality from the times rounded to FP32
     DevBuf<double> dLoc, dTimes, dRecF64, dTileMin, dTileMax;
     DevBuf<int32_t> dRanks;
     DevBuf<int> dTileChanges;  // FP32 mode, sorted times: ranks computed on the device
     DevBuf<int32_t> dOrder2, dOrder4;  // FP32 mode: spatial row order of R = 2 and 4 strips
+    bool ordered2 = false, ordered4 = false;  // formed for the uploaded events
+    bool packedF64 = false;                   // FP32-compensated mode
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 
@@ -220,6 +223,15 @@ struct EventSet {
         }
         haveBox = true;
     }
+    // The bounds from copy_checked's (D = 1 and 2).
+    void set_box(const double* box) {
+        if (D > 2) return;
+        locMin[0] = D == 1 ? std::min(box[0], box[1]) : box[0];
+        locMax[0] = D == 1 ? std::max(box[2], box[3]) : box[2];
+        locMin[1] = D == 1 ? 0.0 : box[1];
+        locMax[1] = D == 1 ? 0.0 : box[3];
+        haveBox = true;
+    }
     void widen_box(const double* row) {
         for (int k = 0; k < D; ++k) {
             locMin[k] = std::min(locMin[k], row[k]);
@@ -230,6 +242,7 @@ struct EventSet {
     cudaError_t alloc(int dim, int n, int precision) {
         D = dim;
         N = n;
+        precision64 = precision == HPHC_PRECISION_FP64;
         floatTimes = precision == HPHC_PRECISION_FP32;
         const int nTiles = (N + kTile - 1) / kTile;
         cudaError_t e;
@@ -243,6 +256,10 @@ struct EventSet {
                    (e = dOrder2.reserve(N)) || (e = dOrder4.reserve(N))) {
             return e;
         }
+        // large gridded evaluations of the FP32-compensated mode (Executor::enqueue)
+        if (precision == HPHC_PRECISION_FP32_COMP && D <= 2 && N >= kGridHighOrderEvents &&
+            (e = dRecF64.reserve((size_t)N * 4)))
+            return e;
         std::memset(hTimes.p, 0, (size_t)N * sizeof(double));
         std::memset(hRanks.p, 0, (size_t)N * sizeof(int32_t));
         hTileMin.assign(nTiles, 0.0);
@@ -322,11 +339,7 @@ struct EventSet {
             *launches += 2;
             return e;
         }
-        if ((e = launch_strip_order(D, N, 2, dLoc.p, dOrder2.p, s)) ||
-            (e = launch_strip_order(D, N, 4, dLoc.p, dOrder4.p, s)))
-            return e;
-        for (int S = 2 * kSweepThreads; S <= 4 * kSweepThreads; S *= 2)
-            *launches += (N >= S) + (N % S != 0);
+        ordered2 = ordered4 = packedF64 = false;
         if (sorted) {
             if ((e = launch_tile_bounds(N, dTimes.p, dTileMin.p, dTileMax.p, dTileChanges.p, s,
                                         floatTimes)))
@@ -343,7 +356,7 @@ struct EventSet {
         return e;
     }
 
-    SetView view() const {
+    SetView view() {
         SetView v;
         v.N = N;
         v.dLoc = dLoc.p;
@@ -351,7 +364,10 @@ struct EventSet {
         v.dRanks = dRanks.p;
         v.dOrder2 = dOrder2.p;
         v.dOrder4 = dOrder4.p;
+        v.ordered2 = &ordered2;
+        v.ordered4 = &ordered4;
         v.dRecF64 = dRecF64.p;
+        v.packedF64 = precision64 ? nullptr : &packedF64;
         v.dTileMin = dTileMin.p;
         v.dTileMax = dTileMax.p;
         v.hTimes = hTimes.p;
@@ -457,29 +473,43 @@ bool all_finite(const double* v, size_t n, size_t* bad) {
 // partly written and must be discarded).  ASC: *ascending = src is
 // non-decreasing.
 //
+// BOX: the bounds of the even and of the odd entries go to box[0..1] (minima)
+// and box[2..3], which D = 1 and D = 2 locations need (EventSet::set_box).
+//
 // The destination is a pinned mirror the next upload reads by DMA; with SSE2
 // and a 16-byte aligned destination the copy uses streaming stores, which
 // write it without first reading it into the cache (a third of the memory
 // traffic of the pass).
-template <bool ASC>
+template <bool ASC, bool BOX = false>
 bool copy_checked(const double* __restrict__ src, double* __restrict__ dst, size_t n,
-                  size_t* bad, bool* ascending) {
+                  size_t* bad, bool* ascending, double* box = nullptr) {
     constexpr uint64_t kExp = 0x7ff0000000000000ULL;
     uint64_t any = 0, desc = 0;
     size_t i0 = 0;
+    if (BOX)
+        for (int k = 0; k < 2; ++k) box[k] = box[2 + k] = src[n > 1 ? k : 0];
 #if defined(__SSE2__)
     if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && n >= 4) {
         const __m128d zero = _mm_setzero_pd();
         __m128d bad2 = zero, desc2 = zero;
+        __m128d low = _mm_loadu_pd(src), high = low;
         const size_t n2 = n & ~size_t(1);
         for (size_t i = 0; i < n2; i += 2) {
             const __m128d v = _mm_loadu_pd(src + i);
             const __m128d z = _mm_mul_pd(v, zero);  // 0 for finite values, NaN otherwise
             bad2 = _mm_or_pd(bad2, _mm_cmpunord_pd(z, z));
             if (ASC && i > 0) desc2 = _mm_or_pd(desc2, _mm_cmpgt_pd(_mm_loadu_pd(src + i - 1), v));
+            if (BOX) {
+                low = _mm_min_pd(low, v);
+                high = _mm_max_pd(high, v);
+            }
             _mm_stream_pd(dst + i, v);
         }
         _mm_sfence();
+        if (BOX) {
+            _mm_storeu_pd(box, low);
+            _mm_storeu_pd(box + 2, high);
+        }
         if (ASC && n2 > 1 && src[0] > src[1]) desc = 1;
         if (_mm_movemask_pd(bad2)) any = 1;
         if (_mm_movemask_pd(desc2)) desc = 1;
@@ -492,6 +522,10 @@ bool copy_checked(const double* __restrict__ src, double* __restrict__ dst, size
         std::memcpy(&u, &v, sizeof u);
         any |= (uint64_t)((u & kExp) == kExp);
         if (ASC && i > 0) desc |= (uint64_t)(src[i - 1] > v);
+        if (BOX) {
+            box[i & 1] = std::min(box[i & 1], v);
+            box[2 + (i & 1)] = std::max(box[2 + (i & 1)], v);
+        }
         dst[i] = v;
     }
     if (ASC) *ascending = desc == 0;
@@ -523,6 +557,8 @@ struct hphc_engine {
     // value is finite: a rejected input leaves the events unchanged.
     HostBuf<double> hLocSpare, hTimesSpare;
     EventSet set;
+    double storedMin[kMaxDim] = {}, storedMax[kMaxDim] = {};  // stored locations' bounds
+    bool storedBox = false;
     DevBuf<double> dProbs;
     std::vector<double> hOut;
     bool dirty = true;
@@ -743,6 +779,7 @@ struct hphc_engine {
             lastLaunches += 2;
         }
         if (hadMoves && !wasDirty && rt.mode.precision == HPHC_PRECISION_FP64) recStale = true;
+        if (hadMoves) set.packedF64 = false;
         lastIncTerms = (double)moved.size() * (3.0 * N - 2.0);
         clear_moved();
         const FinishConsts f = rt.ex.finish_consts(p, set.view());
@@ -997,10 +1034,12 @@ int hphc_update_locations(hphc_engine* e, int locationIndex, const double* locat
     }
     size_t bad = 0;
     if (locationIndex == -1) {
-        if (!copy_checked<false>(location, e->hLocSpare.p, length, &bad, nullptr))
+        double box[4];
+        if (!copy_checked<false, true>(location, e->hLocSpare.p, length, &bad, nullptr, box))
             return e->fail(HPHC_ERR_NONFINITE, "locations: entry %zu is not finite", bad);
         e->hLoc[e->curLoc].swap(e->hLocSpare);
         e->set.haveBox = false;
+        e->set.set_box(box);
         e->invalidate_sums();
         e->dirty = true;
         return HPHC_OK;
@@ -1078,6 +1117,9 @@ int hphc_store_state(hphc_engine* e) {
     if (!e) return HPHC_ERR_INVALID_HANDLE;
     e->storedSumOfLikContribs = e->sumOfLikContribs;
     std::memcpy(e->storedParams, e->params, sizeof e->params);
+    std::memcpy(e->storedMin, e->set.locMin, sizeof e->storedMin);
+    std::memcpy(e->storedMax, e->set.locMax, sizeof e->storedMax);
+    e->storedBox = e->set.haveBox;
     std::memcpy(e->hLoc[1 - e->curLoc].p, e->hLoc[e->curLoc].p,
                 (size_t)e->N * e->D * sizeof(double));
     // the kept sums describe the stored locations when no event has moved since
@@ -1099,7 +1141,9 @@ int hphc_restore_state(hphc_engine* e) {
     e->sumOfLikContribs = e->storedSumOfLikContribs;
     std::memcpy(e->params, e->storedParams, sizeof e->params);
     e->curLoc = 1 - e->curLoc;
-    e->set.haveBox = false;
+    std::swap(e->storedMin, e->set.locMin);
+    std::swap(e->storedMax, e->set.locMax);
+    std::swap(e->storedBox, e->set.haveBox);
     e->dirty = true;
     e->clear_moved();
     if (e->storedSumsValid) {
@@ -1387,6 +1431,7 @@ int hphc_multiset_set_data(hphc_multiset* m, int set, const double* locations, s
     DeviceGuard g(m->rt.device);
     if (!g.ok) return fmt(m->lastError, HPHC_ERR_CUDA, "cannot select device %d", m->rt.device);
     cudaError_t e;
+    double box[4];
     int ascending = -1;
     if (m->ready[set] && !m->dirty[set]) {
         // The device holds the set's current data, so the new values are
@@ -1395,7 +1440,7 @@ int hphc_multiset_set_data(hphc_multiset* m, int set, const double* locations, s
         if ((e = cudaEventSynchronize(m->uploaded[set])) != cudaSuccess)
             return cuda_status(m->lastError, e, "wait for the set's upload");
         bool asc = false;
-        if (!copy_checked<false>(locations, m->hLoc[set].p, locLength, &bad, nullptr) ||
+        if (!copy_checked<false, true>(locations, m->hLoc[set].p, locLength, &bad, nullptr, box) ||
             !copy_checked<true>(times, es.hTimes.p, timesLength, &bad, &asc)) {
             if ((e = cudaMemcpy(m->hLoc[set].p, es.dLoc.p, locLength * sizeof(double),
                                 cudaMemcpyDeviceToHost)) ||
@@ -1415,7 +1460,8 @@ int hphc_multiset_set_data(hphc_multiset* m, int set, const double* locations, s
     }
     es.derive_times(ascending);
     es.haveBox = false;
-    if (m->rt.ex.selfWindow) es.update_box(m->hLoc[set].p);
+    if (ascending >= 0) es.set_box(box);
+    if (m->rt.ex.selfWindow) es.update_box(m->hLoc[set].p);  // if not known yet
     m->ready[set] = 1;
     m->dirty[set] = 1;
     // upload now, overlapping the host work on the next sets

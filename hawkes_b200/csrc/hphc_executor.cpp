@@ -309,12 +309,17 @@ void append_tune_file(const std::string& device, int sms, const TuneKey& key, in
 }
 
 // Gridded background sums: cost estimates (plan_grid) and limits.  Microseconds
-// from measured times (one B200): the FP64 sweep's background terms took 6.86 ms
-// for 3.38e9 pairs at N = 100k and 0.25 ms for 1.13e8 at N = 20k; the grid
-// kernels 0.20, 0.28 and 0.56 ms at N = 1,500, 20k and 100k with 1.24e6 nodes,
-// and 0.12 and 0.21 ms at N = 3,000 and 20k with 2.3e5 nodes.
-constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 0.83e-6;  // a pair
-constexpr double kGridCostFixed = 105.0, kGridCostEvent = 3.6e-3, kGridCostNode = 7.0e-5;
+// from measured times (one B200): the background terms of the sweeps took, at
+// N = 100k, 6.86 ms for 3.38e9 pairs in FP64 and 2.42 ms for 2.89e9 in FP32; the
+// grid kernels of order 16 0.48 ms at N = 100k with 1.24e6 nodes; those of order 12
+// 0.18 and 0.32 ms at N = 20k and 60k with 5.4e5 nodes, and 0.088 ms a problem
+// with 16 problems of N = 20k in a launch, which share the launches' latency.
+constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 0.90e-6;  // a pair
+constexpr double kGridCostFixed = 95.0;  // of a group of problems
+struct GridCost {
+    double event, node;
+};
+constexpr GridCost kGridCost16{3.45e-3, 5.0e-5}, kGridCost12{3.2e-3, 5.0e-5};
 constexpr int kGridMinEvents = 1000;
 constexpr double kGridMaxNodes = 4e8;
 constexpr size_t kGridMaxWork = size_t(8) << 30;    // one problem's workspace
@@ -340,7 +345,7 @@ int Executor::cuda_fail(cudaError_t e, const char* what) {
 int Executor::init(int D, int precision, int variant, bool underflowSkip, int device,
                    cudaStream_t stream, double ex2Bias) {
     D_ = D;
-    precision_ = precision;
+    precision_ = planPrecision_ = precision;
     variant_ = variant;
     skip_ = underflowSkip;
     device_ = device;
@@ -357,14 +362,14 @@ int Executor::init(int D, int precision, int variant, bool underflowSkip, int de
     return HPHC_OK;
 }
 
-void Executor::drop_graph() {
-    if (graphExec_) cudaGraphExecDestroy(graphExec_);
-    graphExec_ = nullptr;
-    graphKey_ = GraphKey{};
+void Executor::drop_graph(int kind) {
+    if (graphExec_[kind]) cudaGraphExecDestroy(graphExec_[kind]);
+    graphExec_[kind] = nullptr;
+    graphKey_[kind] = GraphKey{};
 }
 
 void Executor::release() {
-    drop_graph();
+    drop_graphs();
     if (dTables_) cudaFree(dTables_);
     if (hStaging_) cudaFreeHost(hStaging_);
     if (dRecPool_) cudaFree(dRecPool_);
@@ -395,7 +400,7 @@ void Executor::release() {
 
 ConstsSpec Executor::consts_spec() const {
     ConstsSpec s{};
-    s.precision = precision_ == HPHC_PRECISION_FP64 ? 0 : 1;
+    s.precision = planPrecision_ == HPHC_PRECISION_FP64 ? 0 : 1;
     s.D = D_;
     s.variant = variant_;
     s.skip = skip_ ? 1 : 0;
@@ -460,7 +465,7 @@ FinishConsts Executor::finish_consts(const double* p, const SetView& set) const 
 }
 
 int Executor::sweep_grid(int r) const {
-    const int perSM = sweep_list_blocks_per_sm(precision_ == HPHC_PRECISION_FP64 ? 0 : 1, D_, r,
+    const int perSM = sweep_list_blocks_per_sm(planPrecision_ == HPHC_PRECISION_FP64 ? 0 : 1, D_, r,
                                                sweep_variant());
     return numSMs_ * std::max(1, perSM);
 }
@@ -479,11 +484,10 @@ double* Executor::grid_sums(int p) const {
     return p == 0 && sumsOut ? sumsOut : dGridSums_ + gridSumsOff_[p];
 }
 
-// Which problems take their background sums from a grid.  The choice depends
-// on the problem alone (not on the others of its batch), so that a batch and
-// single evaluations take the same path: the estimated time of the grid kernels
-// (fixed, per event and per node) against that of the pairs the sweep would
-// evaluate, counted from sampled tiles of sorted times.  A wide grid (sharp
+// Which problems take their background sums from a grid: those whose estimated
+// time on it (fixed, shared by the problems of a launch, per event and per node)
+// is below that of the pairs the sweep would evaluate, counted from sampled tiles
+// of sorted times.  A wide grid (sharp
 // kernels over a long span) has too many nodes and stays with the sweep.
 void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
                          int P) {
@@ -520,11 +524,15 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
                 tMax = std::max(tMax, s.hTileMax[k]);
             }
         const double direct = pairs * (fp32 ? kPairCostF32 : kPairCostF64);
-        const double maxNodes = (direct - kGridCostFixed - s.N * kGridCostEvent) / kGridCostNode;
+        const int order = fp32 && s.N < kGridHighOrderEvents ? 12 : 16;
+        const GridCost& cost = order == 16 ? kGridCost16 : kGridCost12;
+        const double maxNodes =
+            (direct - kGridCostFixed / std::min(P, kGridMaxJobs) - s.N * cost.event) / cost.node;
         if (!(maxNodes > 0.0)) continue;
         const double lo[3] = {tMin, D_ == 2 ? s.locMin[1] : 0.0, s.locMin[0]};
         const double hi[3] = {tMax, D_ == 2 ? s.locMax[1] : 0.0, s.locMax[0]};
-        const GridShape g = grid_shape(prm[1], prm[2], lo, hi, std::min(maxNodes, kGridMaxNodes));
+        const GridShape g = grid_shape(order, prm[1], prm[2], lo, hi,
+                                       std::min(maxNodes, kGridMaxNodes));
         if (!g.ok) continue;
         const size_t need = grid_workspace(g, s.N);
         if (need > kGridMaxWork) continue;
@@ -572,30 +580,33 @@ int Executor::launch_grid(const std::vector<SetView>& sets, const int* setOf,
     if (kernelTiming && (e = cudaEventRecord(ev_[4], stream_))) return cuda_fail(e, "timing event");
     std::vector<GridJob> jobs;
     size_t used = 0;
-    const auto flush = [&]() {
-        if (jobs.empty()) return cudaSuccess;
-        const cudaError_t err = launch_grid_sums(jobs.data(), (int)jobs.size(), stream_,
-                                                 &gridLaunches_);
-        jobs.clear();
-        used = 0;
-        return err;
-    };
-    for (int p = 0; p < P; ++p) {
-        if (!gridOf_[p]) continue;
-        const SetView& s = sets[setOf[p]];
-        const double* prm = params + (size_t)6 * p;
-        const size_t need = grid_workspace(gridShape_[p], s.N);
-        if (((int)jobs.size() == kGridMaxJobs || used + need > gridWorkCap_) && (e = flush()))
-            return cuda_fail(e, "gridded sums");
-        GridJob j{};
-        j.loc = s.dLoc;
-        j.times = s.dTimes;
-        j.sums = grid_sums(p);
-        grid_job(gridShape_[p], prm[1], prm[2], s.N, D_, static_cast<char*>(dGridWork_) + used, &j);
-        used += need;
-        jobs.push_back(j);
+    for (const int order : {12, 16}) {
+        const auto flush = [&]() {
+            if (jobs.empty()) return cudaSuccess;
+            const cudaError_t err = launch_grid_sums(order, jobs.data(), (int)jobs.size(),
+                                                     numSMs_, stream_, &gridLaunches_);
+            jobs.clear();
+            used = 0;
+            return err;
+        };
+        for (int p = 0; p < P; ++p) {
+            if (!gridOf_[p] || gridShape_[p].order != order) continue;
+            const SetView& s = sets[setOf[p]];
+            const double* prm = params + (size_t)6 * p;
+            const size_t need = grid_workspace(gridShape_[p], s.N);
+            if (((int)jobs.size() == kGridMaxJobs || used + need > gridWorkCap_) && (e = flush()))
+                return cuda_fail(e, "gridded sums");
+            GridJob j{};
+            j.loc = s.dLoc;
+            j.times = s.dTimes;
+            j.sums = grid_sums(p);
+            grid_job(gridShape_[p], prm[1], prm[2], s.N, D_, static_cast<char*>(dGridWork_) + used,
+                     &j);
+            used += need;
+            jobs.push_back(j);
+        }
+        if ((e = flush())) return cuda_fail(e, "gridded sums");
     }
-    if ((e = flush())) return cuda_fail(e, "gridded sums");
     if (kernelTiming && (e = cudaEventRecord(ev_[5], stream_))) return cuda_fail(e, "timing event");
     return HPHC_OK;
 }
@@ -612,7 +623,7 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     pl.stripChunks.clear();
     pl.fb.clear();
     pl.maxN = 0;
-    const bool fp32 = precision_ != HPHC_PRECISION_FP64;
+    const bool fp32 = planPrecision_ != HPHC_PRECISION_FP64;
     const int stripEvents = kSweepThreads * r;
     const int S32 = f32_stride(D_);
 
@@ -723,6 +734,14 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         sp.searchBand = (wideBands_ && s.sorted) ? 1 : 0;
         sp.rowOrder = (fp32 && sp.symmetric) ? (r == 2 ? s.dOrder2 : r == 4 ? s.dOrder4 : nullptr)
                                              : nullptr;
+        // the strips' row order is formed when a sweep first needs it
+        bool* ordered = sp.rowOrder ? (r == 2 ? s.ordered2 : s.ordered4) : nullptr;
+        if (ordered && !*ordered) {
+            const cudaError_t e = launch_strip_order(D_, N, r, s.dLoc, const_cast<int32_t*>(sp.rowOrder),
+                                                     stream_);
+            if (e != cudaSuccess) return cuda_fail(e, "strip order");
+            *ordered = true;
+        }
         sp.colAcc = nullptr;
         if (sp.symmetric) {
             sp.colAcc = reinterpret_cast<unsigned long long*>(colOff + 1);  // offset + 1
@@ -755,6 +774,14 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
             }
         } else {
             sp.rec = s.dRecF64;
+            if (s.packedF64 && !*s.packedF64) {  // FP32 engines: packed when first needed
+                const cudaError_t e =
+                    launch_pack_f64(D_, N, s.dLoc, s.dTimes, const_cast<double*>(s.dRecF64),
+                                    const_cast<double*>(s.dTileMin),
+                                    const_cast<double*>(s.dTileMax), stream_);
+                if (e != cudaSuccess) return cuda_fail(e, "pack FP64 records");
+                *s.packedF64 = true;
+            }
         }
 
         // work items: each strip's band of tiles that may hold a non-zero term
@@ -863,7 +890,9 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     offPJ_ = align16(offFB_ + sizeof(FinishBlock) * pl.fb.size());
     tablesBytes_ = align16(offPJ_ + sizeof(PackJob) * pl.pj.size());
 
-    recNeed_ = recOff;
+    // an FP64 plan of an FP32-compensated engine reserves the records its
+    // self-excitation steps will pack
+    recNeed_ = planPrecision_ == precision_ ? recOff : (size_t)pl.maxN * S32;
     partialsNeed_ = partOff;
     colNeed_ = colOff;
     int st = ensure_buffers();
@@ -948,7 +977,7 @@ int Executor::ensure_buffers() {
         grew = true;
     }
     if (grew) {
-        drop_graph();
+        drop_graphs();
         stale_ = true;
     }
     // the counters and column sums every run leaves at zero: set here when they
@@ -973,7 +1002,7 @@ cudaError_t Executor::record(cudaEvent_t ev) {
 // The stage sequence of one run on stream_ (also what the graph captures).
 int Executor::launch_sequence(int grid) {
     const Plan& pl = plan_;
-    const int prec = precision_ == HPHC_PRECISION_FP64 ? 0 : 1;
+    const int prec = planPrecision_ == HPHC_PRECISION_FP64 ? 0 : 1;
     char* d = static_cast<char*>(dTables_);
     const auto* sp = reinterpret_cast<const SweepProblem*>(d + offSP_);
     const auto* items = reinterpret_cast<const WorkItem*>(d + offItems_);
@@ -1013,7 +1042,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
     pairs /= std::max(1, shardWorld);  // work of this rank
     const int mode = variant_ | (symmetric ? 16 : 0) | (fastTail ? 32 : 0) | (skip_ ? 64 : 0) |
                      (truncateTail ? 128 : 0) | (selfOnly_ ? 256 : 0);
-    const TuneKey key = std::make_tuple(D_, precision_, mode, log2_bucket(pairs), log2_bucket(P));
+    const TuneKey key = std::make_tuple(D_, planPrecision_, mode, log2_bucket(pairs), log2_bucket(P));
     if (deviceName_.empty()) {
         cudaDeviceProp prop{};
         deviceName_ = cudaGetDeviceProperties(&prop, device_) == cudaSuccess ? prop.name : "?";
@@ -1037,7 +1066,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
     }
     std::vector<int> rs, its;
     if (fixedR) rs = {fixedR};
-    else if (precision_ == HPHC_PRECISION_FP64) rs = {1, 2};
+    else if (planPrecision_ == HPHC_PRECISION_FP64) rs = {1, 2};
     else rs = {2, 4};
     if (fixedItems) its = {fixedItems};
     else if (selfOnly_) its = {8, 16, 32};  // short sweeps: fewer items to plan and upload
@@ -1102,13 +1131,14 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
 int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
                            const double* params, int P, double* dProbs) {
     selfOnly_ = self_only(P);
-    Shape& s = shape_[selfOnly_ ? 1 : 0];
+    kind_ = !selfOnly_ ? 0 : planPrecision_ == precision_ ? 1 : 2;
+    Shape& s = shape_[kind_];
     if (fixedR && fixedItems) {
         s.R = fixedR;
         s.items = fixedItems;
         s.tuned = true;
     }
-    if (!s.tuned && shape_[0].tuned) {
+    if (kind_ == 1 && !s.tuned && shape_[0].tuned) {
         s = shape_[0];
         // a few thousand events: more, smaller strips fill the SMs
         if (selfOnly_ && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
@@ -1132,6 +1162,18 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
         return HPHC_ERR_BAD_ARGUMENT;
     }
     plan_grid(sets, setOf, params, P);
+    // Large gridded evaluations of the FP32-compensated mode sweep their
+    // self-excitation terms in FP64 too: the grid's sums are exact to 1e-15, and
+    // the sweep's 0.19 instead of 0.13 ms at N = 100k make the whole evaluation so
+    // (log-likelihood 2.7e-11 -> 1.1e-16, worst gradient component 9.6e-10 ->
+    // 3.6e-15 relative).
+    planPrecision_ = precision_;
+    if (precision_ == HPHC_PRECISION_FP32_COMP && !keptB && self_only(P)) {
+        bool large = true;
+        for (int p = 0; p < P; ++p)
+            large &= gridShape_[p].order == 16 && sets[setOf[p]].dRecF64 != nullptr;
+        if (large) planPrecision_ = HPHC_PRECISION_FP64;
+    }
     int st = choose_shape(sets, setOf, params, P, dProbs);
     if (st) return st;
     // the gridded sums need no plan: the device forms them while the host plans
@@ -1159,17 +1201,19 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     key.colNeed = colNeed_;
     key.tables = dTables_;
     key.timing = kernelTiming;
-    key.variant = sweep_variant();
-    const bool same = graphExec_ && key.P == graphKey_.P && key.nJobs == graphKey_.nJobs &&
-                      key.nBlocks == graphKey_.nBlocks &&
-                      key.maxN == graphKey_.maxN && key.R == graphKey_.R &&
-                      key.grid == graphKey_.grid && key.tablesBytes == graphKey_.tablesBytes &&
-                      key.colNeed == graphKey_.colNeed &&
-                      key.tables == graphKey_.tables && key.timing == graphKey_.timing &&
-                      key.variant == graphKey_.variant;
+    key.variant = sweep_variant() | planPrecision_ << 16;
+    cudaGraphExec_t& exec = graphExec_[kind_];
+    GraphKey& last = graphKey_[kind_];
+    const bool same = exec && key.P == last.P && key.nJobs == last.nJobs &&
+                      key.nBlocks == last.nBlocks &&
+                      key.maxN == last.maxN && key.R == last.R &&
+                      key.grid == last.grid && key.tablesBytes == last.tablesBytes &&
+                      key.colNeed == last.colNeed &&
+                      key.tables == last.tables && key.timing == last.timing &&
+                      key.variant == last.variant;
     cudaError_t e;
     if (!same) {
-        drop_graph();
+        drop_graph(kind_);
         cudaGraph_t graph = nullptr;
         if ((e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal)))
             return cuda_fail(e, "begin graph capture");
@@ -1182,18 +1226,18 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
             return st;
         }
         if (e != cudaSuccess) return cuda_fail(e, "end graph capture");
-        e = cudaGraphInstantiate(&graphExec_, graph, 0);
+        e = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) {
-            graphExec_ = nullptr;
+            exec = nullptr;
             return cuda_fail(e, "instantiate graph");
         }
-        graphKey_ = key;
+        last = key;
     }
     if (take_fault(HPHC_FAULT_LAUNCH))
         return cuda_fail(cudaErrorLaunchOutOfResources, "launch graph (injected)");
-    if ((e = cudaGraphLaunch(graphExec_, stream_))) return cuda_fail(e, "launch graph");
-    lastLaunches = (precision_ == HPHC_PRECISION_FP64 ? 2 : 3) + gridLaunches_;
+    if ((e = cudaGraphLaunch(exec, stream_))) return cuda_fail(e, "launch graph");
+    lastLaunches = (planPrecision_ == HPHC_PRECISION_FP64 ? 2 : 3) + gridLaunches_;
     timedValid = kernelTiming;
     return HPHC_OK;
 }
@@ -1234,17 +1278,18 @@ int Executor::setup_device_loop(const std::vector<SetView>& sets, const int* set
         return HPHC_ERR_BAD_ARGUMENT;
     }
     gridOf_.clear();  // the loop sweeps every term that is not kept
+    planPrecision_ = precision_;
     int st = choose_shape(sets, setOf, params, P, nullptr);
     if (st) return st;
     wideBands_ = true;
     st = build_plan(sets, setOf, params, P, nullptr, R, itemsPerSM);
     wideBands_ = false;
     if (st) return st;
-    drop_graph();  // the tables' layout changed under any captured graph
+    drop_graphs();  // the tables' layout changed under any captured graph
     cudaError_t e;
     if ((e = cudaMemcpyAsync(dTables_, hStaging_, tablesBytes_, cudaMemcpyHostToDevice, stream_)))
         return cuda_fail(e, "stage tables");
-    if (precision_ != HPHC_PRECISION_FP64) {
+    if (planPrecision_ != HPHC_PRECISION_FP64) {
         char* d = static_cast<char*>(dTables_);
         if ((e = launch_pack_f32_jobs(D_, (int)plan_.pj.size(), plan_.maxN,
                                       reinterpret_cast<const PackJob*>(d + offPJ_), stream_)))
@@ -1256,7 +1301,7 @@ int Executor::setup_device_loop(const std::vector<SetView>& sets, const int* set
 }
 
 int Executor::enqueue_device_body() {
-    const int prec = precision_ == HPHC_PRECISION_FP64 ? 0 : 1;
+    const int prec = planPrecision_ == HPHC_PRECISION_FP64 ? 0 : 1;
     char* d = static_cast<char*>(dTables_);
     const auto* sp = reinterpret_cast<const SweepProblem*>(d + offSP_);
     auto* items = reinterpret_cast<WorkItem*>(d + offItems_);

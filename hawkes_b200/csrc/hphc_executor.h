@@ -35,7 +35,10 @@ struct SetView {
     const int32_t* dRanks = nullptr;   // dense time ranks (FP32 mode)
     const int32_t* dOrder2 = nullptr;  // spatial row order of strips of R = 2 and 4 (FP32
     const int32_t* dOrder4 = nullptr;  //   mode, launch_strip_order), or null
-    const double* dRecF64 = nullptr;   // FP64 records (FP64 mode)
+    bool* ordered2 = nullptr;          // whether they hold the present events' order
+    bool* ordered4 = nullptr;
+    const double* dRecF64 = nullptr;   // FP64 records (FP64 mode; large FP32-compensated sets)
+    bool* packedF64 = nullptr;         // FP32-compensated: whether they hold the present events
     const double* dTileMin = nullptr;  // per-tile time bounds
     const double* dTileMax = nullptr;
     const double* hTimes = nullptr;    // host copies
@@ -135,6 +138,7 @@ public:
     int lastLaunches = 0;
 
 private:
+    int planPrecision_ = 0;  // of the current plan's sweep
     int D_ = 0, precision_ = 0, variant_ = 0, device_ = 0, numSMs_ = 148;
     bool skip_ = true;
     bool wideBands_ = false;  // build_plan: bands for any sampled parameters
@@ -144,12 +148,12 @@ private:
     double ex2Bias_ = 0.0;
     std::string deviceName_;  // for the persistent tune cache
     cudaStream_t stream_ = nullptr;
-    // shapes in use, of sweeps with background terms [0] and of
-    // self-excitation-only sweeps [1]
+    // shapes in use: sweeps with background terms, self-excitation-only sweeps, and
+    // those in FP64 of an FP32-compensated engine
     struct Shape {
         bool tuned = false;
         int R = 0, items = 0;
-    } shape_[2];
+    } shape_[3];
 
     // plan of the last enqueue
     struct Plan {
@@ -204,14 +208,17 @@ private:
     size_t colNeed_ = 0;                     // column-sum words the last plan needs
 
     // graph
-    cudaGraphExec_t graphExec_ = nullptr;
+    // one graph per kind of plan (shape_'s kinds), so that a sampler that mixes
+    // full evaluations and self-excitation steps captures each once
+    cudaGraphExec_t graphExec_[3] = {};
     struct GraphKey {
         int P = -1, nJobs = -1, nBlocks = -1, maxN = -1, R = -1, grid = -1;
         size_t tablesBytes = 0, colNeed = 0;
         void* tables = nullptr;
         int variant = 0;
         bool timing = false;
-    } graphKey_;
+    } graphKey_[3];
+    int kind_ = 0;  // of the current plan
 
     ConstsSpec consts_spec() const;
     int build_plan(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,
@@ -230,7 +237,10 @@ private:
     int autotune(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,
                  double* dProbs);
     int cuda_fail(cudaError_t e, const char* what);
-    void drop_graph();
+    void drop_graph(int kind);
+    void drop_graphs() {
+        for (int k = 0; k < 3; ++k) drop_graph(k);
+    }
     cudaError_t record(cudaEvent_t ev);
     bool capturing_ = false;
 

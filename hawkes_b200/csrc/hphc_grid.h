@@ -17,13 +17,18 @@
 // come from the derivatives of the gathered spline:
 //   sum_j B_ij u_k^2 = (f_kk + 2 f) / 4.
 //
-// Accuracy: a pair's term differs from the exact one by at most 2.5e-17, its
-// squared-distance weighted terms by at most 1.2e-15 (root mean square 4e-16),
-// in units of an event's own term B_ii = 1 (the splines' aliasing, evaluated in
-// extended precision over random pairs; the error alternates in sign with the
-// position against the grid).  Everything is FP64, and every sum but the
-// derivative weights is over positive numbers, so rounding adds no more than it
-// does in the pair sweep.
+// Two orders are built, with kInv and kTaps chosen for each (largest error of a
+// pair's term, and of its squared-distance weighted terms, in units of an event's
+// own term B_ii = 1: the splines' aliasing, evaluated in extended precision over
+// random pairs; it alternates in sign with the position against the grid):
+//
+//   kP   kInv  kTaps  term     weighted terms (root mean square)
+//   16   8     48     2.5e-17  1.2e-15 (4e-16)   FP64 accuracy
+//   12   6     32     1e-12    1.4e-10 (4e-11)   far below FP32 rounding of the
+//                                                coordinates (5e-8)
+//
+// Everything is FP64, and every sum but the derivative weights is over positive
+// numbers, so rounding adds no more than it does in the pair sweep.
 //
 // Work: O(N kP^3) for spread and gather and O(nodes kTaps) for the convolution,
 // against O(N^2) pair terms.
@@ -34,10 +39,28 @@
 
 namespace hphc {
 
-constexpr int kGridP = 16;    // spline order = nodes per event and coordinate
-constexpr int kGridInv = 8;   // nodes per unit of u
-constexpr int kGridTaps = 48; // |lag| of the convolution table (6 units of u)
+// Spline order -> nodes per unit of u, |lag| of the convolution table.
+template <int P>
+struct GridOrder;
+template <>
+struct GridOrder<16> {
+    static constexpr int kInv = 8, kTaps = 48;
+};
+template <>
+struct GridOrder<12> {
+    static constexpr int kInv = 6, kTaps = 32;
+};
+
+// The FP32-compensated mode takes order 12 below this size, where the order's
+// smaller cost shows most in batches of evaluations, and order 16 with FP64
+// self-excitation sums from it on (Executor::enqueue).  A step in sigma or omega,
+// which keeps the background and stays FP32-compensated, then costs below a
+// quarter of a full evaluation, as samplers expect of it.
+constexpr int kGridHighOrderEvents = 1 << 16;
+
 constexpr int kGridBin = 8;   // cells per bin and coordinate
+constexpr int kGridSpan = 24;  // nodes of a bin's events, rounded up to whole bins
+constexpr int kGridItemEvents = 128;
 constexpr int kGridMaxJobs = 16;  // jobs of one launch (kernel parameters)
 
 // One problem: an event set at one (tauX, tauT).  Coordinates are ordered
@@ -48,13 +71,16 @@ struct GridJob {
     double* sums;         // [3][N] unit background sums out (weights 1, d^2, dt^2)
     // workspace
     int* start;           // [bins + 1] counts, then exclusive prefix sums
+    int2* items;          // gather work: bin and first slot, at most kGridItemEvents slots each
+    int* nItems;
     int* binOf;           // [N] bin of event e, times kGridBin, plus its t cell in the bin
     int* pos;             // [N] arrival position of event e in its bin
     unsigned* key;        // [N] by slot: t cell in the bin << 28 | event, in arrival order
     int* event;           // [N] by slot: event, ordered by key within each bin
-    int4* cell;           // [N] by slot: cells (t, y, x)
-    double* wv;           // [N][3][kGridP] by slot: spline weights
-    double* wd;           // [N][3][kGridP] by slot: their second derivatives
+    int* cell;            // [N] by slot: cells in the bin, t | y << 8 | x << 16
+    double* wv;           // [N][3][kGridSpan] by slot: spline weights on the nodes from the
+                          // bin's first on (zeros around the kP of the event)
+    double* wd;           // [N][3][kP] by slot: their second derivatives
     double* ga;           // [nodes] grids
     double* gb;
     double scaleHi[3], scaleLo[3];  // grid units per coordinate unit, double-double
@@ -62,33 +88,31 @@ struct GridJob {
     double unitX2, unitT2;  // coordinate units^2 per u^2: 2 / a^2, 2 / b^2
     int nc[3];            // cells
     int nb[3];            // bins
-    int n[3];             // nodes (cells + kGridP - 1)
+    int n[3];             // nodes (cells + kP - 1)
     int N, D;
-};
-
-// Convolution table G[|lag|].
-struct GridTaps {
-    double g[kGridTaps + 1];
 };
 
 struct GridShape {
     bool ok = false;
+    int order = 0;
     double scaleHi[3], scaleLo[3], origin[3];
     int nc[3], nb[3], n[3];
     size_t nodes = 0, bins = 0;
 };
 
-// Grid of an event set with coordinates in [lo, hi] (order t, y, x) at
-// precisions a (space) and b (time); ok = false if it would hold more than
-// maxNodes nodes or the scales are unusable.
-GridShape grid_shape(double a, double b, const double* lo, const double* hi, double maxNodes);
+// Grid of spline order `order` (12 or 16) for an event set with coordinates in
+// [lo, hi] (order t, y, x) at precisions a (space) and b (time); ok = false if it
+// would hold more than maxNodes nodes or the scales are unusable.
+GridShape grid_shape(int order, double a, double b, const double* lo, const double* hi,
+                     double maxNodes);
 
 // Workspace bytes of one job.
 size_t grid_workspace(const GridShape& s, int N);
 // Fill a job's geometry and workspace pointers (workspace 256-byte aligned).
 void grid_job(const GridShape& s, double a, double b, int N, int D, void* workspace, GridJob* job);
 
-// Sums of up to kGridMaxJobs jobs; *launches += kernels launched.
-cudaError_t launch_grid_sums(const GridJob* jobs, int nJobs, cudaStream_t s, int* launches);
+// Sums of up to kGridMaxJobs jobs of one order; *launches += kernels launched.
+cudaError_t launch_grid_sums(int order, const GridJob* jobs, int nJobs, int numSMs,
+                             cudaStream_t s, int* launches);
 
 }  // namespace hphc

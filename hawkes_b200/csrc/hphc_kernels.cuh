@@ -175,13 +175,14 @@ constexpr double kNegligibleLog2F32 = 60.0;
 //
 // x = ln M + ln x + 60 ln 2 + E, where E is the exponent of an event's closest
 // earlier neighbour that all but about exp(-kSelfMisses) of the events stay
-// under: the expected number of neighbours with exponent below E, from the mean
+// under (more in FP64, whose longer underflow distance makes a completion
+// dearer): the expected number of neighbours with exponent below E, from the mean
 // density of the events, is C(E) = density (2/sigma^2)^(D/2) E^(D/2 + 1) / omega.
 // Without a window (unknown density, a fixed sweep shape, a shard's partial
 // sums, the full-sum flags, the plain FP32 mode) only the underflow skip is
 // left.  Measured at N = 100k (omega = 1 / h): 8.1e8 -> 9.9e7 terms and 1.24 -> 0.18 ms
 // in FP64, 1.30e8 -> 9.0e7 terms and 0.177 -> 0.128 ms in the FP32-compensated mode.
-constexpr double kSelfMisses = 16.0;
+constexpr double kSelfMisses = 24.0, kSelfMissesF32 = 16.0;
 
 // x y 32 log2(e), rounded once: two-product terms carry the rounding errors
 // of x y and of the constant, so the scaled coefficient is as accurate as the
@@ -243,7 +244,7 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     if (s.selfCount > 0.0 && c.skipS > 0.0 && c.cS < 0.0) {
         double perE = s.selfDensity / omega;
         for (int k = 0; k < s.D; ++k) perE *= sqrt(2.0) / fabs(sigma);
-        const double E = pow(kSelfMisses / perE, 1.0 / (0.5 * s.D + 1.0));
+        const double E = pow((fp32 ? kSelfMissesF32 : kSelfMisses) / perE, 1.0 / (0.5 * s.D + 1.0));
         // 41.6 = 60 ln 2, 25.0 = 36 ln 2; 6.6 = ln 710
         const double x = log(s.selfCount) + 6.6 + (fp32 ? 25.0 : 41.6) + E;
         // worth it where it leaves out whole tiles
