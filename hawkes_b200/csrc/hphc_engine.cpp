@@ -187,7 +187,7 @@ struct EventSet {
     DevBuf<int32_t> dRanks;
     DevBuf<int> dTileChanges;  // FP32 mode, sorted times: ranks computed on the device
     DevBuf<int32_t> dOrder2, dOrder4;  // FP32 mode: spatial row order of R = 2 and 4 strips
-    bool ordered2 = false, ordered4 = false;  // formed for the uploaded events
+    RowOrder order2, order4;
     bool packedF64 = false;                   // FP32-compensated mode
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
@@ -339,7 +339,15 @@ struct EventSet {
             *launches += 2;
             return e;
         }
-        ordered2 = ordered4 = packedF64 = false;
+        packedF64 = false;
+        order2.ready = order4.ready = false;
+        for (int R = 2; R <= 4; R += 2) {
+            RowOrder& order = R == 2 ? order2 : order4;
+            if (!order.wanted) continue;
+            if ((e = launch_strip_order(D, N, R, dLoc.p, R == 2 ? dOrder2.p : dOrder4.p, s))) return e;
+            order.ready = true;
+            *launches += (N >= R * kSweepThreads) + (N % (R * kSweepThreads) != 0);
+        }
         if (sorted) {
             if ((e = launch_tile_bounds(N, dTimes.p, dTileMin.p, dTileMax.p, dTileChanges.p, s,
                                         floatTimes)))
@@ -364,8 +372,8 @@ struct EventSet {
         v.dRanks = dRanks.p;
         v.dOrder2 = dOrder2.p;
         v.dOrder4 = dOrder4.p;
-        v.ordered2 = &ordered2;
-        v.ordered4 = &ordered4;
+        v.order2 = &order2;
+        v.order4 = &order4;
         v.dRecF64 = dRecF64.p;
         v.packedF64 = precision64 ? nullptr : &packedF64;
         v.dTileMin = dTileMin.p;

@@ -315,6 +315,7 @@ void append_tune_file(const std::string& device, int sms, const TuneKey& key, in
 // 0.18 and 0.32 ms at N = 20k and 60k with 5.4e5 nodes, and 0.088 ms a problem
 // with 16 problems of N = 20k in a launch, which share the launches' latency.
 constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 0.90e-6;  // a pair
+constexpr double kSelfCostF64 = 1.9e-6;  // a self-excitation term
 constexpr double kGridCostFixed = 95.0;  // of a group of problems
 struct GridCost {
     double event, node;
@@ -475,6 +476,19 @@ bool Executor::self_only(int P) const {
     if (gridOf_.empty()) return false;
     for (int p = 0; p < P; ++p)
         if (!gridOf_[p]) return false;
+    return true;
+}
+
+// Whether a self-excitation-only plan needs no work list: sorted times, one size.
+// A device loop over more than kLoopTiles tiles keeps its list: its bands may
+// come to hold every earlier tile, and then largest first counts (16 chains
+// at N = 10,000: 0.86 ms an iteration without, 0.64 with).
+bool Executor::self_listless(const std::vector<SetView>& sets, const int* setOf, int P) const {
+    constexpr int kLoopTiles = 32;
+    const int N = sets[setOf[0]].N;
+    if (shardWorld != 1 || (wideBands_ && N > kLoopTiles * kTile)) return false;
+    for (int p = 0; p < P; ++p)
+        if (!sets[setOf[p]].sorted || sets[setOf[p]].N != N) return false;
     return true;
 }
 
@@ -647,24 +661,17 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // tiles before each strip.  Problems of one size with sorted times need no
     // work list for that: every strip gets the same number of slots, enough for
     // the widest band (the device loop: for every earlier tile), and an item's
-    // tiles follow from its number (SweepProblem::itemsPerProblem).  A slot holds
+    // tiles follow from its number (SweepProblem::slotItems).  A slot holds
     // the tiles that make about four items per resident CTA, at most a whole band.
     selfOnly_ = self_only(P);
     int selfSlots = 0, selfTiles = 1;
-    // A device loop over more than kLoopTiles tiles keeps its list: its bands may
-    // come to hold every earlier tile, and then largest first counts (16 chains
-    // at N = 10,000: 0.86 ms an iteration without, 0.64 with).
-    constexpr int kLoopTiles = 32;
-    bool listless = selfOnly_ && shardWorld == 1 &&
-                    !(wideBands_ && sets[setOf[0]].N > kLoopTiles * kTile);
-    for (int p = 0; p < P && listless; ++p)
-        listless = sets[setOf[p]].sorted && sets[setOf[p]].N == sets[setOf[0]].N;
+    const bool listless = selfOnly_ && self_listless(sets, setOf, P);
     if (listless) {
         const int nTiles = (sets[setOf[0]].N + kTile - 1) / kTile;
         const int nStrips = (sets[setOf[0]].N + stripEvents - 1) / stripEvents;
-        int widest = wideBands_ ? nTiles : 1;
-        double bandTiles = wideBands_ ? (double)P * nStrips * nTiles : 0.0;
-        for (int p = 0; p < P && !wideBands_; ++p) {
+        int widest = 1;
+        double bandTiles = 0.0;
+        for (int p = 0; p < P; ++p) {
             const SetView& s = sets[setOf[p]];
             const StripGaps gap(problem_consts(p));
             StripCursor at;
@@ -677,6 +684,7 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         }
         selfTiles = std::min(widest, std::max(1, (int)std::lround(bandTiles /
                                                                   (4.0 * sweep_grid(r)))));
+        if (wideBands_) widest = nTiles;  // for any sigma and omega
         selfSlots = (widest + selfTiles - 1) / selfTiles;
     }
 
@@ -734,13 +742,15 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         sp.searchBand = (wideBands_ && s.sorted) ? 1 : 0;
         sp.rowOrder = (fp32 && sp.symmetric) ? (r == 2 ? s.dOrder2 : r == 4 ? s.dOrder4 : nullptr)
                                              : nullptr;
-        // the strips' row order is formed when a sweep first needs it
-        bool* ordered = sp.rowOrder ? (r == 2 ? s.ordered2 : s.ordered4) : nullptr;
-        if (ordered && !*ordered) {
+        // the strips' row order is formed when a sweep first needs it, after that
+        // with each upload
+        RowOrder* order = sp.rowOrder ? (r == 2 ? s.order2 : s.order4) : nullptr;
+        if (order) order->wanted = true;
+        if (order && !order->ready) {
             const cudaError_t e = launch_strip_order(D_, N, r, s.dLoc, const_cast<int32_t*>(sp.rowOrder),
                                                      stream_);
             if (e != cudaSuccess) return cuda_fail(e, "strip order");
-            *ordered = true;
+            order->ready = true;
         }
         sp.colAcc = nullptr;
         if (sp.symmetric) {
@@ -788,8 +798,8 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         chunkBase[p] = pl.stripChunks.size();
         if (listless) {
             maxSlots = selfSlots;
-            sp.itemsPerProblem = nStrips * selfSlots;
-            sp.slots = selfSlots;
+            sp.slotItems = P * nStrips;
+            sp.strips = nStrips;
             sp.chunkTiles = selfTiles;
         }
         StripCursor at;
@@ -881,7 +891,7 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // table layout and buffer capacities
     offSP_ = 0;
     offItems_ = align16(offSP_ + sizeof(SweepProblem) * P);
-    const size_t nItems = listless ? (size_t)P * pl.sp[0].itemsPerProblem : pl.items.size();
+    const size_t nItems = listless ? (size_t)selfSlots * pl.sp[0].slotItems : pl.items.size();
     itemsCap_ = std::max(itemsCap_, pl.items.size());
     offNItems_ = align16(offItems_ + sizeof(WorkItem) * itemsCap_);
     offChunks_ = align16(offNItems_ + sizeof(int));
@@ -1081,7 +1091,6 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
             R = r;
             itemsPerSM = it;
             if ((st = build_plan(sets, setOf, params, P, dProbs, r, it))) break;
-            if (plan_.sp[0].itemsPerProblem > 0 && it != its[0]) continue;  // no list: no choice
             const int grid = sweep_grid(r);
             // median of four sweeps after one that warms the caches: the
             // shapes' typical times differ by ~1 %, about as much as the
@@ -1126,7 +1135,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
 }
 
 // R and itemsPerSM for the current kind of plan: fixed by the caller, or tuned
-// the first time the kind runs.  A self-excitation-only sweep of an engine
+// the first time the kind runs with a list.  A self-excitation-only sweep of an engine
 // whose full sweeps are tuned keeps their shape.
 int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
                            const double* params, int P, double* dProbs) {
@@ -1143,6 +1152,14 @@ int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
         // a few thousand events: more, smaller strips fill the SMs
         if (selfOnly_ && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
     }
+    // without a list there is one question left, and the smaller strips answer it:
+    // R = 2 against 4 in FP32 0.125 : 0.155 ms at N = 100k and 1.15 : 1.30 at 400k, R = 1
+    // against 2 in FP64 0.041 : 0.055 ms at N = 30k and 2.12 : 2.09 at 400k
+    if (!s.tuned && selfOnly_ && self_listless(sets, setOf, P)) {
+        R = fixedR ? fixedR : planPrecision_ == HPHC_PRECISION_FP64 ? 1 : 2;
+        itemsPerSM = fixedItems ? fixedItems : 8;
+        return HPHC_OK;
+    }
     if (!s.tuned) {
         const int st = autotune(sets, setOf, params, P, dProbs);
         if (st) return st;
@@ -1155,6 +1172,25 @@ int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
     return HPHC_OK;
 }
 
+// Self-excitation terms an FP64 sweep of the set would evaluate, estimated from
+// sampled tiles.
+double Executor::self_terms(const SetView& s, const double* p) const {
+    ConstsSpec spec = consts_spec(s, p[3]);
+    spec.precision = 0;
+    PairConsts c{};
+    FinishConsts f{};
+    param_consts(p, spec, c, f);
+    if (!s.sorted || !(c.skipS >= 0.0 && c.cW < 0.0)) return 0.5 * s.N * (double)s.N;
+    const double d = c.skipS / -c.cW;
+    const int nTiles = (s.N + kTile - 1) / kTile, step = std::max(1, nTiles / 32);
+    double tiles = 0.0;
+    int n = 0;
+    for (int k = 0; k < nTiles; k += step, ++n)
+        tiles += k + 1 - (std::upper_bound(s.hTileMax, s.hTileMax + k + 1, s.hTileMin[k] - d) -
+                          s.hTileMax);
+    return tiles / n * kTile * s.N;
+}
+
 int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const double* params,
                       int P, double* dProbs) {
     if (P < 1) {
@@ -1163,15 +1199,20 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     }
     plan_grid(sets, setOf, params, P);
     // Large gridded evaluations of the FP32-compensated mode sweep their
-    // self-excitation terms in FP64 too: the grid's sums are exact to 1e-15, and
-    // the sweep's 0.19 instead of 0.13 ms at N = 100k make the whole evaluation so
-    // (log-likelihood 2.7e-11 -> 1.1e-16, worst gradient component 9.6e-10 ->
-    // 3.6e-15 relative).
+    // self-excitation terms in FP64 too, where that is a small part of them: the
+    // grid's sums are exact to 1e-15, and the sweep's 0.19 instead of 0.13 ms at
+    // N = 100k make the whole evaluation so (log-likelihood 2.7e-11 -> 1.1e-16,
+    // worst gradient component 9.6e-10 -> 3.6e-15 relative).  Where the terms are
+    // many they stay in FP32 (N = 500k clustered: 2.2 against 4.1 ms, beside 2.0 ms
+    // of grid kernels).
     planPrecision_ = precision_;
     if (precision_ == HPHC_PRECISION_FP32_COMP && !keptB && self_only(P)) {
         bool large = true;
         for (int p = 0; p < P; ++p)
-            large &= gridShape_[p].order == 16 && sets[setOf[p]].dRecF64 != nullptr;
+            large &= gridShape_[p].order == 16 && sets[setOf[p]].dRecF64 != nullptr &&
+                     self_terms(sets[setOf[p]], params + (size_t)6 * p) * kSelfCostF64 <
+                         0.5 * (gridShape_[p].nodes * kGridCost16.node +
+                                sets[setOf[p]].N * kGridCost16.event);
         if (large) planPrecision_ = HPHC_PRECISION_FP64;
     }
     int st = choose_shape(sets, setOf, params, P, dProbs);
@@ -1338,14 +1379,14 @@ void Executor::count_terms(const std::vector<SetView>& sets, double* bTerms, dou
     double nb = 0.0, ns = 0.0, ne = 0.0;
     const int stripEvents = kSweepThreads * R;
     std::vector<WorkItem> listless;  // the items of a plan without a list (see work_item)
-    for (int p = 0; p < plan_.P && plan_.sp[p].itemsPerProblem > 0; ++p) {
+    for (int p = 0; p < plan_.P && plan_.sp[p].slotItems > 0; ++p) {
         const SweepProblem& sp = plan_.sp[p];
-        for (int k = 0; k < sp.itemsPerProblem; ++k) {
+        for (int k = 0; k < sp.strips * plan_.fp[p].slots; ++k) {
             WorkItem w{};
             w.problem = p;
-            w.strip = k / sp.slots;
+            w.strip = k % sp.strips;
             w.jt1 = std::max(0, std::min((w.strip + 1) * R, sp.nTiles) -
-                                    k % sp.slots * sp.chunkTiles);
+                                    k / sp.strips * sp.chunkTiles);
             w.jt0 = std::max(0, w.jt1 - sp.chunkTiles);
             listless.push_back(w);
         }

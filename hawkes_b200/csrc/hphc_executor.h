@@ -27,6 +27,11 @@
 
 namespace hphc {
 
+// Whether a strip row order holds the present events', and whether sweeps use it.
+struct RowOrder {
+    bool ready = false, wanted = false;
+};
+
 // An event set resident on the device, with host copies used for planning.
 struct SetView {
     int N = 0;
@@ -35,8 +40,8 @@ struct SetView {
     const int32_t* dRanks = nullptr;   // dense time ranks (FP32 mode)
     const int32_t* dOrder2 = nullptr;  // spatial row order of strips of R = 2 and 4 (FP32
     const int32_t* dOrder4 = nullptr;  //   mode, launch_strip_order), or null
-    bool* ordered2 = nullptr;          // whether they hold the present events' order
-    bool* ordered4 = nullptr;
+    RowOrder* order2 = nullptr;        // their state
+    RowOrder* order4 = nullptr;
     const double* dRecF64 = nullptr;   // FP64 records (FP64 mode; large FP32-compensated sets)
     bool* packedF64 = nullptr;         // FP32-compensated: whether they hold the present events
     const double* dTileMin = nullptr;  // per-tile time bounds
@@ -227,7 +232,9 @@ private:
     void plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
                    int P);
     double* grid_sums(int p) const;
-    bool self_only(int P) const;  // no problem of the plan has background terms to sweep
+    double self_terms(const SetView& s, const double* p) const;
+    bool self_only(int P) const;
+    bool self_listless(const std::vector<SetView>& sets, const int* setOf, int P) const;  // no problem of the plan has background terms to sweep
     int choose_shape(const std::vector<SetView>& sets, const int* setOf, const double* params,
                      int P, double* dProbs);
     int launch_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,

@@ -407,10 +407,11 @@ struct SweepProblem {
     // bisection on the tile time bounds instead of scanning to it.
     int searchBand;
     // Self-excitation-only plans of problems with sorted times and one size
-    // carry no work list: item k of the launch is problem k / itemsPerProblem,
-    // there strip (k % itemsPerProblem) / slots, and of that strip's tiles, counted
-    // back from its own last one, the chunkTiles of slot k % slots.
-    int itemsPerProblem, slots, chunkTiles;
+    // carry no work list: item k of the launch is slot k / slotItems (all strips of
+    // all problems), there problem (k % slotItems) / strips and its strip, and of
+    // that strip's tiles, counted back from its own last one, the chunkTiles of the
+    // slot.
+    int slotItems, strips, chunkTiles;
     // FP32 sweep: event of row r of thread t of a full strip, at
     // [stripBase + r * 128 + t] (launch_strip_order for the sweep's R), or
     // null for the identity order.

@@ -344,6 +344,21 @@ __device__ __forceinline__ int first_tile_with_terms(const SweepProblem& P, int 
     return lo;
 }
 
+// Whether a self-excitation-only item holds no term; its sums are zeros then.
+__device__ __forceinline__ bool empty_self_item(const double* __restrict__ tileMin,
+                                                const double* __restrict__ tileMax,
+                                                const PairConsts& c, int ts0, int ts1, int jt0,
+                                                int jt1) {
+    double tminI = INFINITY, tmaxI = -INFINITY;
+    for (int t = ts0; t < ts1; ++t) {
+        tminI = fmin(tminI, tileMin[t]);
+        tmaxI = fmax(tmaxI, tileMax[t]);
+    }
+    for (int jt = jt0; jt < jt1; ++jt)
+        if (tile_mode(tminI, tmaxI, tileMin[jt], tileMax[jt], c).doS) return false;
+    return true;
+}
+
 // One work item of the FP64 sweep: target strip `strip` (kSweepThreads * R
 // events) against j tiles [jt0, jt1); unit pair sums to partial slot `slot`.
 // sym: tiles before the strip are evaluated once per pair (rows + columns).
@@ -363,6 +378,16 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
     const int stripBase = strip * kSweepThreads * R;
     const int ts0 = stripBase / kTile, ts1 = min(ts0 + R, nTiles);
 
+    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, jt0, jt1)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = stripBase + r * kSweepThreads + tid;
+            if (i < N)
+                for (int q = 3; q < kNumAcc; ++q)
+                    partials[((size_t)slot * kNumAcc + q) * Npad + i] = 0.0;
+        }
+        return;
+    }
     const double table = exp_table_lane();
     double xi[R][D], ti[R];
 #pragma unroll
@@ -495,19 +520,19 @@ __device__ __forceinline__ int next_item(int* counter, int* sNext) {
 }
 
 // Item `it` of a launch: from the list, or (SELF) from its number where the
-// problems carry no list.  A slot before the first tile is empty: its sums are
-// written as zeros.
+// problems carry no list: slot by slot, so that the items nearest the diagonal,
+// which hold terms, come first and the empty ones of wide plans fill the end.
 template <bool SELF, int R>
 __device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ problems,
                                               const WorkItem* __restrict__ items, int it) {
-    if (!SELF || problems[0].itemsPerProblem == 0) return items[it];
-    const int per = problems[0].itemsPerProblem;
+    if (!SELF || problems[0].slotItems == 0) return items[it];
     WorkItem w;
-    w.problem = it / per;
+    const int perSlot = problems[0].slotItems;
+    w.slot = it / perSlot;
+    const int k = it - w.slot * perSlot;
+    w.problem = k / problems[0].strips;
     const SweepProblem& P = problems[w.problem];
-    const int k = it - w.problem * per;
-    w.strip = k / P.slots;
-    w.slot = k - w.strip * P.slots;
+    w.strip = k - w.problem * P.strips;
     w.jt1 = max(0, min((w.strip + 1) * R, P.nTiles) - w.slot * P.chunkTiles);
     w.start = w.jt0 = max(0, w.jt1 - P.chunkTiles);
     if (P.searchBand && w.jt1 - w.jt0 > 2)
@@ -1012,6 +1037,16 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
     const int tid = threadIdx.x;
     const int stripBase = strip * kSweepThreads * R;
     const int ts0 = stripBase / kTile, ts1 = min(ts0 + R, nTiles);
+    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, jt0, jt1)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = stripBase + r * kSweepThreads + tid;
+            if (i < N)
+                for (int q = 3; q < kNumAcc; ++q)
+                    partials[((size_t)slot * kNumAcc + q) * Npad + i] = 0.0;
+        }
+        return;
+    }
     // full strips read their rows through the spatial row order
     const bool ordered = rowOrder != nullptr && stripBase + kSweepThreads * R <= N;
 
