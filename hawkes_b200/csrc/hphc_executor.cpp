@@ -664,7 +664,30 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // tiles follow from its number (SweepProblem::slotItems).  A slot holds
     // the tiles that make about four items per resident CTA, at most a whole band.
     selfOnly_ = self_only(P);
-    int selfSlots = 0, selfTiles = 1;
+    int selfSlots = 0, selfTiles = 1, selfShift = 0;
+    // Small plans take their tiles in halves or quarters (WorkItem::cols), so that
+    // every SM has an item and the time of one is less (N = 1000 FP64 sweep 46 -> 23
+    // us, whole evaluation 71 -> 53): not in a fixed shape or a shard, whose sums are
+    // compared, and not in the plain FP32 mode, where an item's length shows in the
+    // sums' rounding.
+    const bool partTiles = shardWorld == 1 && !(fixedR && fixedItems) && !(variant_ & 8);
+    const auto part_shift = [&](double tiles) {  // log2 of the parts of items of so many tiles
+        return !partTiles || tiles > 0.5 ? 0 : tiles > 0.25 ? 1 : 2;
+    };
+    // In the list form all problems take the same, from the largest.  The last
+    // digits of FP32-compensated row sums show an item's length, so there the sizes
+    // alone decide for up to eight problems (chunks of one tile too), whose results
+    // then equal single evaluations'; more fill the SMs with whole tiles (64 problems
+    // of N = 2000: 0.172 ms, in quarters 0.180).
+    int partShift = 0;
+    bool oneTile = false;
+    if (!wideBands_) {
+        int most = 1;
+        for (int p = 0; p < P; ++p) most = std::max(most, (sets[setOf[p]].N + kTile - 1) / kTile);
+        if (!fp32) partShift = part_shift((double)most / nChunksTarget);
+        else if (P <= 8) partShift = part_shift(most / 64.0);
+        oneTile = fp32 && partShift > 0;
+    }
     const bool listless = selfOnly_ && self_listless(sets, setOf, P);
     if (listless) {
         const int nTiles = (sets[setOf[0]].N + kTile - 1) / kTile;
@@ -682,10 +705,14 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
                 bandTiles += hi - lo;
             }
         }
-        selfTiles = std::min(widest, std::max(1, (int)std::lround(bandTiles /
-                                                                  (4.0 * sweep_grid(r)))));
-        if (wideBands_) widest = nTiles;  // for any sigma and omega
-        selfSlots = (widest + selfTiles - 1) / selfTiles;
+        const double perItem = bandTiles / (4.0 * sweep_grid(r));
+        selfTiles = std::min(widest, std::max(1, (int)std::lround(perItem)));
+        selfShift = part_shift(perItem);
+        if (wideBands_) {  // for any sigma and omega
+            widest = nTiles;
+            selfShift = part_shift((double)P * nStrips * nTiles / (4.0 * sweep_grid(r)));
+        }
+        selfSlots = (widest + selfTiles - 1) / selfTiles << selfShift;
     }
 
     size_t recOff = 0, partOff = 0, colOff = 0;
@@ -709,8 +736,8 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         const int nStrips = (N + stripEvents - 1) / stripEvents;
         const int Npad = nStrips * stripEvents;
         // tiles a chunk, from the tuned items per SM
-        const int generalCT = std::max(1, (nTiles + nChunksTarget - 1) / nChunksTarget);
-        const int CT = generalCT;
+        const int CT =
+            oneTile ? 1 : std::max(1, (nTiles + nChunksTarget - 1) / nChunksTarget);
         int maxSlots = 1;  // partial-sum slots the widest strip band uses
         pl.maxN = std::max(pl.maxN, N);
         SweepProblem& sp = pl.sp[p];
@@ -796,6 +823,7 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
 
         // work items: each strip's band of tiles that may hold a non-zero term
         chunkBase[p] = pl.stripChunks.size();
+        sp.partShift = listless ? selfShift : partShift;
         if (listless) {
             maxSlots = selfSlots;
             sp.slotItems = P * nStrips;
@@ -821,11 +849,12 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
                 w.jt1 = std::min(hi, (c + 1) * CT);
                 w.slot = c - cFirst;
                 w.start = w.jt0;
+                w.cols = kTile;
                 pl.items.push_back(w);
                 itemCost.push_back(item_cost(sc, sp.c.noB != 0, w.jt0, w.jt1));
             }
-            pl.stripChunks.push_back(cLast - cFirst);
-            maxSlots = std::max(maxSlots, cLast - cFirst);
+            pl.stripChunks.push_back((cLast - cFirst) << partShift);
+            maxSlots = std::max(maxSlots, (cLast - cFirst) << partShift);
         }
         // partial sums: as many slots per strip as the widest band uses
         sp.partials = reinterpret_cast<double*>(partOff);  // offset, fixed up later
@@ -891,7 +920,8 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     // table layout and buffer capacities
     offSP_ = 0;
     offItems_ = align16(offSP_ + sizeof(SweepProblem) * P);
-    const size_t nItems = listless ? (size_t)selfSlots * pl.sp[0].slotItems : pl.items.size();
+    const size_t nItems =
+        listless ? (size_t)selfSlots * pl.sp[0].slotItems : pl.items.size() << partShift;
     itemsCap_ = std::max(itemsCap_, pl.items.size());
     offNItems_ = align16(offItems_ + sizeof(WorkItem) * itemsCap_);
     offChunks_ = align16(offNItems_ + sizeof(int));
@@ -1092,7 +1122,8 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
             itemsPerSM = it;
             if ((st = build_plan(sets, setOf, params, P, dProbs, r, it))) break;
             const int grid = sweep_grid(r);
-            // median of four sweeps after one that warms the caches: the
+            // sweep and finish, whose work grows with the number of items;
+            // median of four after one that warms the caches: the
             // shapes' typical times differ by ~1 %, about as much as the
             // best of a few launches varies
             float times[kTuneReps];
@@ -1101,7 +1132,7 @@ int Executor::autotune(const std::vector<SetView>& sets, const int* setOf, const
                 if ((st = launch_sequence(grid))) break;
                 cudaError_t e = cudaStreamSynchronize(stream_);
                 float t = 0.f;
-                if (e == cudaSuccess) e = cudaEventElapsedTime(&t, ev_[1], ev_[2]);
+                if (e == cudaSuccess) e = cudaEventElapsedTime(&t, ev_[1], ev_[3]);
                 if (e != cudaSuccess) {
                     st = cuda_fail(e, "autotune timing");
                     break;
@@ -1385,8 +1416,10 @@ void Executor::count_terms(const std::vector<SetView>& sets, double* bTerms, dou
             WorkItem w{};
             w.problem = p;
             w.strip = k % sp.strips;
-            w.jt1 = std::max(0, std::min((w.strip + 1) * R, sp.nTiles) -
-                                    k / sp.strips * sp.chunkTiles);
+            const int slot = k / sp.strips, at = slot >> sp.partShift;
+            w.cols = kTile >> sp.partShift;
+            w.col0 = (slot - (at << sp.partShift)) * w.cols;
+            w.jt1 = std::max(0, std::min((w.strip + 1) * R, sp.nTiles) - at * sp.chunkTiles);
             w.jt0 = std::max(0, w.jt1 - sp.chunkTiles);
             listless.push_back(w);
         }
@@ -1407,7 +1440,7 @@ void Executor::count_terms(const std::vector<SetView>& sets, double* bTerms, dou
             bool b, se;
             tile_needs(tminI, tmaxI, s.hTileMin[jt], s.hTileMax[jt], c, &b, &se);
             if (sym && jt >= ts1) b = false;
-            const double nj = std::min(kTile, s.N - jt * kTile);
+            const double nj = std::max(0, std::min(w.cols, s.N - jt * kTile - w.col0));
             if (b) {
                 // a symmetric tile also accounts for the pairs' other order
                 nb += (sym && jt < ts0 ? 2.0 : 1.0) * ni * nj;

@@ -580,6 +580,7 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
     const FinishConsts f = P.f;
     const int N = P.N;
     const int i = fb.i0 + threadIdx.x;
+    double ti = 0.0;
     double v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = 0.0;
@@ -588,27 +589,49 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
     for (int q = 0; q < kNumAcc; ++q) s[q] = 0.0;
     if (i < N) {
         const int nc = P.stripChunks ? P.stripChunks[i / P.stripEvents] : P.slots;
+        const bool kept = P.keptB != nullptr;
+        // all loads that do not depend on another go first: small problems' blocks
+        // wait for nothing else
+        ti = P.times[i];
+        unsigned long long hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
+        double sums[kNumAcc];
+#pragma unroll
+        for (int q = 0; q < kNumAcc; ++q) sums[q] = 0.0;
+        if (kept) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) sums[q] = P.keptB[(size_t)q * N + i];
+        } else if (P.colAcc) {
+            unsigned long long* w = P.colAcc + i;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const size_t at = (size_t)(P.colWords * q) * P.Npad;
+                hi[q] = w[at];
+                w[at] = 0;
+                if (P.colWords == 2) {
+                    lo[q] = w[at + P.Npad];
+                    w[at + P.Npad] = 0;
+                }
+            }
+        }
+        const double* at = P.partials + i;
+#pragma unroll 8
+        for (int ch = 0; ch < nc; ++ch, at += (size_t)kNumAcc * P.Npad)
+#pragma unroll
+            for (int q = 0; q < kNumAcc; ++q)
+                if (q >= 3 || !kept) sums[q] += at[(size_t)q * P.Npad];
 #pragma unroll
         for (int q = 0; q < kNumAcc; ++q) {
-            if (q < 3 && P.keptB) {
-                s[q] = P.keptB[(size_t)q * N + i];  // unchanged: not written back
+            if (q < 3 && kept) {
+                s[q] = sums[q];  // unchanged: not written back
                 continue;
             }
-            double acc = 0.0;
-            for (int ch = 0; ch < nc; ++ch)
-                acc += P.partials[((size_t)ch * kNumAcc + q) * P.Npad + i];
+            double acc = sums[q];
             if (q < 3 && P.colAcc) {
-                if (P.colWords == 2) {  // FP64 sweep: two-word fixed point
-                    unsigned long long* hi = P.colAcc + (size_t)(2 * q) * P.Npad + i;
-                    unsigned long long* lo = hi + P.Npad;
-                    acc += ldexp((double)*hi, -P.colShift[q]) +
-                           ldexp((double)*lo, -(P.colShift[q] + kColLoBits));
-                    *hi = *lo = 0;
-                } else {
-                    unsigned long long* w = P.colAcc + (size_t)q * P.Npad + i;
-                    acc += (double)*w * kColInv;
-                    *w = 0;
-                }
+                if (P.colWords == 2)  // FP64 sweep: two-word fixed point
+                    acc += ldexp((double)hi[q], -P.colShift[q]) +
+                           ldexp((double)lo[q], -(P.colShift[q] + kColLoBits));
+                else
+                    acc += (double)hi[q] * kColInv;
             }
             s[q] = acc * f.accScale[q];
         }
@@ -658,7 +681,7 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
 #pragma unroll
             for (int q = 0; q < kNumAcc; ++q)
                 if (q >= 3 || !P.keptB) P.sums[(size_t)q * N + i] = s[q];
-        event_contributions(f, s, P.times[i], v, P.probs ? P.probs + i : nullptr);
+        event_contributions(f, s, ti, v, P.probs ? P.probs + i : nullptr);
     }
     block_sum<8, kFinishThreads>(v);
     if (finish_total(v, blockSums, blockIdx.x, P.blockBase, P.nBlocks, arrived + 1 + fb.problem,

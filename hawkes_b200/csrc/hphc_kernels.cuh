@@ -412,6 +412,7 @@ struct SweepProblem {
     // that strip's tiles, counted back from its own last one, the chunkTiles of the
     // slot.
     int slotItems, strips, chunkTiles;
+    int partShift;  // log2 of the items a tile's columns are split over
     // FP32 sweep: event of row r of thread t of a full strip, at
     // [stripBase + r * 128 + t] (launch_strip_order for the sweep's R), or
     // null for the identity order.
@@ -425,9 +426,12 @@ struct SweepProblem {
 // counter, so slow and fast items balance across SMs, and every item writes
 // fixed slots, so results do not depend on which CTA ran it.  The sweep
 // starts at tile `start`: jt0, or in the device-resident loop the first tile
-// not ruled out by its time gap for the current constants (band_starts).
+// not ruled out by its time gap for the current constants (band_starts).  Of
+// each tile it takes columns [col0, col0 + cols): all kTile, or a half or a
+// quarter in plans with few items (SweepProblem::partShift: a list entry and its slot
+// then stand for that many items).
 struct WorkItem {
-    int problem, strip, jt0, jt1, slot, start, pad1, pad2;
+    int problem, strip, jt0, jt1, slot, start, col0, cols;
 };
 
 constexpr int kBandThreads = 256;

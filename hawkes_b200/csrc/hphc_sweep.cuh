@@ -238,14 +238,15 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
                                              const PairConsts& c, double (&acc)[R][kNumAcc],
                                              double* __restrict__ sCol,
                                              unsigned long long* __restrict__ colAcc, int Npad,
-                                             int j0, const int (&shift)[3], double table) {
+                                             int j0, int nj, const int (&shift)[3],
+                                             double table) {
     static_assert(kSweepThreads == kTile, "one column per thread in the column flush");
     constexpr int S = Layout<D>::kF64Stride;
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int p = (lane >> 3) & 3;
 #pragma unroll 1
-    for (int g = 0; g < kTile; g += kSymGroup64) {
+    for (int g = 0; g < nj; g += kSymGroup64) {
         double cp[3][kSymGroup64];
 #pragma unroll
         for (int m = 0; m < kSymGroup64; ++m) {
@@ -303,6 +304,7 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
         }
     }
     __syncthreads();
+    if (tid >= nj) return;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         double v = 0.0;
@@ -359,8 +361,8 @@ __device__ __forceinline__ bool empty_self_item(const double* __restrict__ tileM
     return true;
 }
 
-// One work item of the FP64 sweep: target strip `strip` (kSweepThreads * R
-// events) against j tiles [jt0, jt1); unit pair sums to partial slot `slot`.
+// One work item of the FP64 sweep: target strip item.strip (kSweepThreads * R
+// events) against j tiles [start, jt1); unit pair sums to partial slot item.slot.
 // sym: tiles before the strip are evaluated once per pair (rows + columns).
 // SELF: a self-excitation-only sweep (every problem has noB), with the
 // background's code and sums compiled out.
@@ -369,22 +371,23 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
                                          const double* __restrict__ tileMin,
                                          const double* __restrict__ tileMax,
                                          double* __restrict__ partials, int N, int nTiles,
-                                         int Npad, const PairConsts& c, int strip, int jt0,
-                                         int jt1, int slot, double* sRec, bool sym,
+                                         int Npad, const PairConsts& c,
+                                         const WorkItem& item, double* sRec, bool sym,
                                          unsigned long long* __restrict__ colAcc,
                                          const int (&shift)[3], double* sCol) {
     constexpr int S = Layout<D>::kF64Stride;
     const int tid = threadIdx.x;
-    const int stripBase = strip * kSweepThreads * R;
+    const int stripBase = item.strip * kSweepThreads * R;
     const int ts0 = stripBase / kTile, ts1 = min(ts0 + R, nTiles);
+    const int jt1 = item.jt1;
 
-    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, jt0, jt1)) {
+    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, item.start, jt1)) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int i = stripBase + r * kSweepThreads + tid;
             if (i < N)
                 for (int q = 3; q < kNumAcc; ++q)
-                    partials[((size_t)slot * kNumAcc + q) * Npad + i] = 0.0;
+                    partials[((size_t)item.slot * kNumAcc + q) * Npad + i] = 0.0;
         }
         return;
     }
@@ -416,12 +419,13 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
 #pragma unroll
         for (int q = 0; q < kNumAcc; ++q) acc[r][q] = 0.0;
 
-    for (int jt = jt0; jt < jt1; ++jt) {
+    for (int jt = item.start; jt < jt1; ++jt) {
         TileMode m = tile_mode(tminI, tmaxI, tileMin[jt], tileMax[jt], c);
         if (SELF || (sym && jt >= ts1)) m.doB = false;  // sym: as columns by later strips
         if (!m.doB && !m.doS) continue;
-        const int j0 = jt * kTile;
-        const int nj = min(kTile, N - j0);
+        const int j0 = jt * kTile + item.col0;
+        const int nj = min(item.cols, N - j0);
+        if (nj <= 0) continue;  // a part beyond the last event
         __syncthreads();
         const double2* src = reinterpret_cast<const double2*>(rec + (size_t)j0 * S);
         double2* dst = reinterpret_cast<double2*>(sRec);
@@ -448,10 +452,10 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         } else if (sym && m.doB && jt < ts0 && m.fastB) {
             if (!m.doS)
                 tile_sym_f64<D, R, false, false, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad,
-                                                       j0, shift, table);
+                                                       j0, nj, shift, table);
             else
                 tile_sym_f64<D, R, true, false, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad,
-                                                      j0, shift, table);
+                                                      j0, nj, shift, table);
         } else if (m.doB && m.fastB && !(sym && jt < ts0)) {
             if (!m.doS)
                 body_f64<D, R, true, false, false, true>(sRec, nj, xi, ti, c, acc, table);
@@ -460,14 +464,11 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         } else if (sym && m.doB && jt < ts0) {
             // jt < ts0 <= nTiles - 1: a full tile
             if (!m.doS)
-                tile_sym_f64<D, R, false, false>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0,
-                                                 shift, table);
+                tile_sym_f64<D, R, false, false>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0, nj, shift, table);
             else if (m.allCausal)
-                tile_sym_f64<D, R, true, false>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0,
-                                                shift, table);
+                tile_sym_f64<D, R, true, false>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0, nj, shift, table);
             else
-                tile_sym_f64<D, R, true, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0,
-                                               shift, table);
+                tile_sym_f64<D, R, true, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad, j0, nj, shift, table);
         } else if (m.doB) {
             if (!m.doS)
                 body_f64<D, R, true, false, false>(sRec, nj, xi, ti, c, acc, table);
@@ -490,7 +491,7 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
             for (int q = 0; q < kNumAcc; ++q)
                 // a self-excitation-only sweep leaves the background rows to
                 // the kept sums: they are neither written nor read
-                if (q >= 3 || (!SELF && !c.noB)) partials[((size_t)slot * kNumAcc + q) * Npad + i] = acc[r][q];
+                if (q >= 3 || (!SELF && !c.noB)) partials[((size_t)item.slot * kNumAcc + q) * Npad + i] = acc[r][q];
         }
     }
 }
@@ -504,19 +505,14 @@ sweep_f64_kernel(SweepGeometry g, const double* __restrict__ rec,
     __shared__ __align__(16) double sRec[kTile * Layout<D>::kF64Stride];
     const int strip = blockIdx.x / g.nChunks;
     const int chunk = blockIdx.x - strip * g.nChunks;
-    const int jt0 = chunk * g.chunkTiles;
-    const int jt1 = min(jt0 + g.chunkTiles, g.nTiles);
+    WorkItem w{};
+    w.strip = strip;
+    w.jt0 = w.start = chunk * g.chunkTiles;
+    w.jt1 = min(w.start + g.chunkTiles, g.nTiles);
+    w.slot = chunk;
+    w.cols = kTile;
     const int noShift[3] = {0, 0, 0};
-    f64_item<D, R>(rec, tileMin, tileMax, partials, g.N, g.nTiles, g.Npad, c, strip, jt0, jt1,
-                   chunk, sRec, false, nullptr, noShift, nullptr);
-}
-
-// Takes the next work-list index for the CTA (all threads get the same one).
-__device__ __forceinline__ int next_item(int* counter, int* sNext) {
-    __syncthreads();
-    if (threadIdx.x == 0) *sNext = atomicAdd(counter, 1);
-    __syncthreads();
-    return *sNext;
+    f64_item<D, R>(rec, tileMin, tileMax, partials, g.N, g.nTiles, g.Npad, c, w, sRec, false, nullptr, noShift, nullptr);
 }
 
 // Item `it` of a launch: from the list, or (SELF) from its number where the
@@ -525,7 +521,15 @@ __device__ __forceinline__ int next_item(int* counter, int* sNext) {
 template <bool SELF, int R>
 __device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ problems,
                                               const WorkItem* __restrict__ items, int it) {
-    if (!SELF || problems[0].slotItems == 0) return items[it];
+    if (!SELF || problems[0].slotItems == 0) {
+        const int shift = problems[0].partShift;
+        WorkItem w = items[it >> shift];
+        const int part = it & ((1 << shift) - 1);
+        w.slot = (w.slot << shift) + part;
+        w.cols = kTile >> shift;
+        w.col0 = part * w.cols;
+        return w;
+    }
     WorkItem w;
     const int perSlot = problems[0].slotItems;
     w.slot = it / perSlot;
@@ -533,11 +537,32 @@ __device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ p
     w.problem = k / problems[0].strips;
     const SweepProblem& P = problems[w.problem];
     w.strip = k - w.problem * P.strips;
-    w.jt1 = max(0, min((w.strip + 1) * R, P.nTiles) - w.slot * P.chunkTiles);
+    const int at = w.slot >> P.partShift;
+    w.cols = kTile >> P.partShift;
+    w.col0 = (w.slot - (at << P.partShift)) * w.cols;
+    w.jt1 = max(0, min((w.strip + 1) * R, P.nTiles) - at * P.chunkTiles);
     w.start = w.jt0 = max(0, w.jt1 - P.chunkTiles);
     if (P.searchBand && w.jt1 - w.jt0 > 2)
         w.start = first_tile_with_terms(P, R, w.strip, w.jt0, w.jt1);
     return w;
+}
+
+// The CTA's next item, if there is one, into shared memory: its fields are read
+// where they are used, so that they take no registers through the pair loops.
+// The first is the CTA's own number, the others come from the counter (740 CTAs
+// that begin with an atomic on one address cost 4 us: N = 500 FP64 sweep 16 -> 12).
+template <bool SELF, int R>
+__device__ __forceinline__ bool next_item(const SweepProblem* __restrict__ problems,
+                                          const WorkItem* __restrict__ items, int n, int* counter,
+                                          bool first, WorkItem& item) {
+    if (!first) __syncthreads();
+    if (threadIdx.x == 0) {
+        const int it = first ? blockIdx.x : gridDim.x + atomicAdd(counter, 1);
+        if (it < n) item = work_item<SELF, R>(problems, items, it);
+        else item.problem = -1;
+    }
+    __syncthreads();
+    return item.problem >= 0;
 }
 
 // Work-list form: persistent CTAs take items until the list is exhausted.
@@ -551,17 +576,15 @@ sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
                       int* __restrict__ counter) {
     __shared__ __align__(16) double sRec[kTile * Layout<D>::kF64Stride];
     __shared__ __align__(16) double sCol[SELF ? 2 : (kSweepThreads / 32) * 3 * kTile];
-    __shared__ int sNext;
+    __shared__ WorkItem w;
     const int n = *nItems;
-    for (;;) {
-        const int it = next_item(counter, &sNext);
-        if (it >= n) break;
-        const WorkItem w = work_item<SELF, R>(problems, items, it);
+    for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
+         first = false) {
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         const int shift[3] = {P.colShift[0], P.colShift[1], P.colShift[2]};
         f64_item<D, R, SELF>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
-                       P.nTiles, P.Npad, c, w.strip, w.start, w.jt1, w.slot, sRec,
+                       P.nTiles, P.Npad, c, w, sRec,
                        P.symmetric != 0, P.colAcc, shift, sCol);
     }
 }
@@ -964,14 +987,15 @@ __device__ __forceinline__ void sym_group_f32(const StagedTile<D>& t, int g, int
     }
 }
 
-// One full tile J (kTile columns, all real events) before the strip.
+// A full tile J, or nj columns of it (all real events, nj a multiple of the
+// group), before the strip.
 // sCol: [kSweepThreads / 32][3][kTile] floats of shared memory.
 template <int D, int R, int V, int VB, bool FAR, bool DO_S, bool MASK>
 __device__ __forceinline__ void tile_sym_f32(const StagedTile<D>& t, const Rows2<D, R>& w,
                                              const PairConsts& c, RowSums<R>& a,
                                              float* __restrict__ sCol,
                                              unsigned long long* __restrict__ colAcc, int Npad,
-                                             int j0) {
+                                             int j0, int nj) {
     static_assert(kSweepThreads == kTile, "one column per thread in the column flush");
     static_assert(kTile % kSymGroup == 0, "group sizes");
     const int tid = threadIdx.x;
@@ -979,7 +1003,7 @@ __device__ __forceinline__ void tile_sym_f32(const StagedTile<D>& t, const Rows2
     const int q = (lane >> 3) & 3;
     const bool hi = (lane >> 2) & 1;
 #pragma unroll 1
-    for (int g = 0; g < kTile; g += kSymGroup) {
+    for (int g = 0; g < nj; g += kSymGroup) {
         float2 cp[3][kSymGroup / 2];
         sym_group_f32<D, R, V, VB, FAR, DO_S, MASK>(t, g, q, w, c, a, cp);
         const float c0 = sym_exchange(cp[0], hi);
@@ -993,6 +1017,7 @@ __device__ __forceinline__ void tile_sym_f32(const StagedTile<D>& t, const Rows2
         }
     }
     __syncthreads();
+    if (tid >= nj) return;
 #pragma unroll
     for (int qq = 0; qq < 3; ++qq) {
         double v = 0.0;
@@ -1030,20 +1055,20 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
                                           double* __restrict__ partials,
                                           unsigned long long* __restrict__ colAcc, int N,
                                           int nTiles, int Npad, bool sym, const PairConsts& c,
-                                          int strip, int jt0, int jt1, int slot,
-                                          const int32_t* __restrict__ rowOrder,
+                                          const WorkItem& item, const int32_t* __restrict__ rowOrder,
                                           StagedTile<D>& st, float* sCol) {
     constexpr int S = Layout<D>::kF32Stride;
     const int tid = threadIdx.x;
-    const int stripBase = strip * kSweepThreads * R;
+    const int stripBase = item.strip * kSweepThreads * R;
     const int ts0 = stripBase / kTile, ts1 = min(ts0 + R, nTiles);
-    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, jt0, jt1)) {
+    const int jt1 = item.jt1;
+    if (SELF && empty_self_item(tileMin, tileMax, c, ts0, ts1, item.start, jt1)) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int i = stripBase + r * kSweepThreads + tid;
             if (i < N)
                 for (int q = 3; q < kNumAcc; ++q)
-                    partials[((size_t)slot * kNumAcc + q) * Npad + i] = 0.0;
+                    partials[((size_t)item.slot * kNumAcc + q) * Npad + i] = 0.0;
         }
         return;
     }
@@ -1085,15 +1110,16 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
     RowSums<R> acc;
     start_rows<R>(acc, c);
 
-    for (int jt = jt0; jt < jt1; ++jt) {
+    for (int jt = item.start; jt < jt1; ++jt) {
         TileMode m = tile_mode(tminI, tmaxI, tileMin[jt], tileMax[jt], c);
         // plain FP32: causal only where the FP32-rounded times differ, so a
         // tile pair with equal rounded bounds keeps the rank mask
         if (V & kPlain) m.allCausal = m.allCausal && (float)tminI > (float)tileMax[jt];
         if (SELF || (sym && jt >= ts1)) m.doB = false;  // sym: as columns by later strips
         if (!m.doB && !m.doS) continue;
-        const int j0 = jt * kTile;
-        const int nj = min(kTile, N - j0);
+        const int j0 = jt * kTile + item.col0;
+        const int nj = min(item.cols, N - j0);
+        if (nj <= 0) continue;  // a part beyond the last event
         __syncthreads();
         // stage the tile: one thread per column, fields negated
         if (tid < nj) {
@@ -1141,19 +1167,19 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
             // jt < ts0 <= nTiles - 1: a full tile
             if (m.fastB && !m.doS)
                 tile_sym_f32<D, R, VG, VF, true, false, false>(st, w, c, acc, sCol, colAcc, Npad,
-                                                               j0);
+                                                               j0, nj);
             else if (m.fastB)
                 tile_sym_f32<D, R, VG, VF, true, true, false>(st, w, c, acc, sCol, colAcc, Npad,
-                                                              j0);
+                                                              j0, nj);
             else if (!m.doS)
                 tile_sym_f32<D, R, V, V, false, false, false>(st, w, c, acc, sCol, colAcc, Npad,
-                                                              j0);
+                                                              j0, nj);
             else if (m.allCausal)
                 tile_sym_f32<D, R, V, V, false, true, false>(st, w, c, acc, sCol, colAcc, Npad,
-                                                             j0);
+                                                             j0, nj);
             else
                 tile_sym_f32<D, R, V, V, false, true, true>(st, w, c, acc, sCol, colAcc, Npad,
-                                                            j0);
+                                                            j0, nj);
         } else if (m.doB) {
             if (m.fastB && !m.doS)
                 tile_f32<D, R, VG, VF, true, true, false, false>(st, nj, w, c, acc);
@@ -1183,7 +1209,7 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
                 // a self-excitation-only sweep leaves the background rows to
                 // the kept sums: they are neither written nor read
                 if (q >= 3 || (!SELF && !c.noB))
-                    partials[((size_t)slot * kNumAcc + q) * Npad + i] =
+                    partials[((size_t)item.slot * kNumAcc + q) * Npad + i] =
                         (((double)acc.hi[r][q].x - (double)c.rowOffset[q]) +
                          ((double)acc.hi[r][q].y - (double)c.rowOffset[q])) +
                         ((double)acc.lo[r][q].x + (double)acc.lo[r][q].y);
@@ -1202,17 +1228,14 @@ sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
                        int* __restrict__ counter) {
     __shared__ __align__(16) StagedTile<D> sTile;
     __shared__ __align__(16) float sCol[SELF ? 4 : (kSweepThreads / 32) * 3 * kTile];
-    __shared__ int sNext;
+    __shared__ WorkItem w;
     const int n = *nItems;
-    for (;;) {
-        const int it = next_item(counter, &sNext);
-        if (it >= n) break;
-        const WorkItem w = work_item<SELF, R>(problems, items, it);
+    for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
+         first = false) {
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         f32c_item<D, R, V, SELF>(static_cast<const float*>(P.rec), P.tileMin, P.tileMax, P.partials,
-                           P.colAcc, P.N, P.nTiles, P.Npad, P.symmetric != 0, c, w.strip, w.start,
-                           w.jt1, w.slot, P.rowOrder, sTile, sCol);
+                           P.colAcc, P.N, P.nTiles, P.Npad, P.symmetric != 0, c, w, P.rowOrder, sTile, sCol);
     }
 }
 
