@@ -314,13 +314,16 @@ void append_tune_file(const std::string& device, int sms, const TuneKey& key, in
 // grid kernels of order 16 0.48 ms at N = 100k with 1.24e6 nodes; those of order 12
 // 0.18 and 0.32 ms at N = 20k and 60k with 5.4e5 nodes, and 0.088 ms a problem
 // with 16 problems of N = 20k in a launch, which share the launches' latency.
-constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 0.90e-6;  // a pair
+// Smaller FP32 sweeps cost more a pair, 1.1e-6 at N = 20k (64 problems of N = 20k:
+// 6.33 ms with 0.9e-6 here, 6.09 with 1.1e-6, 6.34 with 1.3e-6; FP64 flat around its
+// value).  A single problem's fixed cost in order 12 is 95 too; 140 keeps problems
+// that take the same either way with the sweep.
+constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 1.1e-6;  // a pair
 constexpr double kSelfCostF64 = 1.9e-6;  // a self-excitation term
-constexpr double kGridCostFixed = 95.0;  // of a group of problems
 struct GridCost {
-    double event, node;
+    double event, node, fixed;  // fixed: of a group of problems
 };
-constexpr GridCost kGridCost16{3.45e-3, 5.0e-5}, kGridCost12{3.2e-3, 5.0e-5};
+constexpr GridCost kGridCost16{3.45e-3, 5.0e-5, 95.0}, kGridCost12{3.2e-3, 5.0e-5, 140.0};
 constexpr int kGridMinEvents = 1000;
 constexpr double kGridMaxNodes = 4e8;
 constexpr size_t kGridMaxWork = size_t(8) << 30;    // one problem's workspace
@@ -541,7 +544,7 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
         const int order = fp32 && s.N < kGridHighOrderEvents ? 12 : 16;
         const GridCost& cost = order == 16 ? kGridCost16 : kGridCost12;
         const double maxNodes =
-            (direct - kGridCostFixed / std::min(P, kGridMaxJobs) - s.N * cost.event) / cost.node;
+            (direct - cost.fixed / std::min(P, kGridMaxJobs) - s.N * cost.event) / cost.node;
         if (!(maxNodes > 0.0)) continue;
         const double lo[3] = {tMin, D_ == 2 ? s.locMin[1] : 0.0, s.locMin[0]};
         const double hi[3] = {tMax, D_ == 2 ? s.locMax[1] : 0.0, s.locMax[0]};
@@ -1067,7 +1070,7 @@ int Executor::launch_sequence(int grid) {
     if (kernelTiming && (e = record(ev_[2]))) return cuda_fail(e, "timing event");
     // the results go straight to the pinned host buffer
     if ((e = launch_finish_list(pl.nBlocks, fp, fb, pl.P, dBlockSums_, dArrived_, dCounter_, hOut_,
-                                stream_)))
+                                !kernelTiming, stream_)))
         return cuda_fail(e, "finish kernel");
     launches += 2;
     if (kernelTiming && (e = record(ev_[3]))) return cuda_fail(e, "timing event");
@@ -1381,17 +1384,18 @@ int Executor::enqueue_device_body() {
     const auto* fp = reinterpret_cast<const FinishProblem*>(d + offFP_);
     const auto* fb = reinterpret_cast<const FinishBlock*>(d + offFB_);
     cudaError_t e;
+    const int variant = sweep_variant() | kAfterKernel;  // the step's, or the band kernel
     // a listed plan holds every earlier tile for any sigma and omega: start each
     // item where the current constants allow a term (the sweep of a plan without
     // a list finds that itself)
     if (!plan_.items.empty() &&
         (e = launch_band_starts((int)plan_.items.size(), sp, items, nItems, R, stream_)))
         return cuda_fail(e, "band kernel");
-    if ((e = launch_sweep_list(prec, D_, R, sweep_variant(), loopGrid_, sp, items, nItems,
+    if ((e = launch_sweep_list(prec, D_, R, variant, loopGrid_, sp, items, nItems,
                                dCounter_, stream_)))
         return cuda_fail(e, "sweep kernel");
     if ((e = launch_finish_list(plan_.nBlocks, fp, fb, plan_.P, dBlockSums_, dArrived_, dCounter_,
-                                dOut_, stream_)))
+                                dOut_, true, stream_)))
         return cuda_fail(e, "finish kernel");
     lastLaunches = 3;
     return HPHC_OK;

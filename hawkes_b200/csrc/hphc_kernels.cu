@@ -575,6 +575,8 @@ finish_list_kernel(const FinishProblem* __restrict__ problems,
                    const FinishBlock* __restrict__ blocks, int nProblems,
                    double* __restrict__ blockSums, int* __restrict__ arrived,
                    int* __restrict__ counter, double* __restrict__ out) {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     const FinishBlock fb = blocks[blockIdx.x];
     const FinishProblem& P = problems[fb.problem];
     const FinishConsts f = P.f;
@@ -908,11 +910,12 @@ cudaError_t launch_band_starts(int maxItems, const SweepProblem* problems, WorkI
 
 cudaError_t launch_finish_list(int nBlocks, const FinishProblem* problems,
                                const FinishBlock* blocks, int nProblems, double* blockSums,
-                               int* arrived, int* counter, double* out, cudaStream_t s) {
-    finish_list_kernel<<<nBlocks, kFinishThreads, 0, s>>>(problems, blocks, nProblems, blockSums,
-                                                          arrived, counter, out);
-    return cudaGetLastError();
+                               int* arrived, int* counter, double* out, bool afterKernel,
+                               cudaStream_t s) {
+    return launch_dependent(finish_list_kernel, nBlocks, kFinishThreads, afterKernel, s, problems,
+                            blocks, nProblems, blockSums, arrived, counter, out);
 }
+
 cudaError_t launch_finish(const SweepGeometry& g, const double* partials, const double* times,
                           const FinishConsts& f, double* blockSums, double* probs,
                           cudaStream_t s) {

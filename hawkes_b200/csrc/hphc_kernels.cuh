@@ -483,6 +483,7 @@ cudaError_t launch_pack_f32_jobs(int D, int nJobs, int maxN, const PackJob* jobs
 
 // Variant bit of the sweeps below: every problem of the list has noB set.
 constexpr int kSelfOnly = 32;
+constexpr int kAfterKernel = 64;  // in V: launched while the stream's last kernel ends
 
 // Persistent sweep over a work list: `grid` CTAs take items from *counter
 // (which must be 0 at launch) until *nItems are taken.  precision: 0 = FP64,
@@ -497,10 +498,34 @@ int sweep_list_blocks_per_sm(int precision, int D, int R, int V);
 
 // arrived: 1 + nProblems counters, zero between runs; counter: the sweep's work
 // counter, reset; out[8p .. 8p+7] for every problem p: log-likelihood, gradient, 0
-// (device or pinned host memory).
+// (device or pinned host memory).  afterKernel: the stream's last work is the
+// sweep's launch (no event between).
 cudaError_t launch_finish_list(int nBlocks, const FinishProblem* problems,
                                const FinishBlock* blocks, int nProblems, double* blockSums,
-                               int* arrived, int* counter, double* out, cudaStream_t s);
+                               int* arrived, int* counter, double* out, bool afterKernel,
+                               cudaStream_t s);
+
+// Launches a kernel that waits (cudaGridDependencySynchronize) for the stream's
+// last kernel, so that its blocks are set up while that one ends (overlap; the
+// earlier kernel allows it by cudaTriggerProgrammaticLaunchCompletion).  A kernel
+// launched so allows the next one only after its own wait: when a kernel starts,
+// all before the last one have then ended, and what they wrote may be read before
+// the wait.  N = 1000: 1.2 us less an evaluation, 16 chains of the device sampler
+// 42.7 -> 38.5 us an iteration.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), int blocks, int threads, bool overlap,
+                             cudaStream_t s, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks);
+    config.blockDim = dim3(threads);
+    config.stream = s;
+    config.attrs = &attr;
+    config.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
 
 // ---- incremental evaluation ------------------------------------------------
 //

@@ -577,6 +577,8 @@ sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
     __shared__ __align__(16) double sRec[kTile * Layout<D>::kF64Stride];
     __shared__ __align__(16) double sCol[SELF ? 2 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ WorkItem w;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();  // the finish may be set up (it waits)
     const int n = *nItems;
     for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
          first = false) {
@@ -1229,6 +1231,8 @@ sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
     __shared__ __align__(16) StagedTile<D> sTile;
     __shared__ __align__(16) float sCol[SELF ? 4 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ WorkItem w;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();  // the finish may be set up (it waits)
     const int n = *nItems;
     for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
          first = false) {
@@ -1274,14 +1278,16 @@ template <int D, int R>
 cudaError_t sweep_list_dispatch_v(int precision, int V, int grid, const SweepProblem* problems,
                                   const WorkItem* items, const int* nItems, int* counter,
                                   cudaStream_t s, int* blocksPerSM) {
-    const void* fn = sweep_list_function<D, R>(precision, V);
+    const void* fn = sweep_list_function<D, R>(precision, V & ~kAfterKernel);
     if (!fn) return cudaErrorInvalidValue;
     if (blocksPerSM) {
         *blocksPerSM = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, kSweepThreads, 0);
     }
-    void* args[] = {(void*)&problems, (void*)&items, (void*)&nItems, (void*)&counter};
-    return cudaLaunchKernel(fn, dim3(grid), dim3(kSweepThreads), args, 0, s);
+    return launch_dependent(
+        reinterpret_cast<void (*)(const SweepProblem*, const WorkItem*, const int*, int*)>(
+            const_cast<void*>(fn)),
+        grid, kSweepThreads, (V & kAfterKernel) != 0, s, problems, items, nItems, counter);
 }
 
 template <int D>

@@ -170,3 +170,61 @@ def test_self_excitation_window_keeps_every_sum(flags, form, D):
         assert abs(lw - lf) <= 1e-8 * abs(lf)
         big = pf > 1e-30  # above the FP32 terms' underflow
         np.testing.assert_allclose(pw[big], pf[big], rtol=5e-6)
+
+
+@pytest.mark.parametrize("form,D,n", [("plain", 1, 40000), ("unsorted", 2, 40000),
+                                      ("far_from_zero", 2, 40000), ("one_cell", 2, 40000),
+                                      ("line", 2, 40000), ("plain", 2, 65535),
+                                      ("plain", 2, 65536)])
+def test_gridded_fp32_compensated_sums(form, D, n):
+    # Below 65,536 events the grid's weighted sums are within 1.4e-10 of themselves;
+    # the self-excitation terms carry FP32 roundings (2^-24 of an event's sum, of
+    # either sign).  From there on both are as exact as in the FP64 mode.
+    rng = np.random.default_rng([11, D, n])
+    loc, t = _events(form, n, D, rng)
+    p = np.asarray(workloads.BASE_PARAMS) * np.array([1.0, 0.9, 1.2, 1.0, 1.1, 0.9])
+    out = {}
+    for flags in (FP64, FP32C):
+        with hb.CudaHawkes(D, n, flags, 0) as e:
+            e.setTimesData(t)
+            e.updateLocations(-1, loc)
+            e.setParameters(p)
+            out[flags] = *e.getLogLikelihoodAndGradient(), e.lastLaunchEvals()
+    (lw, gw, _), (lg, gg, evals) = out[FP64], out[FP32C]
+    scale = oracle.oracle_eval(loc, t, p, threads=16)["grad_scale"]
+    assert evals == 0.0 or form == "unsorted"
+    assert abs(lg - lw) <= 1e-8 * abs(lw)
+    assert np.all(np.abs(gg - gw) <= 6e-8 * scale)
+
+
+def test_large_fp32_compensated_evaluations_follow_the_events():
+    # the FP64 records such an evaluation sweeps are those of the present events
+    loc, t = workloads.uniform(70000, 5)
+    p = np.asarray(workloads.BASE_PARAMS)
+    moved = loc.copy()
+    moved[123] += 0.4
+    want = {}
+    for name, x in (("first", loc), ("moved", moved)):
+        with hb.CudaHawkes(2, len(t), FP64, 0) as f:
+            f.setTimesData(t)
+            f.updateLocations(-1, x)
+            f.setParameters(p)
+            want[name] = f.getLogLikelihoodAndGradient()
+    with hb.CudaHawkes(2, len(t), FP32C, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        e.setParameters(p * 1.1)
+        e.getLogLikelihoodAndGradient()
+        e.storeState()
+        e.updateLocations(123, moved[123])
+        e.setParameters(p)
+        got = e.getLogLikelihoodAndGradient()
+        assert abs(got[0] - want["moved"][0]) <= 1e-8 * abs(want["moved"][0])
+        np.testing.assert_allclose(got[1], want["moved"][1], rtol=1e-6)
+        assert abs(want["moved"][0] - want["first"][0]) > 1e-7 * abs(want["first"][0])
+        e.restoreState()
+        e.setParameters(p * 1.05)
+        e.getLogLikelihoodAndGradient()
+        e.setParameters(p)
+        back = e.getLogLikelihoodAndGradient()
+        assert abs(back[0] - want["first"][0]) <= 1e-8 * abs(want["first"][0])
