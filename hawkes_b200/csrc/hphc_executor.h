@@ -233,8 +233,8 @@ private:
                    int P);
     double* grid_sums(int p) const;
     double self_terms(const SetView& s, const double* p) const;
-    bool self_only(int P) const;
-    bool self_listless(const std::vector<SetView>& sets, const int* setOf, int P) const;  // no problem of the plan has background terms to sweep
+    bool self_only(int P) const;  // no problem of the plan has background terms to sweep
+    bool self_listless(const std::vector<SetView>& sets, const int* setOf, int P) const;
     int choose_shape(const std::vector<SetView>& sets, const int* setOf, const double* params,
                      int P, double* dProbs);
     int launch_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
