@@ -75,8 +75,28 @@ FP32_PER_B, FP32_PER_COL, FP32_PER_S = 11.0, 3.0, 5.0
 # background terms (each at most 2^-10 of the event's own term) and the
 # symmetric column adds keep the plain count.
 FP32C_PER_NEAR_B, FP32C_PER_S = FP32_PER_B + 11.0, FP32_PER_S + 11.0
+# A gridded evaluation (lastLaunchEvals() == 0: the background sums of large sets
+# in one or two dimensions) evaluates no background pair.  Its FP64 instructions
+# (FMA = 1): an event's 16^3 nodes once in the spread and twice in the gather
+# (plain and second-derivative weights) and 5 x 16^2 for the products of weights
+# and the contractions of planes; 97 taps a node and axis of the convolution; 19 a
+# self-excitation term (differences 3, d^2 2, exponent 2, exponential 9, sums 3).
+# Zeros that the matrix tiles carry along are not counted.
+GRID_ORDER, GRID_INV, GRID_TAPS = 16, 8, 48
+FP64_PER_S = 19.0
+FP64_LANES_PER_SM = 64
 FP32_LANES_PER_SM = 128
 MUFU_LANES_PER_SM = 16
+
+
+def grid_instructions(loc, t, params):
+    """FP64 instructions of the gridded background sums (see above)."""
+    nodes = 1.0
+    for x, precision in [(t, params[2])] + [(loc[:, k], params[1]) for k in range(loc.shape[1])]:
+        scale = GRID_INV / math.sqrt(2.0) * abs(precision)
+        nodes *= (math.floor(x.max() * scale) - math.floor(x.min() * scale) + 3 + GRID_ORDER - 1)
+    events = len(t) * (3.0 * GRID_ORDER ** 3 + 5.0 * GRID_ORDER ** 2)
+    return events + nodes * (loc.shape[1] + 1) * (2 * GRID_TAPS + 1)
 
 
 def env_int(name, default):
@@ -580,12 +600,14 @@ def ours_arm(args):
     # the roofline counts the terms the launch evaluated; "effective" counts
     # the brute-force work (every ordered pair) the launch stands for
     # algorithmic count of the evaluated terms (compensation not counted)
-    inst = FP32_PER_B * nev + FP32_PER_COL * (nb - nev) + FP32_PER_S * ns
+    # (a set's gridded pairs count in nb alone: at most one other order a term)
+    gridded = w["kind"] == "single" and nev == 0 and nb > 0
+    inst = FP32_PER_B * nev + FP32_PER_COL * min(nb - nev, nev) + FP32_PER_S * ns
     achieved = inst / (sweep_mean / 1e3) / 1e12
     far = (far_tail_share(w["t"], w["params"][2], shape32[0])
            if w["kind"] == "single" and shape32 else 1.0)
     inst_comp = (FP32C_PER_NEAR_B * (1.0 - far) * nev + FP32_PER_B * far * nev +
-                 FP32_PER_COL * (nb - nev) + FP32C_PER_S * ns)
+                 FP32_PER_COL * min(nb - nev, nev) + FP32C_PER_S * ns)
     ncu = None
     npath = os.path.join(ROOT, "profiles", "sweep_pipes.json")
     if os.path.exists(npath):
@@ -619,7 +641,9 @@ def ours_arm(args):
         "metric": metric, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step32, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 pair terms (compensated), f64 reductions", "data": "synthetic",
+        "dtype": ("f64 gridded background sums, f64 reductions; self-excitation terms f64, or "
+                  "compensated f32 where they are many" if gridded else "f32 pair terms (compensated), f64 reductions"),
+        "data": "synthetic",
         "computes": "log-likelihood + 6-parameter gradient",
         "config": config,
         "fp64_plain": {"value": value64, "ms_per_step": ms_step64,
@@ -677,6 +701,28 @@ def ours_arm(args):
         "gpu_launches": launches * args.steps,
         "clocks": clock_summary,
     }
+    if gridded:
+        # the engines agree to the bit where both sweep these terms in FP64
+        self64 = np.array_equal(ll32, ll64) and np.array_equal(g32, g64)
+        work = (grid_instructions(w["loc"], w["t"], w["params"]) +
+                (FP64_PER_S * ns if self64 else 0.0))
+        peak64 = sm_count * FP64_LANES_PER_SM * max_mhz * 1e6 / 1e12
+        rate = work / (sweep_mean / 1e3) / 1e12
+        out["terms"]["note"] = ("gridded: the background sums stand for every ordered pair and "
+                                "evaluate none; self-excitation terms within the window whose "
+                                "bound the finish checks")
+        out["roofline"] = {
+            "bound": "fp64", "kernel": "spread, convolution and gather kernels of order 16, "
+                                       "self-excitation sweep",
+            "achieved": rate, "peak": peak64, "unit": "Tinst/s", "frac": rate / peak64,
+            "traffic": None, "instructions_per_launch": work,
+            "count": "FP64 instructions (FMA = 1) of the grid kernels, without the zeros their "
+                     "matrix tiles carry, and of the self-excitation terms where they are "
+                     "FP64, over the mean CUDA-event duration from the first grid kernel to "
+                     "the end of the sweep",
+            "peak_source": f"{sm_count} SMs x {FP64_LANES_PER_SM} FP64 lanes x {max_mhz:.0f} MHz "
+                           f"(sm_max_mhz, {peak_src})",
+            "effective": out["roofline"]["effective"], "sweep_ms": sweep_mean}
     if world == 1 and not args.no_cpu_baseline:
         out["cpu_baseline"] = cpu_baseline()
     print(json.dumps(out))

@@ -129,7 +129,7 @@ void strip_band(const SetView& s, const StripGaps& gap, bool symmetric, bool wid
 // half a near one in the FP32-compensated mode (whose near terms take the
 // software exponential and three compensated sums) and 7/10 in the FP64
 // mode; the self-excitation terms of a tile add about half a tile in the
-// FP32 mode and a whole one in the FP64 mode (CUDA's exp() for each).
+// FP32 mode and a whole one in the FP64 mode (an exponential for each).
 // Ordering by these costs instead of tile counts: sweep at N = 100k 2.588 ->
 // 2.498 ms (FP32, plain block sums then) and 10.06 -> 9.69 ms (FP64); the
 // FP32 far weight 0.75 -> 0.5 with the compensated sums: 2.676 -> 2.620 ms

@@ -55,8 +55,8 @@ struct PairConsts {
     double skipB, skipS;                   // natural-log thresholds; < 0 disables
     // A tile pair whose background terms are all below exp(-fastB) (natural
     // log; <= 0 disables) takes them from the hardware ex2.approx: instead of
-    // the polynomial in the FP32 mode (2^-10, kFastTailLog2), of CUDA's exp()
-    // in the FP64 mode (2^-60, kFastTailLog2F64).
+    // the polynomial in the FP32 mode (2^-10, kFastTailLog2), of the
+    // table exponential in the FP64 mode (2^-60, kFastTailLog2F64).
     double fastB;
     // Self-excitation-only sweep: no background term is evaluated (the
     // finish takes the background sums from an earlier sweep, which depend

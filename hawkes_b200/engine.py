@@ -235,8 +235,8 @@ class CudaHawkes:
 
     def kernelTimes(self):
         """(sweep ms, finish ms, step ms) of the last evaluation made with kernel
-        timing on; the step spans table upload, record build, sweep, finish and
-        result copy on the device."""
+        timing on; the step spans table upload, record build, sweep and finish on
+        the device.  Gridded background sums count with the sweep."""
         a = ctypes.c_float()
         b = ctypes.c_float()
         c = ctypes.c_float()
@@ -245,8 +245,9 @@ class CudaHawkes:
         return a.value, b.value, c.value
 
     def lastLaunchStats(self):
-        """(kernel launches, background terms evaluated, self-excitation terms
-        evaluated) of the last evaluation."""
+        """(kernel launches, background terms accounted for, self-excitation terms
+        evaluated) of the last evaluation; gridded background sums account for
+        N^2 terms."""
         n = ctypes.c_int()
         nb = ctypes.c_double()
         ns = ctypes.c_double()
@@ -256,7 +257,7 @@ class CudaHawkes:
 
     def lastLaunchEvals(self):
         """Background exponentials the last evaluation computed (a pair
-        evaluated once for both of its events counts once)."""
+        evaluated once for both of its events counts once; gridded sums: none)."""
         v = ctypes.c_double()
         self._check(_lib.hphc_get_last_launch_evals(self._h, ctypes.byref(v)), "lastLaunchEvals")
         return v.value

@@ -90,7 +90,9 @@ extern "C" {
                                                 whose background terms are all below 2^-91
                                                 (FP64) or 2^-60 (FP32 modes) of an event's
                                                 own term are skipped: together under 2^-60
-                                                and 2^-33 of any event's sums) */
+                                                and 2^-33 of any event's sums); neither
+                                                gridded background sums nor the
+                                                self-excitation window */
 
 /* How the last evaluation was computed (hphc_get_last_evaluation_path). */
 #define HPHC_PATH_SWEEP 0        /* the O(N^2) pair sweep                             */
@@ -420,11 +422,14 @@ int hphc_get_last_evaluation_path(hphc_engine* engine, int* path);
  * level: the non-causal half of the self-excitation sum, tile pairs whose
  * terms all underflow to exactly zero in the working precision, and (tail
  * truncation) background tile pairs whose terms are all below 2^-91 (FP64) or
- * 2^-60 (FP32 modes) of an event's own term. */
+ * 2^-60 (FP32 modes) of an event's own term, and self-excitation tile pairs
+ * outside the window (together under 2^-60 or 2^-36 of the event's sum, which the
+ * finish checks).  Gridded background sums count as N^2 terms. */
 int hphc_get_last_launch_stats(hphc_engine* engine, int* kernelLaunches,
                                double* backgroundTerms, double* selfExciteTerms);
 
-/* Background exponentials the most recent evaluation's sweep computed.  In the
+/* Background exponentials the most recent evaluation's sweep computed (none for
+ * gridded background sums).  In the
  * FP32-compensated mode each background pair (i, j) with j in a tile before
  * i's strip is evaluated once and counted once, but stands for two terms in
  * backgroundTerms above (B_ij in event i's sum, B_ji in event j's). */
@@ -434,7 +439,8 @@ int hphc_get_last_launch_evals(hphc_engine* engine, double* backgroundEvals);
  * as many) and the number of (strip, j-range) work items per SM the j range is
  * split into.  0 for either lets the engine's autotuner choose it (timed on the
  * engine's own data at the first evaluation, cached per process by problem
- * size and mode). */
+ * size and mode).  A shape fixed in both keeps every problem with the pair sweep
+ * of whole tiles: no gridded sums, no self-excitation window. */
 int hphc_set_sweep_shape(hphc_engine* engine, int eventsPerThread, int itemsPerSM);
 int hphc_get_sweep_shape(hphc_engine* engine, int* eventsPerThread, int* itemsPerSM);
 
