@@ -346,14 +346,15 @@ struct EventSet {
             if (!order.wanted) continue;
             if ((e = launch_strip_order(D, N, R, dLoc.p, R == 2 ? dOrder2.p : dOrder4.p, s))) return e;
             order.ready = true;
-            *launches += (N >= R * kSweepThreads) + (N % (R * kSweepThreads) != 0);
+            *launches += N >= R * kSweepThreads;
         }
         if (sorted) {
             if ((e = launch_tile_bounds(N, dTimes.p, dTileMin.p, dTileMax.p, dTileChanges.p, s,
                                         floatTimes)))
                 return e;
-            e = launch_sorted_ranks(N, dTimes.p, dTileChanges.p, dRanks.p, s, floatTimes);
-            *launches += 3;
+            e = launch_sorted_ranks(N, dTimes.p, dTileChanges.p, dRanks.p, s, floatTimes,
+                                    launches);
+            *launches += 1;
         } else {
             if ((e = cudaMemcpyAsync(dRanks.p, hRanks.p, (size_t)N * sizeof(int32_t),
                                      cudaMemcpyHostToDevice, s)))

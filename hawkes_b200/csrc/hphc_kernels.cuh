@@ -321,16 +321,16 @@ cudaError_t launch_pack_f64(int D, int N, const double* loc, const double* times
 cudaError_t launch_tile_bounds(int N, const double* times, double* tileMin, double* tileMax,
                                int* tileChanges, cudaStream_t s, int floatTimes = 0);
 // Dense time ranks of SORTED times from the tile counts of launch_tile_bounds
-// (which it overwrites with their exclusive prefix sums): rank[j] = number of
-// k in 1..j with t_k != t_{k-1}.  Two launches.
+// (which it may overwrite with their exclusive prefix sums): rank[j] = number of
+// k in 1..j with t_k != t_{k-1}.  One or two launches, added to *launches.
 cudaError_t launch_sorted_ranks(int N, const double* times, int* tileChanges, int32_t* ranks,
-                                cudaStream_t s, int floatTimes = 0);
+                                cudaStream_t s, int floatTimes, int* launches);
 
 // Target-row order of the FP32 symmetric sweep with R events per thread:
 // within each full strip of 128 R events, rows sorted along a Morton curve of
 // their first two coordinates and dealt to threads in runs of R (spatial
-// neighbours share a thread); the last partial strip keeps its order.  One
-// or two launches.
+// neighbours share a thread); the last partial strip has none.  One launch, or
+// none without a full strip.
 cudaError_t launch_strip_order(int D, int N, int R, const double* loc, int32_t* order,
                                cudaStream_t s);
 

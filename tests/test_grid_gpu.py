@@ -228,3 +228,24 @@ def test_large_fp32_compensated_evaluations_follow_the_events():
         e.setParameters(p)
         back = e.getLogLikelihoodAndGradient()
         assert abs(back[0] - want["first"][0]) <= 1e-8 * abs(want["first"][0])
+
+
+@pytest.mark.parametrize("n", [262143, 262144, 262145, 262273])
+def test_ranks_of_tied_times(n):
+    # Ranks decide which FP32 terms are causal; the FP64 mode compares times.  On
+    # both sides of the size up to which each tile adds up the ones before it.
+    rng = np.random.default_rng(n)
+    t = np.floor(np.sort(rng.uniform(0.0, 40000.0, n)) / 4.0) * 4.0
+    loc = rng.uniform(0.0, 3000.0, (n, 1))
+    p = np.asarray(workloads.BASE_PARAMS) * np.array([1, 1, 40, 1, 1, 1])
+    out = {}
+    for flags in (FP64, FP32C):
+        with hb.CudaHawkes(1, n, flags, 0) as e:
+            e.setSweepShape(2, 64)  # the pair sweep: FP32 terms whatever their number
+            e.setTimesData(t)
+            e.updateLocations(-1, loc)
+            e.setParameters(p)
+            out[flags] = e.getLogLikelihoodAndGradient()[0], e.getProbsSelfExcite()
+    # a tie counted as causal, or an event left out, moves its P_i by about its size
+    assert abs(out[FP64][0] - out[FP32C][0]) <= 1e-8 * abs(out[FP64][0])
+    assert np.abs(out[FP64][1] - out[FP32C][1]).max() <= 1e-4
