@@ -20,6 +20,7 @@
 //
 // Every sweep goes through hphc::Executor: one launch per stage for any
 // number of (event set, parameter vector) problems, replayed from a CUDA graph.
+#include <atomic>
 #include <cuda_runtime.h>
 #if defined(__SSE2__)
 #include <emmintrin.h>
@@ -189,6 +190,7 @@ struct EventSet {
     DevBuf<int32_t> dOrder2, dOrder4;  // FP32 mode: spatial row order of R = 2 and 4 strips
     RowOrder order2, order4;
     bool packedF64 = false;                   // FP32-compensated mode
+    uint64_t version = 0;                     // of the device's events (changed())
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 
@@ -222,6 +224,13 @@ struct EventSet {
             locMax[k] = hi[k];
         }
         haveBox = true;
+    }
+    // The device's events are about to change: records packed from them are stale.
+    // (Versions are never reused, by another set either.)
+    void changed() {
+        static std::atomic<uint64_t> last{0};
+        version = ++last;
+        packedF64 = false;
     }
     // The bounds from copy_checked's (D = 1 and 2).
     void set_box(const double* box) {
@@ -329,6 +338,7 @@ struct EventSet {
     // device-side derived data.
     cudaError_t upload(const double* hLoc, int precision, cudaStream_t s, int* launches) {
         cudaError_t e;
+        changed();
         if ((e = cudaMemcpyAsync(dLoc.p, hLoc, (size_t)N * D * sizeof(double),
                                  cudaMemcpyHostToDevice, s)) ||
             (e = cudaMemcpyAsync(dTimes.p, hTimes.p, (size_t)N * sizeof(double),
@@ -339,7 +349,6 @@ struct EventSet {
             *launches += 2;
             return e;
         }
-        packedF64 = false;
         order2.ready = order4.ready = false;
         for (int R = 2; R <= 4; R += 2) {
             RowOrder& order = R == 2 ? order2 : order4;
@@ -368,6 +377,7 @@ struct EventSet {
     SetView view() {
         SetView v;
         v.N = N;
+        v.version = version;
         v.dLoc = dLoc.p;
         v.dTimes = dTimes.p;
         v.dRanks = dRanks.p;
@@ -772,6 +782,7 @@ struct hphc_engine {
         cudaStream_t s = rt.stream;
         const PairConsts c = rt.ex.pair_consts(p, set.view());
         cudaError_t e = cudaSuccess;
+        if (hadMoves) set.changed();
         for (size_t m = 0; m < moved.size(); ++m) {
             MovedEvent mv{};
             mv.k = moved[m];
@@ -788,7 +799,6 @@ struct hphc_engine {
             lastLaunches += 2;
         }
         if (hadMoves && !wasDirty && rt.mode.precision == HPHC_PRECISION_FP64) recStale = true;
-        if (hadMoves) set.packedF64 = false;
         lastIncTerms = (double)moved.size() * (3.0 * N - 2.0);
         clear_moved();
         const FinishConsts f = rt.ex.finish_consts(p, set.view());

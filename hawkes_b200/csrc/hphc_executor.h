@@ -35,6 +35,7 @@ struct RowOrder {
 // An event set resident on the device, with host copies used for planning.
 struct SetView {
     int N = 0;
+    uint64_t version = 0;              // of the device's events: another after any change
     const double* dLoc = nullptr;      // N x D raw coordinates
     const double* dTimes = nullptr;    // N raw times
     const int32_t* dRanks = nullptr;   // dense time ranks (FP32 mode)
@@ -215,14 +216,24 @@ private:
     // graph
     // one graph per kind of plan (shape_'s kinds), so that a sampler that mixes
     // full evaluations and self-excitation steps captures each once
-    cudaGraphExec_t graphExec_[3] = {};
+    // (and, the second three, once more for runs whose records are packed)
+    cudaGraphExec_t graphExec_[6] = {};
     struct GraphKey {
         int P = -1, nJobs = -1, nBlocks = -1, maxN = -1, R = -1, grid = -1;
         size_t tablesBytes = 0, colNeed = 0;
         void* tables = nullptr;
         int variant = 0;
         bool timing = false;
-    } graphKey_[3];
+    } graphKey_[6];
+    // What the record pool holds: one set's FP32 records at one scaling.  A plan that
+    // needs just those launches no pack: the sampler's sigma and omega steps, which
+    // leave events, tauX and tauT alone.
+    struct Packed {
+        uint64_t version = 0;  // 0: none
+        const double* loc = nullptr;
+        double sX = 0.0, sT = 0.0;
+    } packed_, willPack_;
+    bool skipPack_ = false;  // of the current plan
     int kind_ = 0;  // of the current plan
 
     ConstsSpec consts_spec() const;
@@ -246,7 +257,7 @@ private:
     int cuda_fail(cudaError_t e, const char* what);
     void drop_graph(int kind);
     void drop_graphs() {
-        for (int k = 0; k < 3; ++k) drop_graph(k);
+        for (int k = 0; k < 6; ++k) drop_graph(k);
     }
     cudaError_t record(cudaEvent_t ev);
     bool capturing_ = false;
