@@ -279,6 +279,17 @@ strip_order_kernel(int D, const double* __restrict__ loc, int32_t* __restrict__ 
     }
 }
 
+// Small tables from pinned host memory: the next kernel can be set up meanwhile,
+// which it cannot behind a copy engine's transfer.
+constexpr int kCopyThreads = 128;
+
+__global__ void __launch_bounds__(kCopyThreads)
+copy_tables_kernel(int4* __restrict__ dst, const int4* __restrict__ src, int n) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int i = blockIdx.x * kCopyThreads + threadIdx.x;
+    if (i < n) dst[i] = src[i];
+}
+
 // Device-resident loop: before each sweep, one thread per work item sets the
 // item's first tile from the problem's current constants (a separate launch,
 // so the sweep kernels themselves only read WorkItem::start).
@@ -915,6 +926,13 @@ cudaError_t launch_pack_f32_jobs(int D, int nJobs, int maxN, const PackJob* jobs
 #undef X
         default: return cudaErrorInvalidValue;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_copy_tables(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    const int n = (int)(bytes / 16);
+    copy_tables_kernel<<<(n + kCopyThreads - 1) / kCopyThreads, kCopyThreads, 0, s>>>(
+        static_cast<int4*>(dst), static_cast<const int4*>(src), n);
     return cudaGetLastError();
 }
 

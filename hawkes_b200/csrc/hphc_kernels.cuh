@@ -434,6 +434,10 @@ struct WorkItem {
     int problem, strip, jt0, jt1, slot, start, col0, cols;
 };
 
+// Copies `bytes` (a multiple of 16, both ends 16-byte aligned) from pinned host
+// memory to the device by a kernel.
+cudaError_t launch_copy_tables(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 constexpr int kBandThreads = 256;
 
 // Device-resident loop: items[k].start for the first *nItems items (maxItems
