@@ -556,9 +556,9 @@ __device__ __forceinline__ void add_left_out(const FinishProblem& P, const Finis
 // total in CTA order to out[0..7] (which may be pinned host memory), so that no
 // launch and no copy follow.  Returns true on the problem's last CTA's thread 0.
 // *arrived is zero before and after.
-__device__ __forceinline__ bool finish_total(double (&v)[8], double* __restrict__ blockSums,
-                                             int block, int first, int count, int* arrived,
-                                             double constant, double* __restrict__ out) {
+__device__ __forceinline__ bool finish_total(double (&v)[8], double* blockSums, int block,
+                                             int first, int count, int* arrived, double constant,
+                                             double* out) {
     static_assert(kFinishThreads == kFinalThreads, "the total's order");
     __shared__ bool sLast;
     if (threadIdx.x == 0) {
@@ -572,9 +572,11 @@ __device__ __forceinline__ bool finish_total(double (&v)[8], double* __restrict_
     __threadfence();
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    // other CTAs of this launch wrote them
+    const volatile double* sums = blockSums + (size_t)first * 8;
     for (int b = threadIdx.x; b < count; b += kFinishThreads)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] += __ldcg(blockSums + (size_t)(first + b) * 8 + q);
+        for (int q = 0; q < 8; ++q) v[q] += sums[(size_t)b * 8 + q];
     block_sum<8, kFinishThreads>(v);
     if (threadIdx.x != 0) return false;
     out[0] = v[0] + constant;
@@ -594,10 +596,8 @@ __device__ __forceinline__ bool finish_total(double (&v)[8], double* __restrict_
 // the blocks of N = 100k in one wave (18 us instead of 23).
 template <int CTAS>
 __global__ void __launch_bounds__(kFinishThreads, CTAS)
-finish_list_kernel(const FinishProblem* __restrict__ problems,
-                   const FinishBlock* __restrict__ blocks, int nProblems,
-                   double* __restrict__ blockSums, int* __restrict__ arrived,
-                   int* __restrict__ counter, double* __restrict__ out) {
+finish_list_kernel(const FinishProblem* problems, const FinishBlock* blocks, int nProblems,
+                   double* blockSums, int* arrived, int* counter, double* out) {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
     const FinishBlock fb = blocks[blockIdx.x];
@@ -797,8 +797,8 @@ move_event_row_kernel(int N, int k, int nBlocks, const double* __restrict__ rowP
 
 __global__ void __launch_bounds__(kFinishThreads)
 finish_sums_kernel(int N, const double* __restrict__ sums, const double* __restrict__ times,
-                   FinishConsts f, double* __restrict__ blockSums, int* __restrict__ arrived,
-                   double* __restrict__ probs, double* __restrict__ out) {
+                   FinishConsts f, double* blockSums, int* arrived, double* __restrict__ probs,
+                   double* out) {
     const int i = blockIdx.x * kFinishThreads + threadIdx.x;
     double v[8];
 #pragma unroll

@@ -64,12 +64,10 @@ struct SampledSet {
 constexpr int kStepThreads = 32;
 
 __global__ void __launch_bounds__(kStepThreads)
-mh_step_kernel(Chain* __restrict__ chains, SampledSet sampled, double* __restrict__ prop,
-               hphc::SweepProblem* __restrict__ sp, hphc::FinishProblem* __restrict__ fp,
-               hphc::ConstsSpec spec, const double* __restrict__ results,
-               int* __restrict__ iteration, bool accepting, int iterations, int burnIn, int saved,
-               double* __restrict__ samples, double* __restrict__ targets) {
-    cudaTriggerProgrammaticLaunchCompletion();  // the next sweep may be set up (it waits)
+mh_step_kernel(Chain* chains, SampledSet sampled, double* prop, hphc::SweepProblem* sp,
+               hphc::FinishProblem* fp, hphc::ConstsSpec spec, const double* results,
+               int* iteration, bool accepting, int iterations, int burnIn, int saved,
+               double* samples, double* targets) {
     const int k = blockIdx.x, lane = threadIdx.x;
     __shared__ Chain c;
     __shared__ double p[kParams];
@@ -81,15 +79,16 @@ mh_step_kernel(Chain* __restrict__ chains, SampledSet sampled, double* __restric
     if (lane < kParams) p[lane] = prop[(size_t)k * kParams + lane];
     int done = iteration[k];
     __syncwarp();
+    double term = 0.0;
+    if (accepting && lane < hphc::mh::kAcceptTerms) term = hphc::mh::accept_term(c, p, lane);
+    cudaGridDependencySynchronize();  // the finish: results written, constants read
+    cudaTriggerProgrammaticLaunchCompletion();  // the next sweep may be set up (it waits)
     if (accepting) {
-        const double term = lane < hphc::mh::kAcceptTerms ? hphc::mh::accept_term(c, p, lane) : 0.0;
         double terms[hphc::mh::kAcceptTerms];
 #pragma unroll
         for (int q = 0; q < hphc::mh::kAcceptTerms; ++q)
             terms[q] = __shfl_sync(0xffffffffu, term, q);
         ++done;
-        __syncwarp();
-        cudaGridDependencySynchronize();  // the finish: results written, constants read
         if (lane == 0) {
             hphc::mh::accept(c, p, results[(size_t)8 * k], terms);
             iteration[k] = done;

@@ -519,8 +519,8 @@ sweep_f64_kernel(SweepGeometry g, const double* __restrict__ rec,
 // problems carry no list: slot by slot, so that the items nearest the diagonal,
 // which hold terms, come first and the empty ones of wide plans fill the end.
 template <bool SELF, int R>
-__device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ problems,
-                                              const WorkItem* __restrict__ items, int it) {
+__device__ __forceinline__ WorkItem work_item(const SweepProblem* problems, const WorkItem* items,
+                                              int it) {
     if (!SELF || problems[0].slotItems == 0) {
         const int shift = problems[0].partShift;
         WorkItem w = items[it >> shift];
@@ -552,9 +552,8 @@ __device__ __forceinline__ WorkItem work_item(const SweepProblem* __restrict__ p
 // The first is the CTA's own number, the others come from the counter (740 CTAs
 // that begin with an atomic on one address cost 4 us: N = 500 FP64 sweep 16 -> 12).
 template <bool SELF, int R>
-__device__ __forceinline__ bool next_item(const SweepProblem* __restrict__ problems,
-                                          const WorkItem* __restrict__ items, int n, int* counter,
-                                          bool first, WorkItem& item) {
+__device__ __forceinline__ bool next_item(const SweepProblem* problems, const WorkItem* items, int n,
+                                          int* counter, bool first, WorkItem& item) {
     if (!first) __syncthreads();
     if (threadIdx.x == 0) {
         const int it = first ? blockIdx.x : gridDim.x + atomicAdd(counter, 1);
@@ -571,9 +570,8 @@ __device__ __forceinline__ bool next_item(const SweepProblem* __restrict__ probl
 // (with the full underflow distance).
 template <int D, int R, bool SELF>
 __global__ void __launch_bounds__(kSweepThreads, (R == 1 ? 4 : 3) + (SELF ? R : 0))
-sweep_f64_list_kernel(const SweepProblem* __restrict__ problems,
-                      const WorkItem* __restrict__ items, const int* __restrict__ nItems,
-                      int* __restrict__ counter) {
+sweep_f64_list_kernel(const SweepProblem* problems, const WorkItem* items, const int* nItems,
+                      int* counter) {
     __shared__ __align__(16) double sRec[kTile * Layout<D>::kF64Stride];
     __shared__ __align__(16) double sCol[SELF ? 2 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ WorkItem w;
@@ -1225,9 +1223,8 @@ __device__ __forceinline__ void f32c_item(const float* __restrict__ rec,
 // 0.206 -> 0.177 ms (with the full underflow distance).
 template <int D, int R, int V, bool SELF>
 __global__ void __launch_bounds__(kSweepThreads, SELF ? (R <= 2 ? 5 : 3) : (R <= 2 ? 4 : 2))
-sweep_f32c_list_kernel(const SweepProblem* __restrict__ problems,
-                       const WorkItem* __restrict__ items, const int* __restrict__ nItems,
-                       int* __restrict__ counter) {
+sweep_f32c_list_kernel(const SweepProblem* problems, const WorkItem* items, const int* nItems,
+                       int* counter) {
     __shared__ __align__(16) StagedTile<D> sTile;
     __shared__ __align__(16) float sCol[SELF ? 4 : (kSweepThreads / 32) * 3 * kTile];
     __shared__ WorkItem w;
