@@ -1258,6 +1258,8 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
         error = "no problems to evaluate";
         return HPHC_ERR_BAD_ARGUMENT;
     }
+    // the choice of the grid asks for the engine's own cuts, not those of the plan before
+    planPrecision_ = precision_;
     plan_grid(sets, setOf, params, P);
     // Large gridded evaluations of the FP32-compensated mode sweep their
     // self-excitation terms in FP64 too, where that is a small part of them: the
@@ -1266,7 +1268,6 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     // worst gradient component 9.6e-10 -> 3.6e-15 relative).  Where the terms are
     // many they stay in FP32 (N = 500k clustered: 2.2 against 4.1 ms, beside 2.0 ms
     // of grid kernels).
-    planPrecision_ = precision_;
     if (precision_ == HPHC_PRECISION_FP32_COMP && !keptB && self_only(P)) {
         bool large = true;
         for (int p = 0; p < P; ++p)

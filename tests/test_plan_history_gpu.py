@@ -1,0 +1,54 @@
+"""The plan of an evaluation follows from its events, parameters and settings, not from
+what the engine evaluated before: the same call gives the same bits."""
+import numpy as np
+import pytest
+
+import hawkes_b200 as hb
+from hawkes_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+FP64 = hb.CUDA
+FP32C = hb.CUDA | hb.COMPENSATED
+
+
+def _evaluate(e, p):
+    """(log-likelihood, gradient, background terms evaluated as pairs)."""
+    e.setParameters(p)
+    ll, g = e.getLogLikelihoodAndGradient()
+    return ll, np.asarray(g), e.lastLaunchEvals()
+
+
+def test_grid_choice_after_an_fp64_plan():
+    # A large FP32-compensated evaluation sweeps in FP64 beside the grid.  A problem just
+    # on the pair sweep's side of the choice is taken the same way after it: the edge is
+    # found by bisection in tauX (a finer grid costs more) with pair sweeps in between, and
+    # the FP64 cut counts up to 1.23 times the pairs, 1.1 times as large a tauX.
+    n = 66000
+    loc, t = workloads.uniform(n, 3)
+    base = np.asarray(workloads.BASE_PARAMS)
+    with hb.CudaHawkes(2, n, FP32C | hb.NO_INCREMENTAL, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+
+        def at(scale):
+            return base * np.array([1, scale, 1, 1, 1, 1])
+
+        pairs, gridded = at(64.0), at(1.0)
+        assert _evaluate(e, gridded)[2] == 0.0
+        lo, hi = 1.0, 64.0
+        while hi / lo > 1.01:
+            mid = np.sqrt(lo * hi)
+            assert _evaluate(e, pairs)[2] > 0.0
+            if _evaluate(e, at(mid))[2] == 0.0:
+                lo = mid
+            else:
+                hi = mid
+        edge = at(hi * 1.02)
+        assert _evaluate(e, pairs)[2] > 0.0
+        ll, g, evals = _evaluate(e, edge)
+        assert evals > 0.0
+        assert _evaluate(e, gridded)[2] == 0.0
+        again = _evaluate(e, edge)
+        assert again[2] == evals
+        assert again[0] == ll and np.array_equal(again[1], g)
