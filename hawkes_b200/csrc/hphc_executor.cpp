@@ -1211,7 +1211,7 @@ int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
     if (kind_ == 1 && !s.tuned && shape_[0].tuned) {
         s = shape_[0];
         // a few thousand events: more, smaller strips fill the SMs
-        if (selfOnly_ && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
+        if (!fixedR && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
     }
     // without a list there is one question left, and the smaller strips answer it:
     // R = 2 against 4 in FP32 0.125 : 0.155 ms at N = 100k and 1.15 : 1.30 at 400k, R = 1

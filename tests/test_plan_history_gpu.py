@@ -52,3 +52,21 @@ def test_grid_choice_after_an_fp64_plan():
         again = _evaluate(e, edge)
         assert again[2] == evals
         assert again[0] == ll and np.array_equal(again[1], g)
+
+
+@pytest.mark.parametrize("flags,R", [(FP64, 1), (FP64, 2), (FP32C, 2), (FP32C, 4)])
+def test_fixed_events_per_thread_hold_for_every_plan(flags, R):
+    # set alone, with the items per SM left to the engine: full sweeps and
+    # self-excitation steps, of a few thousand events too
+    loc, t = workloads.uniform(3000, 12)
+    p = np.asarray(workloads.BASE_PARAMS)
+    with hb.CudaHawkes(2, len(t), flags, 0) as e:
+        e.setSweepShape(R, 0)
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        e.setParameters(p)
+        e.getLogLikelihoodAndGradient()
+        assert e.lastEvaluationPath == hb.PATH_SWEEP and e.sweepShape()[0] == R
+        e.setParameters(p * np.array([1.1, 1, 1, 1, 1, 1]))
+        e.getLogLikelihoodAndGradient()
+        assert e.lastEvaluationPath == hb.PATH_SELF_EXCITATION and e.sweepShape()[0] == R
