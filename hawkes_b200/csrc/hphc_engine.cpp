@@ -194,8 +194,7 @@ struct EventSet {
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 
-    // Bounds of the coordinates hLoc, once after each new block of locations;
-    // a moved event only widens them.
+    // Bounds of the coordinates hLoc, where they are not known.
     void update_box(const double* hLoc) {
         if (haveBox) return;
         constexpr int W = 8;  // independent running bounds: the loop vectorises
@@ -241,10 +240,14 @@ struct EventSet {
         locMax[1] = D == 1 ? 0.0 : box[3];
         haveBox = true;
     }
-    void widen_box(const double* row) {
+    // One event moves: the bounds widen to its new place, or are formed anew
+    // (update_box) if its old one may have been theirs, so that they are always those
+    // of the present events and plans do not depend on where events have been.
+    void move_in_box(const double* from, const double* to) {
         for (int k = 0; k < D; ++k) {
-            locMin[k] = std::min(locMin[k], row[k]);
-            locMax[k] = std::max(locMax[k], row[k]);
+            haveBox = haveBox && from[k] != locMin[k] && from[k] != locMax[k];
+            locMin[k] = std::min(locMin[k], to[k]);
+            locMax[k] = std::max(locMax[k], to[k]);
         }
     }
 
@@ -1082,8 +1085,8 @@ int hphc_update_locations(hphc_engine* e, int locationIndex, const double* locat
         e->invalidate_sums();
         e->dirty = true;
     }
+    e->set.move_in_box(row, location);
     std::memcpy(row, location, length * sizeof(double));
-    e->set.widen_box(row);
     return HPHC_OK;
 }
 

@@ -70,3 +70,36 @@ def test_fixed_events_per_thread_hold_for_every_plan(flags, R):
         e.setParameters(p * np.array([1.1, 1, 1, 1, 1, 1]))
         e.getLogLikelihoodAndGradient()
         assert e.lastEvaluationPath == hb.PATH_SELF_EXCITATION and e.sweepShape()[0] == R
+
+
+@pytest.mark.parametrize("flags,n", [(FP64, 30000), (FP32C, 40000)])
+def test_plan_after_an_event_has_been_far_away(flags, n):
+    # An event moves out of the box and back, or another one on its edge moves in: the
+    # grid is laid over the present events, as in an engine that has seen no others.
+    loc, t = workloads.uniform(n, 13)
+    p = np.asarray(workloads.BASE_PARAMS)
+    inward = loc.copy()
+    edge = int(np.argmin(loc[:, 0]))
+    inward[edge] = loc.mean(0)
+
+    def fresh(x):
+        with hb.CudaHawkes(2, n, flags, 0) as f:
+            f.setTimesData(t)
+            f.updateLocations(-1, x)
+            return _evaluate(f, p)
+
+    with hb.CudaHawkes(2, n, flags, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        first = _evaluate(e, p)
+        assert first[2] == 0.0  # gridded
+        e.updateLocations(5, loc[5] - 37.3)
+        _evaluate(e, p * 1.1)
+        e.updateLocations(5, loc[5])
+        back = _evaluate(e, p)
+        assert back[0] == first[0] and np.array_equal(back[1], first[1])
+        e.updateLocations(edge, inward[edge])
+        _evaluate(e, p * 1.1)
+        got, want = _evaluate(e, p), fresh(inward)
+        assert got[2] == want[2] == 0.0
+        assert got[0] == want[0] and np.array_equal(got[1], want[1])
