@@ -150,7 +150,9 @@ private:
     bool wideBands_ = false;  // build_plan: bands for any sampled parameters
     int loopGrid_ = 0;        // sweep grid of the device loop
     bool selfOnly_ = false;   // the current plan's sweep is self-excitation-only
-    int sweep_variant() const { return variant_ | (selfOnly_ ? kSelfOnly : 0); }
+    int sweep_variant() const {
+        return variant_ | (!selfOnly_ ? 0 : kSelfOnly | (planPrecision_ != precision_ ? kShortExp : 0));
+    }
     double ex2Bias_ = 0.0;
     std::string deviceName_;  // for the persistent tune cache
     cudaStream_t stream_ = nullptr;

@@ -39,11 +39,11 @@ struct Layout {
 //              S_u = exp(cS d^2 + cW dt)   for dt > 0,
 // with cA = -a^2/2, cB = -b^2/2, cS = -sigma^2/2, cW = -omega.
 struct PairConsts {
-    double cA, cB, cS, cW;                 // natural-log units (tile decisions, moved events)
-    // The same four in units of 1/32 octave (times 32 log2(e), each the correctly
-    // rounded product to within 2^-100), the argument of the FP64 sweep's
-    // table-driven exponential (exp2_32 in hphc_sweep.cuh).
-    double eA, eB, eS, eW;
+    double cA, cB, cS, cW;                 // natural-log units
+    // cS and cW in units of 1/32 octave (times 32 log2(e), each the correctly rounded
+    // product to within 2^-100), the argument of the short exponential (exp2_32 in
+    // hphc_sweep.cuh).
+    double eS, eW;
     // FP32 path, on records scaled by sX = |a| sqrt(log2(e)/2), sT = |b| sqrt(log2(e)/2):
     // S exponent (log2 units) = kS |dx'|^2 + kW dt' with kS = -sigma^2 / a^2 and
     // kW = -omega log2(e) / sT, each split hi + lo.
@@ -216,8 +216,6 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     c.cB = -0.5 * b * b;
     c.cS = -0.5 * sigma * sigma;
     c.cW = -omega;
-    c.eA = -0.5 * times_32_log2e(a, a);
-    c.eB = -0.5 * times_32_log2e(b, b);
     c.eS = -0.5 * times_32_log2e(sigma, sigma);
     c.eW = -times_32_log2e(omega, 1.0);
     const double recScale = sqrt(0.5 * kLog2eC);  // record scale per unit precision
@@ -488,6 +486,9 @@ cudaError_t launch_pack_f32_jobs(int D, int nJobs, int maxN, const PackJob* jobs
 // Variant bit of the sweeps below: every problem of the list has noB set.
 constexpr int kSelfOnly = 32;
 constexpr int kAfterKernel = 64;  // in V: launched while the stream's last kernel ends
+// In V, with kSelfOnly and precision 0: the short exponential (exp2_32), for the FP64
+// self-excitation sweeps of the FP32-compensated mode.
+constexpr int kShortExp = 128;
 
 // Persistent sweep over a work list: `grid` CTAs take items from *counter
 // (which must be 0 at launch) until *nItems are taken.  precision: 0 = FP64,

@@ -89,29 +89,45 @@ __device__ __forceinline__ TileMode tile_mode(double tminI, double tmaxI, double
 
 // ----------------------------------------------------------- FP64 sweep --
 
-// ---- FP64 exponential ----
+// ---- FP64 exponentials ----
 //
-// The FP64 sweep is bound by the FP64 pipe (64 operations per SM and clock),
-// and about half of a pair's operations were CUDA's exp().  Here the
-// exponent comes in units of 1/32 octave (PairConsts::eA .. eW: the scaling
-// sits in the coefficients), so the reduction is exact and needs no
-// constant: s = n + f with n = rint(s), |f| <= 1/2, and
-//   2^(s/32) = 2^(n >> 5) * 2^((n & 31)/32) * 2^(f/32),
-// the table-driven method of P. T. P. Tang ("Table-driven implementation of
-// the exponential function in IEEE floating-point arithmetic", ACM TOMS 15,
-// 1989).  2^(f/32) - 1 = f q(f) with q of degree 4, fitted in relative error
-// with zero mean, since sums of many terms collect the mean (maximum
-// 1.1e-16, mean 1e-18 with these coefficients, tests/test_exp64.py); the 32
-// table values sit one per lane and are fetched by a shuffle, whose 32
-// words per clock and SM are far from bound and have no bank conflicts; the
-// power of two goes into the exponent field.  9 FP64 operations a term.
-// Against exp() at N = 100k: full sweep 9.63 -> 8.16 ms, self-excitation
-// sweep 1.87 -> 1.37 ms.
+// The FP64 sweep is bound by the FP64 pipe (64 operations per SM and clock), and
+// about half of a pair's operations were CUDA's exp().  Here e^x = 2^(n/32) e^r with
+// n the integer next to 32 log2(e) x, the table-driven method of P. T. P. Tang
+// ("Table-driven implementation of the exponential function in IEEE floating-point
+// arithmetic", ACM TOMS 15, 1989).  The 32 values 2^((n & 31)/32) sit one per lane and
+// are fetched by a shuffle, whose 32 words per clock and SM are far from bound and
+// have no bank conflicts; 2^(n >> 5) goes into the exponent field.  Two forms:
+//
+//   exp_f64, the FP64 mode's: r = x - n ln2/32 in two steps, e^r - 1 to degree 6 (within
+//     1e-18), and the rounding error of the table value, relative to it, as the
+//     polynomial's constant term (the upper word of a double is plenty).  A term is
+//     within 0.54 units in the last place of e^x and 0.29 in the mean square, what one
+//     rounding gives (0.5 and 0.29): sums are as exact as with exp().  11 FP64
+//     operations, exp() takes 16.
+//   exp2_32, of the FP64 self-excitation sweeps of the FP32-compensated mode
+//     (kShortExp): the exponent comes in units of 1/32 octave (PairConsts::eS, eW: the
+//     scaling sits in the coefficients), so the reduction needs no constant; degree 5
+//     fitted in relative error with zero mean, since sums of many terms collect
+//     the mean (maximum 1.1e-16, mean 1e-18, tests/test_exp64.py), no correction.  Within
+//     1.93 units, 0.55 in the mean square, and the coefficients are rounded once more
+//     than in natural units; 9 operations.
+//
+// Against exp() at N = 100k with the second form: full sweep 9.63 -> 8.16 ms,
+// self-excitation sweep 1.87 -> 1.37 ms.
 constexpr double kE1 = 0x1.62e42fefa39e4p-6;
 constexpr double kE2 = 0x1.ebfbdff80fb49p-13;
 constexpr double kE3 = 0x1.c6b08d722f8fbp-20;
 constexpr double kE4 = 0x1.3b2b207411f62p-27;
 constexpr double kE5 = 0x1.5d85c0fe404bap-35;
+// e^r = 1 + r + r^2 (kG2 + ... + kG6 r^4) for |r| <= ln2/64
+constexpr double kG2 = 0.5;
+constexpr double kG3 = 0x1.555555554dd45p-3;
+constexpr double kG4 = 0x1.55555555518a1p-5;
+constexpr double kG5 = 0x1.11114f8a83dabp-7;
+constexpr double kG6 = 0x1.6c17002448c03p-10;
+constexpr double kInvStep = 0x1.71547652b82fep+5;                             // 32 / ln2
+constexpr double kStep = 0x1.62e42fefa39efp-6, kStepLow = 0x1.abc9e3b39803fp-61;  // ln2 / 32
 
 // 2^(lane / 32), correctly rounded.
 __device__ const double kExpTable[32] = {
@@ -125,20 +141,66 @@ __device__ const double kExpTable[32] = {
     0x1.d5818dcfba487p+0, 0x1.dfc97337b9b5fp+0, 0x1.ea4afa2a490dap+0, 0x1.f50765b6e4540p+0,
 };
 
-__device__ __forceinline__ double exp_table_lane() { return kExpTable[threadIdx.x & 31]; }
+// (2^(lane / 32) - kExpTable[lane]) / 2^(lane / 32): upper words, the lower cut off.
+__device__ const unsigned kExpLow[32] = {
+    0x00000000u, 0x3c8cce84u, 0x3c979c64u, 0xbc955912u, 0xbc801ad9u, 0x3c9aebaeu,
+    0x3c968e8eu, 0x3c82f561u, 0x3c8349beu, 0xbc924887u, 0x3c85a416u, 0x3c42e969u,
+    0x3c768e09u, 0xbc78e6b5u, 0x3c90622fu, 0xbc8c2e57u, 0xbc93b5e9u, 0xbc7821c6u,
+    0xbc7b411fu, 0xbc936c49u, 0x3c8db4aau, 0xbc5dd29cu, 0x3c71b24cu, 0xbc91bc2au,
+    0x3c8c1853u, 0xbc68dfe7u, 0x3c736e3au, 0x3c6766f1u, 0x3c74a6c8u, 0xbc82d779u,
+    0xbc8ffb1bu, 0x3c8a60b2u,
+};
 
-// 2^(s/32); every lane of the warp calls it.  table: exp_table_lane().
+// A lane's table entry.
+struct ExpTable {
+    double value;
+    int low;
+};
+
+__device__ __forceinline__ ExpTable exp_table_lane() {
+    return {kExpTable[threadIdx.x & 31], (int)kExpLow[threadIdx.x & 31]};
+}
+
+// e^x; every lane of the warp calls it.  table: exp_table_lane().
+// Results below about 2^-1021 are +0 (the smallest normal numbers and the subnormals),
+// above 2^1024 +inf.  OVER = false: x is known to be below 1024 ln2.
+template <bool OVER>
+__device__ __forceinline__ double exp_f64(double x, const ExpTable& table) {
+    constexpr double kRound = 0x1.8p52;  // adding it rounds to an integer in the low word
+    const double m = fma(x, kInvStep, kRound);
+    const int n = __double2loint(m);
+    const double nd = m - kRound;
+    const double r = fma(-nd, kStepLow, fma(-nd, kStep, x));
+    const double T = __shfl_sync(0xffffffffu, table.value, n);  // source lane n & 31
+    const double low = __hiloint2double(__shfl_sync(0xffffffffu, table.low, n), 0);
+    double q = fma(kG6, r, kG5);
+    q = fma(q, r, kG4);
+    q = fma(q, r, kG3);
+    q = fma(q, r, kG2);
+    q = fma(q, r, 1.0);
+    const double e = fma(T, fma(q, r, low), T);
+    const int top = __double2hiint(x);
+    // n >> 5 into the exponent field, which starts at bit 20
+    int hi = __double2hiint(e) + (n & ~31) * (1 << 15), lo = __double2loint(e);
+    // x <= -1021 ln2, x >= 1024 ln2 (as their top words; infinities too)
+    const bool under = (unsigned)top >= 0xC0861DA0u, over = OVER && top >= 0x40862E42;
+    hi = under ? 0 : over ? 0x7ff00000 : hi;
+    lo = under || over ? 0 : lo;
+    return __hiloint2double(hi, lo);
+}
+
+// 2^(s/32); every lane of the warp calls it.
 // Results below 2^-1021 are +0 (the smallest normal numbers and the
 // subnormals: at most 4.5e-308), above 2^1024 +inf.  s = -inf gives 0; a NaN
 // exponent comes only from NaN parameters, which make every rate NaN in the
 // finish.  OVER = false: s is known to be below 1024 * 32.
 template <bool OVER>
-__device__ __forceinline__ double exp2_32(double s, double table) {
+__device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
     constexpr double kRound = 0x1.8p52;  // s + kRound rounds s to an integer in the low word
     const double m = s + kRound;
     const int n = __double2loint(m);
     const double f = s - (m - kRound);
-    const double T = __shfl_sync(0xffffffffu, table, n);  // source lane n & 31
+    const double T = __shfl_sync(0xffffffffu, table.value, n);  // source lane n & 31
     double q = fma(kE5, f, kE4);
     q = fma(q, f, kE3);
     q = fma(q, f, kE2);
@@ -154,20 +216,28 @@ __device__ __forceinline__ double exp2_32(double s, double table) {
     return __hiloint2double(hi, lo);
 }
 
-// FP64 background term 2^(s/32): the table-driven exponential, or for
-// far-tail tile pairs (every term at most 2^-60, see kFastTailLog2F64) the
-// FP32 hardware exponential.
+// FP64 background term e^x: the table-driven exponential, or for far-tail tile pairs
+// (every term at most 2^-60, see kFastTailLog2F64) the FP32 hardware exponential.
 template <bool FAST>
-__device__ __forceinline__ double background_f64(double s, double table) {
-    if (FAST) return (double)ex2_ftz((float)s * 0.03125f);
-    return exp2_32<false>(s, table);
+__device__ __forceinline__ double background_f64(double x, const ExpTable& table) {
+    if (FAST) return (double)ex2_ftz((float)(x * 1.44269504088896340735992468100189214));
+    return exp_f64<false>(x, table);
 }
 
-template <int D, int R, bool DO_B, bool DO_S, bool MASK, bool FAST = false, bool OVER = true>
+// FP64 self-excitation term.
+template <bool OVER, bool SHORT>
+__device__ __forceinline__ double excitation_f64(const PairConsts& c, double d2, double dt,
+                                                 const ExpTable& table) {
+    if (SHORT) return exp2_32<OVER>(fma(c.eS, d2, c.eW * dt), table);
+    return exp_f64<OVER>(fma(c.cS, d2, c.cW * dt), table);
+}
+
+template <int D, int R, bool DO_B, bool DO_S, bool MASK, bool FAST = false, bool OVER = true,
+          bool SHORT = false>
 __device__ __forceinline__ void body_f64(const double* __restrict__ sRec, int nj,
                                          const double (&xi)[R][D], const double (&ti)[R],
                                          const PairConsts& c, double (&acc)[R][kNumAcc],
-                                         double table) {
+                                         const ExpTable& table) {
     constexpr int S = Layout<D>::kF64Stride;
 #pragma unroll 2
     for (int j = 0; j < nj; ++j) {
@@ -189,13 +259,13 @@ __device__ __forceinline__ void body_f64(const double* __restrict__ sRec, int nj
             const double dt = ti[r] - rj[D];
             if (DO_B) {
                 const double t2 = dt * dt;
-                const double B = background_f64<FAST>(fma(c.eA, d2, c.eB * t2), table);
+                const double B = background_f64<FAST>(fma(c.cA, d2, c.cB * t2), table);
                 acc[r][0] += B;
                 acc[r][1] = fma(B, d2, acc[r][1]);
                 acc[r][2] = fma(B, t2, acc[r][2]);
             }
             if (DO_S) {
-                double Sv = exp2_32<OVER>(fma(c.eS, d2, c.eW * dt), table);
+                double Sv = excitation_f64<OVER, SHORT>(c, d2, dt, table);
                 if (MASK) Sv = dt > 0.0 ? Sv : 0.0;
                 acc[r][3] += Sv;
                 acc[r][4] = fma(Sv, d2, acc[r][4]);
@@ -239,7 +309,7 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
                                              double* __restrict__ sCol,
                                              unsigned long long* __restrict__ colAcc, int Npad,
                                              int j0, int nj, const int (&shift)[3],
-                                             double table) {
+                                             const ExpTable& table) {
     static_assert(kSweepThreads == kTile, "one column per thread in the column flush");
     constexpr int S = Layout<D>::kF64Stride;
     const int tid = threadIdx.x;
@@ -268,7 +338,7 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
                 }
                 const double dt = ti[r] - rj[D];
                 const double t2 = dt * dt;
-                const double B = background_f64<FAST>(fma(c.eA, d2, c.eB * t2), table);
+                const double B = background_f64<FAST>(fma(c.cA, d2, c.cB * t2), table);
                 const double Bd = B * d2, Bt = B * t2;
                 acc[r][0] += B;
                 acc[r][1] += Bd;
@@ -283,7 +353,7 @@ __device__ __forceinline__ void tile_sym_f64(const double* __restrict__ sRec,
                     cp[2][m] += Bt;
                 }
                 if (DO_S) {
-                    double Sv = exp2_32<true>(fma(c.eS, d2, c.eW * dt), table);
+                    double Sv = excitation_f64<true, false>(c, d2, dt, table);
                     if (MASK) Sv = dt > 0.0 ? Sv : 0.0;
                     acc[r][3] += Sv;
                     acc[r][4] = fma(Sv, d2, acc[r][4]);
@@ -365,8 +435,8 @@ __device__ __forceinline__ bool empty_self_item(const double* __restrict__ tileM
 // events) against j tiles [start, jt1); unit pair sums to partial slot item.slot.
 // sym: tiles before the strip are evaluated once per pair (rows + columns).
 // SELF: a self-excitation-only sweep (every problem has noB), with the
-// background's code and sums compiled out.
-template <int D, int R, bool SELF = false>
+// background's code and sums compiled out; SHORT: with the short exponential.
+template <int D, int R, bool SELF = false, bool SHORT = false>
 __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
                                          const double* __restrict__ tileMin,
                                          const double* __restrict__ tileMax,
@@ -391,7 +461,7 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         }
         return;
     }
-    const double table = exp_table_lane();
+    const ExpTable table = exp_table_lane();
     double xi[R][D], ti[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -443,12 +513,15 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         if (SELF) {
             // growing kernels (omega < 0) may overflow; terms of pairs that are
             // not causal may too, but the mask drops them
-            if (c.eW > 0.0)
-                body_f64<D, R, false, true, true>(sRec, nj, xi, ti, c, acc, table);
+            if (c.cW > 0.0)
+                body_f64<D, R, false, true, true, false, true, SHORT>(sRec, nj, xi, ti, c, acc,
+                                                                      table);
             else if (m.allCausal)
-                body_f64<D, R, false, true, false, false, false>(sRec, nj, xi, ti, c, acc, table);
+                body_f64<D, R, false, true, false, false, false, SHORT>(sRec, nj, xi, ti, c, acc,
+                                                                        table);
             else
-                body_f64<D, R, false, true, true, false, false>(sRec, nj, xi, ti, c, acc, table);
+                body_f64<D, R, false, true, true, false, false, SHORT>(sRec, nj, xi, ti, c, acc,
+                                                                       table);
         } else if (sym && m.doB && jt < ts0 && m.fastB) {
             if (!m.doS)
                 tile_sym_f64<D, R, false, false, true>(sRec, xi, ti, c, acc, sCol, colAcc, Npad,
@@ -568,7 +641,7 @@ __device__ __forceinline__ bool next_item(const SweepProblem* problems, const Wo
 // The self-excitation-only form needs 96 registers instead of 168 at R = 2, so five
 // CTAs share an SM instead of three: N = 100k self-excitation sweep 1.37 -> 1.24 ms
 // (with the full underflow distance).
-template <int D, int R, bool SELF>
+template <int D, int R, bool SELF, bool SHORT>
 __global__ void __launch_bounds__(kSweepThreads, (R == 1 ? 4 : 3) + (SELF ? R : 0))
 sweep_f64_list_kernel(const SweepProblem* problems, const WorkItem* items, const int* nItems,
                       int* counter) {
@@ -583,7 +656,7 @@ sweep_f64_list_kernel(const SweepProblem* problems, const WorkItem* items, const
         const SweepProblem& P = problems[w.problem];
         const PairConsts c = P.c;
         const int shift[3] = {P.colShift[0], P.colShift[1], P.colShift[2]};
-        f64_item<D, R, SELF>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
+        f64_item<D, R, SELF, SHORT>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
                        P.nTiles, P.Npad, c, w, sRec,
                        P.symmetric != 0, P.colAcc, shift, sCol);
     }
@@ -1243,12 +1316,15 @@ sweep_f32c_list_kernel(const SweepProblem* problems, const WorkItem* items, cons
 template <int D, int R>
 const void* sweep_list_function(int precision, int V) {
     constexpr int R64 = R > 2 ? 2 : R, R32 = R < 2 ? 2 : R;
-    const bool self = (V & kSelfOnly) != 0;
-    V &= ~kSelfOnly;
+    const bool self = (V & kSelfOnly) != 0, shortExp = (V & kShortExp) != 0;
+    V &= ~(kSelfOnly | kShortExp);
     if (precision == 0) {
         if (R > 2) return nullptr;
-        return self ? reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, true>)
-                    : reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, false>);
+        if (!self) return reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, false, false>);
+        if constexpr (D <= 2)  // beside gridded sums
+            if (shortExp)
+                return reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, true, true>);
+        return reinterpret_cast<const void*>(&sweep_f64_list_kernel<D, R64, true, false>);
     }
     if (R < 2) return nullptr;
     if (self) {
