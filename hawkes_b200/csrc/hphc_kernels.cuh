@@ -82,7 +82,8 @@ struct FinishConsts {
     double prefS;     // theta omega sigma^D / sqrt(2 pi) : S_ij = prefS * S_u
     double bgScale;   // prefB / mu0
     double seScale;   // prefS / theta
-    double accScale[6];  // multiplies the six unit pair sums: undoes the record scaling
+    double accScale[6];  // multiplies the six unit pair sums: undoes the record scaling,
+                         // in FP64 the factor 2^kTermScale of the self-excitation terms,
                          // and, with the hardware exponential, divides out its mean
                          // relative error (1 + beta, measured on the device)
     double T;         // t[N-1]
@@ -141,10 +142,14 @@ constexpr double kFastTailLog2F64 = 60.0;
 // Underflow thresholds (natural-log units) for the tile-pair skip.  FP32:
 // both exponentials return +0 for any argument below -126.5 (log2 units); a
 // true exponent <= -88 is <= -126.96 in log2 units, which the FP32 rounding
-// of the computed exponent (relative ~1e-6) cannot lift above -126.5.  FP64:
-// exp(x) is +0 for x < -745.14; -760 leaves a wide margin.
+// of the computed exponent (relative ~1e-6) cannot lift above -126.5.  FP64: the
+// sweep's exponentials are +0 from -744.44 on, exp(x) below -745.14; -750 leaves a
+// margin for their arguments' rounding.
 constexpr double kSkipF32 = 88.0;
-constexpr double kSkipF64 = 710.0;
+constexpr double kSkipF64 = 750.0;
+// FP64 sweeps hold their self-excitation sums times 2^kTermScale (exp_f64 in
+// hphc_sweep.cuh).
+constexpr int kTermScale = 53;
 
 // Background tail truncation.  Every event's background sum holds its own
 // term, B_ii = 1 unit, the largest of all its terms.  A tile pair whose
@@ -162,7 +167,7 @@ constexpr double kNegligibleLog2F32 = 60.0;
 
 // Self-excitation window.  A term decays as exp(-omega dt), and all but a few
 // events have a close earlier neighbour, so of the earlier events within the
-// underflow distance (710 / omega in FP64, 88 / omega in FP32) nearly all add
+// underflow distance (750 / omega in FP64, 88 / omega in FP32) nearly all add
 // nothing to an event's sum.  There is no term that bounds the sum from below
 // in advance, as B_ii does for the background, so the bound is checked
 // afterwards: the sweep leaves out tile pairs more than x / omega apart, and
@@ -243,7 +248,7 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
         double perE = s.selfDensity / omega;
         for (int k = 0; k < s.D; ++k) perE *= sqrt(2.0) / fabs(sigma);
         const double E = pow((fp32 ? kSelfMissesF32 : kSelfMisses) / perE, 1.0 / (0.5 * s.D + 1.0));
-        // 41.6 = 60 ln 2, 25.0 = 36 ln 2; 6.6 = ln 710
+        // 41.6 = 60 ln 2, 25.0 = 36 ln 2; 6.6 > ln x for every x taken
         const double x = log(s.selfCount) + 6.6 + (fp32 ? 25.0 : 41.6) + E;
         // worth it where it leaves out whole tiles
         if (x < 0.7 * thr && thr - x > 3.0 * omega * s.selfTile) {
@@ -287,6 +292,7 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     f.prefB = f.mu0 * f.bgScale;
     f.prefS = f.theta * f.seScale;
     for (int q = 0; q < kNumAcc; ++q) f.accScale[q] = 1.0;
+    if (!fp32) f.accScale[3] = f.accScale[4] = f.accScale[5] = 1.0 / (1LL << kTermScale);
     if (fp32) {
         f.accScale[1] = f.accScale[4] = 1.0 / (sX * sX);  // sums of d'^2
         f.accScale[2] = 1.0 / (sT * sT);                  // sum of dt'^2

@@ -161,12 +161,20 @@ __device__ __forceinline__ ExpTable exp_table_lane() {
     return {kExpTable[threadIdx.x & 31], (int)kExpLow[threadIdx.x & 31]};
 }
 
-// e^x; every lane of the warp calls it.  table: exp_table_lane().
-// Results below about 2^-1021 are +0 (the smallest normal numbers and the subnormals),
-// above 2^1024 +inf.  OVER = false: x is known to be below 1024 ln2.
-template <bool OVER>
+// Self-excitation terms come times 2^kTermScale, so that a sum of terms of which none is
+// a normal number (an event whose closest earlier neighbours are some 708 to 745
+// exponents away) keeps what a subnormal holds; the finish takes the factor out.
+// It costs nothing: it sits in the rounding constant.
+static_assert(kTermScale == 53, "thresholds below");
+
+// e^x, or (SCALED) e^x 2^kTermScale; every lane of the warp calls it.  table:
+// exp_table_lane().  Results below about 2^-1021 are +0 (unscaled the smallest
+// normal numbers and the subnormals, scaled those that round to 0), above 2^1024 +inf.
+// OVER = false: the result is known to be below that.
+template <bool OVER, bool SCALED>
 __device__ __forceinline__ double exp_f64(double x, const ExpTable& table) {
-    constexpr double kRound = 0x1.8p52;  // adding it rounds to an integer in the low word
+    // adding it rounds to an integer in the low word
+    constexpr double kRound = 0x1.8p52 + (SCALED ? 32 * kTermScale : 0);
     const double m = fma(x, kInvStep, kRound);
     const int n = __double2loint(m);
     const double nd = m - kRound;
@@ -182,21 +190,23 @@ __device__ __forceinline__ double exp_f64(double x, const ExpTable& table) {
     const int top = __double2hiint(x);
     // n >> 5 into the exponent field, which starts at bit 20
     int hi = __double2hiint(e) + (n & ~31) * (1 << 15), lo = __double2loint(e);
-    // x <= -1021 ln2, x >= 1024 ln2 (as their top words; infinities too)
-    const bool under = (unsigned)top >= 0xC0861DA0u, over = OVER && top >= 0x40862E42;
+    // x <= -1021 ln2, x >= 1024 ln2; scaled -1074 ln2 and 971 ln2 (as their top words;
+    // infinities too)
+    const bool under = (unsigned)top >= (SCALED ? 0xC0874385u : 0xC0861DA0u),
+               over = OVER && top >= (SCALED ? 0x4085085E : 0x40862E42);
     hi = under ? 0 : over ? 0x7ff00000 : hi;
     lo = under || over ? 0 : lo;
     return __hiloint2double(hi, lo);
 }
 
-// 2^(s/32); every lane of the warp calls it.
-// Results below 2^-1021 are +0 (the smallest normal numbers and the
-// subnormals: at most 4.5e-308), above 2^1024 +inf.  s = -inf gives 0; a NaN
-// exponent comes only from NaN parameters, which make every rate NaN in the
-// finish.  OVER = false: s is known to be below 1024 * 32.
+// 2^(s/32) 2^kTermScale; every lane of the warp calls it.  Results below 2^-1021 are
+// +0, above 2^1024 +inf.  s = -inf gives 0; a NaN exponent comes only from NaN
+// parameters, which make every rate NaN in the finish.  OVER = false: the result is
+// known to be below 2^1024.
 template <bool OVER>
 __device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
-    constexpr double kRound = 0x1.8p52;  // s + kRound rounds s to an integer in the low word
+    // s + kRound rounds s to an integer in the low word
+    constexpr double kRound = 0x1.8p52 + 32 * kTermScale;
     const double m = s + kRound;
     const int n = __double2loint(m);
     const double f = s - (m - kRound);
@@ -209,8 +219,8 @@ __device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
     const int top = __double2hiint(s);
     // n >> 5 into the exponent field, which starts at bit 20
     int hi = __double2hiint(r) + (n & ~31) * (1 << 15), lo = __double2loint(r);
-    // s <= -1021 * 32 (as its top word; -inf too), s >= 1024 * 32
-    const bool under = (unsigned)top >= 0xC0DFE800u, over = OVER && top >= 0x40E00000;
+    // s <= -1074 * 32 (as its top word; -inf too), s >= 971 * 32
+    const bool under = (unsigned)top >= 0xC0E0C800u, over = OVER && top >= 0x40DE5800;
     hi = under ? 0 : over ? 0x7ff00000 : hi;
     lo = under || over ? 0 : lo;
     return __hiloint2double(hi, lo);
@@ -221,15 +231,15 @@ __device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
 template <bool FAST>
 __device__ __forceinline__ double background_f64(double x, const ExpTable& table) {
     if (FAST) return (double)ex2_ftz((float)(x * 1.44269504088896340735992468100189214));
-    return exp_f64<false>(x, table);
+    return exp_f64<false, false>(x, table);
 }
 
-// FP64 self-excitation term.
+// FP64 self-excitation term, times 2^kTermScale.
 template <bool OVER, bool SHORT>
 __device__ __forceinline__ double excitation_f64(const PairConsts& c, double d2, double dt,
                                                  const ExpTable& table) {
     if (SHORT) return exp2_32<OVER>(fma(c.eS, d2, c.eW * dt), table);
-    return exp_f64<OVER>(fma(c.cS, d2, c.cW * dt), table);
+    return exp_f64<OVER, true>(fma(c.cS, d2, c.cW * dt), table);
 }
 
 template <int D, int R, bool DO_B, bool DO_S, bool MASK, bool FAST = false, bool OVER = true,

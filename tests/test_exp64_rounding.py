@@ -1,5 +1,6 @@
 """The FP64 mode's exponential is as good as a correctly rounded one, so that its sums
-are no further from exact ones than with the library's exp()."""
+are no further from exact ones than with the library's exp(), down to the smallest
+numbers."""
 import numpy as np
 import pytest
 
@@ -76,3 +77,50 @@ def test_probabilities_of_short_exponents():
     rel = ((got[1:] - want[1:]) / want[1:]).astype(float)
     assert np.std(rel) <= 1.6e-16
     assert abs(np.mean(rel)) <= 3 * 2.0 ** -53
+
+
+def _probabilities(t, omega=1.0):
+    """P_i of events at one place, and in long double."""
+    import hawkes_b200 as hb
+    p = np.array([1.0, 1.0, 1.0, omega, 1.0, 1.0])
+    with hb.CudaHawkes(1, len(t), hb.CUDA, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, np.zeros((len(t), 1)))
+        e.setParameters(p)
+        got = e.getProbsSelfExcite().astype(np.longdouble)
+    ld = np.longdouble
+    pi = np.arccos(ld(-1))
+    dt = (t[:, None] - t[None, :]).astype(ld)
+    S = omega * np.where(dt > 0, np.exp(-omega * np.abs(dt)), 0).sum(1) / np.sqrt(2 * pi)
+    B = np.exp(-dt * dt / 2).sum(1) / (2 * pi)
+    return got, S / (B + S)
+
+
+@pytest.mark.gpu
+def test_sums_of_subnormal_terms():
+    # Gaps of 700 to 743 / omega: every sum is one term, most of them subnormal, P_i =
+    # prefS S_i / lambda_i with lambda_i = 1 / (2 pi).  S_i and prefS S_i (prefS = 0.4) are
+    # each rounded to a multiple of 2^-1074, S_i after the term's own last place; the
+    # division multiplies those 1.1 units by 2 pi and rounds once more: 8 units.  The
+    # exponent's rounding is at most 745 * 2^-53 relative.
+    t = np.concatenate([[0.0], np.cumsum(np.linspace(700.0, 743.0, 87))])
+    got, want = _probabilities(t)
+    unit = np.longdouble(2.0) ** -1074
+    assert np.all(np.abs(got - want) <= 8 * unit + 1e-12 * want)
+    assert np.all(got[want > 8 * unit] > 0)
+
+
+@pytest.mark.gpu
+def test_sums_of_subnormal_terms_that_the_finish_completes():
+    # Bursts of 640 events, 720 / omega apart: the first event of each has only terms
+    # of the burst before, which lie outside the self-excitation window.  640 terms,
+    # each rounded to a multiple of 2^-1074, as is their sum.
+    rng = np.random.default_rng(8)
+    t = np.concatenate([720.0 * k + np.sort(rng.uniform(0.0, 1.0, 640)) for k in range(5)])
+    t[::640] = 720.0 * np.arange(5)
+    got, want = _probabilities(t)
+    unit = np.longdouble(2.0) ** -1074
+    first = slice(640, None, 640)
+    assert np.all(want[first] < 1e-307)
+    assert np.all(np.abs(got[first] - want[first]) <= 700 * unit + 1e-12 * want[first])
+    assert np.all(np.abs(got - want)[want > 1e-300] <= 1e-12 * want[want > 1e-300])
