@@ -200,7 +200,7 @@ inline double times_32_log2e(double x, double y) {
     const double p = x * y, pe = fma(x, y, -p);
     const double r = p * kHi;
     const double re = fma(p, kHi, -r) + (p * kLo + pe * kHi);
-    return r + re;
+    return fabs(r) < INFINITY ? r + re : r;
 }
 
 // The parameter-dependent constants of one problem: every PairConsts field
@@ -287,7 +287,10 @@ inline void param_consts(const double* p, const ConstsSpec& s, PairConsts& c, Fi
     f.omega = omega;
     f.theta = p[4];
     f.mu0 = p[5];
-    f.bgScale = aD * b / kTwoPiC;
+    // precisions whose squares overflow make an event's own background term NaN (0 times
+    // infinity), and with it every rate; the FP64 sweep's exponential takes numbers
+    const bool overflows = !fp32 && !(fabs(c.cA) < INFINITY && fabs(c.cB) < INFINITY);
+    f.bgScale = overflows ? NAN : aD * b / kTwoPiC;
     f.seScale = omega * sigmaD * kInvSqrt2PiC;
     f.prefB = f.mu0 * f.bgScale;
     f.prefS = f.theta * f.seScale;

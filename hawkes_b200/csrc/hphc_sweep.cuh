@@ -170,7 +170,7 @@ static_assert(kTermScale == 53, "thresholds below");
 // e^x, or (SCALED) e^x 2^kTermScale; every lane of the warp calls it.  table:
 // exp_table_lane().  Results below about 2^-1021 are +0 (unscaled the smallest
 // normal numbers and the subnormals, scaled those that round to 0), above 2^1024 +inf.
-// OVER = false: the result is known to be below that.
+// OVER = false: the result is known to be below that, and x is a number.
 template <bool OVER, bool SCALED>
 __device__ __forceinline__ double exp_f64(double x, const ExpTable& table) {
     // adding it rounds to an integer in the low word
@@ -196,13 +196,13 @@ __device__ __forceinline__ double exp_f64(double x, const ExpTable& table) {
                over = OVER && top >= (SCALED ? 0x4085085E : 0x40862E42);
     hi = under ? 0 : over ? 0x7ff00000 : hi;
     lo = under || over ? 0 : lo;
+    if (OVER && (top & 0x7fffffff) > 0x7ff00000) hi = 0x7ff80000;  // NaN stays NaN
     return __hiloint2double(hi, lo);
 }
 
 // 2^(s/32) 2^kTermScale; every lane of the warp calls it.  Results below 2^-1021 are
-// +0, above 2^1024 +inf.  s = -inf gives 0; a NaN exponent comes only from NaN
-// parameters, which make every rate NaN in the finish.  OVER = false: the result is
-// known to be below 2^1024.
+// +0, above 2^1024 +inf.  OVER = false: the result is known to be below 2^1024, and s
+// is a number.
 template <bool OVER>
 __device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
     // s + kRound rounds s to an integer in the low word
@@ -223,6 +223,7 @@ __device__ __forceinline__ double exp2_32(double s, const ExpTable& table) {
     const bool under = (unsigned)top >= 0xC0E0C800u, over = OVER && top >= 0x40DE5800;
     hi = under ? 0 : over ? 0x7ff00000 : hi;
     lo = under || over ? 0 : lo;
+    if (OVER && (top & 0x7fffffff) > 0x7ff00000) hi = 0x7ff80000;  // NaN stays NaN
     return __hiloint2double(hi, lo);
 }
 
@@ -522,8 +523,9 @@ __device__ __forceinline__ void f64_item(const double* __restrict__ rec,
         // background bound alone, and such a pair needs no causality mask.
         if (SELF) {
             // growing kernels (omega < 0) may overflow; terms of pairs that are
-            // not causal may too, but the mask drops them
-            if (c.cW > 0.0)
+            // not causal may too, but the mask drops them.  A sigma whose square
+            // overflows makes pairs at one place NaN (0 times infinity)
+            if (!(c.cW <= 0.0 && (SHORT ? c.eS : c.cS) > -INFINITY))
                 body_f64<D, R, false, true, true, false, true, SHORT>(sRec, nj, xi, ti, c, acc,
                                                                       table);
             else if (m.allCausal)
