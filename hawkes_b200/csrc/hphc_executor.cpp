@@ -1301,20 +1301,15 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     key.R = R;
     key.grid = grid;
     key.tablesBytes = tablesBytes_;
-    key.colNeed = colNeed_;
+    const size_t offsets[] = {offSP_, offItems_, offNItems_, offChunks_, offFP_, offFB_, offPJ_};
+    std::copy(std::begin(offsets), std::end(offsets), key.offsets);
     key.tables = dTables_;
     key.timing = kernelTiming;
     key.variant = sweep_variant() | planPrecision_ << 16;
     const int slot = kind_ + (skipPack_ ? 3 : 0);
     cudaGraphExec_t& exec = graphExec_[slot];
     GraphKey& last = graphKey_[slot];
-    const bool same = exec && key.P == last.P && key.nJobs == last.nJobs &&
-                      key.nBlocks == last.nBlocks &&
-                      key.maxN == last.maxN && key.R == last.R &&
-                      key.grid == last.grid && key.tablesBytes == last.tablesBytes &&
-                      key.colNeed == last.colNeed &&
-                      key.tables == last.tables && key.timing == last.timing &&
-                      key.variant == last.variant;
+    const bool same = exec && key == last;
     cudaError_t e;
     if (!same) {
         drop_graph(slot);

@@ -19,6 +19,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <iterator>
 #include <string>
 #include <vector>
 
@@ -220,12 +222,19 @@ private:
     // full evaluations and self-excitation steps captures each once
     // (and, the second three, once more for runs whose records are packed)
     cudaGraphExec_t graphExec_[6] = {};
-    struct GraphKey {
+    struct GraphKey {  // all that the captured launches take from the host
         int P = -1, nJobs = -1, nBlocks = -1, maxN = -1, R = -1, grid = -1;
-        size_t tablesBytes = 0, colNeed = 0;
+        size_t tablesBytes = 0;
+        size_t offsets[7] = {};  // of the tables in the staged block
         void* tables = nullptr;
         int variant = 0;
         bool timing = false;
+        bool operator==(const GraphKey& o) const {
+            return P == o.P && nJobs == o.nJobs && nBlocks == o.nBlocks && maxN == o.maxN &&
+                   R == o.R && grid == o.grid && tablesBytes == o.tablesBytes &&
+                   std::equal(std::begin(offsets), std::end(offsets), std::begin(o.offsets)) &&
+                   tables == o.tables && variant == o.variant && timing == o.timing;
+        }
     } graphKey_[6];
     // What the record pool holds: one set's FP32 records at one scaling.  A plan that
     // needs just those launches no pack: the sampler's sigma and omega steps, which
