@@ -214,6 +214,15 @@ std::map<TuneKey, std::pair<int, int>> gTuneCache;
 // invalid shape are ignored) and appended to after each new tuning.  Each
 // line is written with one append of under 200 bytes, so processes sharing
 // the file do not interleave their lines.
+// Runs of one layout of a self-excitation-only plan that are launched directly before
+// they are captured.  A replay takes about 4 us less than the launches (N = 3000 step
+// 34 : 38 us), the capture 80 to 100 us, so about as much is spent on either by then; a
+// short run of sampler steps captures nothing.  First step after an evaluation,
+// FP32-compensated: N = 3000 114 -> 46 us, N = 100k 977 -> 188 with the buffers reserved
+// (build_plan), 491 before plans were of several kinds.
+// Full sweeps are captured at once (N = 500: the first pass of a new set 134 us, 211
+// where the capture falls into it instead of the set's first evaluation).
+constexpr int kDirectRuns = 20;
 // Tables up to this size go to the device by a kernel that reads the pinned host
 // memory; larger ones by the copy engine.  Self-excitation step at N = 20k 61 -> 52 us,
 // at N = 100k 166 -> 163; evaluation at N = 500 36.9 -> 35.8, N = 5000 84 -> 76 (FP64).
@@ -375,6 +384,7 @@ void Executor::drop_graph(int kind) {
     if (graphExec_[kind]) cudaGraphExecDestroy(graphExec_[kind]);
     graphExec_[kind] = nullptr;
     graphKey_[kind] = GraphKey{};
+    directRuns_[kind] = 0;
 }
 
 void Executor::release() {
@@ -938,10 +948,11 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
     offPJ_ = align16(offFB_ + sizeof(FinishBlock) * pl.fb.size());
     tablesBytes_ = align16(offPJ_ + sizeof(PackJob) * pl.pj.size());
 
-    // an FP64 plan of an FP32-compensated engine reserves the records its
-    // self-excitation steps will pack
+    // an FP64 plan of an FP32-compensated engine reserves what its self-excitation
+    // steps will take: the records they pack, and the partial sums of strips twice as
+    // high, which have half the items' tiles and twice the slots
     recNeed_ = planPrecision_ == precision_ ? recOff : (size_t)pl.maxN * S32;
-    partialsNeed_ = partOff;
+    partialsNeed_ = planPrecision_ == precision_ ? partOff : 2 * partOff;
     colNeed_ = colOff;
     int st = ensure_buffers();
     if (st) return st;
@@ -1309,10 +1320,21 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     const int slot = kind_ + (skipPack_ ? 3 : 0);
     cudaGraphExec_t& exec = graphExec_[slot];
     GraphKey& last = graphKey_[slot];
-    const bool same = exec && key == last;
     cudaError_t e;
-    if (!same) {
+    if (!(key == last)) {
         drop_graph(slot);
+        last = key;
+    }
+    // The first runs of a self-excitation-only plan are launched directly
+    if (!exec && selfOnly_ && !kernelTiming && directRuns_[slot] < kDirectRuns) {
+        ++directRuns_[slot];
+        if (take_fault(HPHC_FAULT_LAUNCH))
+            return cuda_fail(cudaErrorLaunchOutOfResources, "launch kernels (injected)");
+        st = launch_sequence(grid);
+        lastLaunches += gridLaunches_;
+        return st;
+    }
+    if (!exec) {
         cudaGraph_t graph = nullptr;
         if ((e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal)))
             return cuda_fail(e, "begin graph capture");
@@ -1331,7 +1353,6 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
             exec = nullptr;
             return cuda_fail(e, "instantiate graph");
         }
-        last = key;
     }
     if (take_fault(HPHC_FAULT_LAUNCH))
         return cuda_fail(cudaErrorLaunchOutOfResources, "launch graph (injected)");
