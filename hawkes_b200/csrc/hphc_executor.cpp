@@ -214,19 +214,6 @@ std::map<TuneKey, std::pair<int, int>> gTuneCache;
 // invalid shape are ignored) and appended to after each new tuning.  Each
 // line is written with one append of under 200 bytes, so processes sharing
 // the file do not interleave their lines.
-// Runs of one layout of a self-excitation-only plan that are launched directly before
-// they are captured.  A replay takes about 4 us less than the launches (N = 3000 step
-// 34 : 38 us), the capture 80 to 100 us, so about as much is spent on either by then; a
-// short run of sampler steps captures nothing.  First step after an evaluation,
-// FP32-compensated: N = 3000 114 -> 46 us, N = 100k 977 -> 188 with the buffers reserved
-// (build_plan), 491 before plans were of several kinds.
-// Full sweeps are captured at once (N = 500: the first pass of a new set 134 us, 211
-// where the capture falls into it instead of the set's first evaluation).
-constexpr int kDirectRuns = 20;
-// Tables up to this size go to the device by a kernel that reads the pinned host
-// memory; larger ones by the copy engine.  Self-excitation step at N = 20k 61 -> 52 us,
-// at N = 100k 166 -> 163; evaluation at N = 500 36.9 -> 35.8, N = 5000 84 -> 76 (FP64).
-constexpr size_t kCopyKernelBytes = 64 << 10;
 constexpr int kTuneCacheVersion = 1;
 constexpr int kTuneReps = 4;  // timed sweeps per candidate shape (even)
 
@@ -321,6 +308,11 @@ void append_tune_file(const std::string& device, int sms, const TuneKey& key, in
     std::fclose(f);
 }
 
+// Tables up to this size go to the device by a kernel that reads the pinned host
+// memory; larger ones by the copy engine.  Self-excitation step at N = 20k 61 -> 52 us,
+// at N = 100k 166 -> 163; evaluation at N = 500 36.9 -> 35.8, N = 5000 84 -> 76 (FP64).
+constexpr size_t kCopyKernelBytes = 64 << 10;
+
 // Gridded background sums: cost estimates (plan_grid) and limits.  Microseconds
 // from measured times (one B200): the background terms of the sweeps took, at
 // N = 100k, 6.86 ms for 3.38e9 pairs in FP64 and 2.42 ms for 2.89e9 in FP32; the
@@ -384,7 +376,7 @@ void Executor::drop_graph(int kind) {
     if (graphExec_[kind]) cudaGraphExecDestroy(graphExec_[kind]);
     graphExec_[kind] = nullptr;
     graphKey_[kind] = GraphKey{};
-    directRuns_[kind] = 0;
+    met_[kind] = false;
 }
 
 void Executor::release() {
@@ -1325,9 +1317,14 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
         drop_graph(slot);
         last = key;
     }
-    // The first runs of a self-excitation-only plan are launched directly
-    if (!exec && selfOnly_ && !kernelTiming && directRuns_[slot] < kDirectRuns) {
-        ++directRuns_[slot];
+    // A step on kept sums is captured the second time its layout comes, so that a first
+    // step costs no capture: first step after an evaluation, FP32-compensated, N = 3000
+    // 114 -> 48 us, N = 100k 977 -> 188 with its buffers reserved (build_plan).  A replay
+    // takes 4 us less than the launches (N = 3000: 34 against 38 us), the capture 80 to
+    // 100.  Evaluations are captured at once (N = 500: the first pass of a new set 134
+    // us, 211 where the capture falls into it instead of the set's first evaluation).
+    if (!exec && keptB && !kernelTiming && !met_[slot]) {
+        met_[slot] = true;
         if (take_fault(HPHC_FAULT_LAUNCH))
             return cuda_fail(cudaErrorLaunchOutOfResources, "launch kernels (injected)");
         st = launch_sequence(grid);

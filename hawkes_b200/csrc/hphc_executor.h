@@ -236,7 +236,7 @@ private:
                    tables == o.tables && variant == o.variant && timing == o.timing;
         }
     } graphKey_[6];
-    int directRuns_[6] = {};  // of the key's layout, without a graph
+    bool met_[6] = {};  // the key's layout has run without a graph
     // What the record pool holds: one set's FP32 records at one scaling.  A plan that
     // needs just those launches no pack: the sampler's sigma and omega steps, which
     // leave events, tauX and tauT alone.
