@@ -349,6 +349,7 @@ int Executor::cuda_fail(cudaError_t e, const char* what) {
     stale_ = true;
     packed_ = Packed{};
     error = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();  // a failed allocation is not the next launch's error
     return e == cudaErrorMemoryAllocation ? HPHC_ERR_OUT_OF_MEMORY : HPHC_ERR_CUDA;
 }
 
@@ -393,11 +394,7 @@ void Executor::release() {
     if (dArrived_) cudaFree(dArrived_);
     dArrived_ = nullptr;
     arrivedCap_ = 0;
-    if (dGridSums_) cudaFree(dGridSums_);
-    if (dGridWork_) cudaFree(dGridWork_);
-    dGridSums_ = nullptr;
-    dGridWork_ = nullptr;
-    gridSumsCap_ = gridWorkCap_ = 0;
+    release_grid();
     for (auto& ev : ev_)
         if (ev) cudaEventDestroy(ev);
     dTables_ = hStaging_ = nullptr;
@@ -1255,15 +1252,23 @@ double Executor::self_terms(const SetView& s, const double* p) const {
     return tiles / n * kTile * s.N;
 }
 
-int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const double* params,
-                      int P, double* dProbs) {
-    if (P < 1) {
-        error = "no problems to evaluate";
-        return HPHC_ERR_BAD_ARGUMENT;
-    }
-    // the choice of the grid asks for the engine's own cuts, not those of the plan before
-    planPrecision_ = precision_;
-    plan_grid(sets, setOf, params, P);
+// The memory of the gridded sums given back, the problems planned for them to the pair
+// sweep; false if there is none.
+bool Executor::release_grid() {
+    if (!dGridWork_ && !dGridSums_) return false;
+    cudaFree(dGridWork_);  // waits for kernels in flight
+    cudaFree(dGridSums_);
+    dGridSums_ = nullptr;
+    dGridWork_ = nullptr;
+    gridSumsCap_ = gridWorkCap_ = 0;
+    gridOf_.clear();
+    return true;
+}
+
+// Precision, shape and tables of a run whose gridded problems are chosen; starts their
+// sums.
+int Executor::plan(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                   int P, double* dProbs) {
     // Large gridded evaluations of the FP32-compensated mode sweep their
     // self-excitation terms in FP64 too, where that is a small part of them: the
     // grid's sums are exact to 1e-15, and the sweep's 0.19 instead of 0.13 ms at
@@ -1271,6 +1276,7 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     // worst gradient component 9.6e-10 -> 3.6e-15 relative).  Where the terms are
     // many they stay in FP32 (N = 500k clustered: 2.2 against 4.1 ms, beside 2.0 ms
     // of grid kernels).
+    planPrecision_ = precision_;
     if (precision_ == HPHC_PRECISION_FP32_COMP && !keptB && self_only(P)) {
         bool large = true;
         for (int p = 0; p < P; ++p)
@@ -1286,7 +1292,22 @@ int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const 
     gridLaunches_ = 0;
     const bool faulty = faultStage == HPHC_FAULT_LAUNCH && faultCount > 0;
     if (!faulty && (st = launch_grid(sets, setOf, params, P))) return st;
-    st = build_plan(sets, setOf, params, P, dProbs, R, itemsPerSM);
+    return build_plan(sets, setOf, params, P, dProbs, R, itemsPerSM);
+}
+
+int Executor::enqueue(const std::vector<SetView>& sets, const int* setOf, const double* params,
+                      int P, double* dProbs) {
+    if (P < 1) {
+        error = "no problems to evaluate";
+        return HPHC_ERR_BAD_ARGUMENT;
+    }
+    // the choice of the grid asks for the engine's own cuts, not those of the plan before
+    planPrecision_ = precision_;
+    plan_grid(sets, setOf, params, P);
+    int st = plan(sets, setOf, params, P, dProbs);
+    // short of memory: again with the pair sweep, without what the grid holds
+    if (st == HPHC_ERR_OUT_OF_MEMORY && release_grid())
+        st = plan(sets, setOf, params, P, dProbs);
     if (st) return st;
     const int grid = sweep_grid(R);
     timedValid = false;
@@ -1402,6 +1423,8 @@ int Executor::setup_device_loop(const std::vector<SetView>& sets, const int* set
     if (st) return st;
     wideBands_ = true;
     st = build_plan(sets, setOf, params, P, nullptr, R, itemsPerSM);
+    if (st == HPHC_ERR_OUT_OF_MEMORY && release_grid())
+        st = build_plan(sets, setOf, params, P, nullptr, R, itemsPerSM);
     wideBands_ = false;
     if (st) return st;
     drop_graphs();  // the tables' layout changed under any captured graph

@@ -255,6 +255,9 @@ private:
     void plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
                    int P);
     double* grid_sums(int p) const;
+    bool release_grid();
+    int plan(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,
+             double* dProbs);
     double self_terms(const SetView& s, const double* p) const;
     bool self_only(int P) const;  // no problem of the plan has background terms to sweep
     bool self_listless(const std::vector<SetView>& sets, const int* setOf, int P) const;

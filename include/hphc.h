@@ -95,7 +95,7 @@ extern "C" {
                                                 self-excitation window */
 
 /* How the last evaluation was computed (hphc_get_last_evaluation_path). */
-#define HPHC_PATH_SWEEP 0        /* the O(N^2) pair sweep                             */
+#define HPHC_PATH_SWEEP 0        /* every sum anew: pair sweep, or grid and self-excitation */
 #define HPHC_PATH_INCREMENTAL 1  /* kept sums updated for moved events, O(N) each     */
 #define HPHC_PATH_KEPT_SUMS 2    /* nothing changed since the sums were kept: O(N) finish */
 #define HPHC_PATH_SELF_EXCITATION 3 /* kept background sums (same events, tauX, tauT):
@@ -122,6 +122,14 @@ typedef struct hphc_engine hphc_engine;
  * (src/factory.cpp:34, :45); otherwise plain FP64.  device: CUDA device ordinal; a value < 0 or
  * beyond the device count selects device 0, as the OpenCL engine falls back to
  * the default device (src/backend/opencl/OpenCLHawkes.hpp:88-92).
+ *
+ * Device memory is O(N D), but for evaluations with gridded background sums: their
+ * workspace takes about 1 KB an event and 16 bytes a grid node, at most 8 GiB for one
+ * problem (and 1 GiB for a group of smaller ones), with a quarter more allocated.  It
+ * is the engine's own, grows with the largest evaluation and is given back with the
+ * engine, or earlier if one of its own later allocations fails; an evaluation that
+ * does not get it, or that would be left without memory for the rest, takes the pair
+ * sweep.  HPHC_FLAG_NO_TAIL_TRUNCATION engines have none.
  */
 int hphc_create(int embeddingDimension, int locationCount, long flags, int device,
                 hphc_engine** out);
