@@ -191,6 +191,7 @@ struct EventSet {
     RowOrder order2, order4;
     bool packedF64 = false;                   // FP32-compensated mode
     uint64_t version = 0;                     // of the device's events (changed())
+    double tiedGap = 0.0;              // derive_times, see SetView
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 
@@ -294,6 +295,37 @@ struct EventSet {
         dOrder4.release();
     }
 
+    // The time from a tied event back to the last earlier time, as seven in eight of up
+    // to 32 tiles' first events have it or less; 0 unless one in eight is tied with the
+    // event before it (then no event beyond those the tile bounds read is looked at).
+    double tied_gap() const {
+        const double* t = hTimes.p;
+        const int nTiles = (N + kTile - 1) / kTile, step = std::max(1, nTiles / 32);
+        double gaps[64];
+        int n = 0;
+        for (int k = 1; k < nTiles && n < 64; k += step, ++n) {
+            const double v = t[k * kTile];
+            int last = k * kTile - 1;  // with a time other than v, once found
+            if (t[last] != v) {
+                gaps[n] = 0.0;
+                continue;
+            }
+            int reach = 1;
+            while (reach <= last && t[last - reach] == v) reach *= 2;
+            int tied = last - reach / 2;  // latest known tie
+            last = std::max(-1, last - reach);
+            while (tied - last > 1) {
+                const int mid = last + (tied - last) / 2;
+                (t[mid] == v ? tied : last) = mid;
+            }
+            gaps[n] = last < 0 ? 0.0 : std::fabs(v - t[last]);
+        }
+        if (n == 0) return 0.0;
+        double* at = gaps + n * 7 / 8;
+        std::nth_element(gaps, at, gaps + n);
+        return *at;
+    }
+
     // Host-side derived data of the times: sortedness, dense ranks (equal
     // times share a rank: the exact strict-causality mask of the FP32
     // records), per-tile bounds.  Sorted times (the usual case) take one pass
@@ -314,8 +346,10 @@ struct EventSet {
                 hTileMin[k] = t[k * kTile];
                 hTileMax[k] = t[std::min(N, (k + 1) * kTile) - 1];
             }
+            tiedGap = tied_gap();
             return;
         }
+        tiedGap = tied_gap();
         std::vector<int> idx(N);
         std::iota(idx.begin(), idx.end(), 0);
         std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return t[x] < t[y]; });
@@ -396,6 +430,7 @@ struct EventSet {
         v.hTileMin = hTileMin.data();
         v.hTileMax = hTileMax.data();
         v.sorted = sorted;
+        v.tiedGap = tiedGap;
         v.haveBox = haveBox;
         for (int k = 0; k < D; ++k) {
             v.locMin[k] = locMin[k];

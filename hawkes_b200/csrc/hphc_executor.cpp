@@ -446,6 +446,7 @@ ConstsSpec Executor::consts_spec(const SetView& set, double omega) const {
                                : *std::max_element(set.hTileMax, set.hTileMax + nTiles) -
                                      *std::min_element(set.hTileMin, set.hTileMin + nTiles);
     s.selfTile = volume / nTiles;
+    s.selfGap = set.tiedGap;
     double ball = 1.0;  // V_D = V_{D-2} 2 pi / D
     for (int d = D_; d > 1; d -= 2) ball *= 2.0 * M_PI / d;
     if (D_ % 2) ball *= 2.0;

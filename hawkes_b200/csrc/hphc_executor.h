@@ -53,6 +53,9 @@ struct SetView {
     const double* hTileMin = nullptr;
     const double* hTileMax = nullptr;
     bool sorted = false;               // times ascending (bands are contiguous)
+    // Where events share their times (dates, say): the time that most of them lie after
+    // the last earlier one; else 0.
+    double tiedGap = 0.0;
     bool haveBox = false;              // bounds of the coordinates
     double locMin[kMaxDim] = {}, locMax[kMaxDim] = {};
 };
