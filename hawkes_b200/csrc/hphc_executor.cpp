@@ -325,6 +325,7 @@ constexpr size_t kCopyKernelBytes = 64 << 10;
 // that take the same either way with the sweep.
 constexpr double kPairCostF64 = 2.05e-6, kPairCostF32 = 1.1e-6;  // a pair
 constexpr double kSelfCostF64 = 1.9e-6;  // a self-excitation term
+constexpr double kLongSelfTerms = 3e8;   // FP64 sweeps of so many take strips twice as high
 struct GridCost {
     double event, node, fixed;  // fixed: of a group of problems
 };
@@ -715,6 +716,10 @@ int Executor::build_plan(const std::vector<SetView>& sets, const int* setOf, con
         }
         const double perItem = bandTiles / (4.0 * sweep_grid(r));
         selfTiles = std::min(widest, std::max(1, (int)std::lround(perItem)));
+        // Long items leave a last wave: there three times as many (N = 70k, omega =
+        // 0.001, every earlier tile: 3105 -> 2987 us FP32-compensated, where a list,
+        // longest first, took 2986)
+        if (selfTiles > 8) selfTiles = std::max(8, selfTiles / 3);
         selfShift = part_shift(perItem);
         if (wideBands_) {  // for any sigma and omega
             widest = nTiles;
@@ -1214,11 +1219,15 @@ int Executor::choose_shape(const std::vector<SetView>& sets, const int* setOf,
         // a few thousand events: more, smaller strips fill the SMs
         if (!fixedR && sets[setOf[0]].N <= 8192) s.R = precision_ == HPHC_PRECISION_FP64 ? 1 : 2;
     }
-    // without a list there is one question left, and the smaller strips answer it:
-    // R = 2 against 4 in FP32 0.125 : 0.155 ms at N = 100k and 1.15 : 1.30 at 400k, R = 1
-    // against 2 in FP64 0.041 : 0.055 ms at N = 30k and 2.12 : 2.09 at 400k
+    // without a list there is one question left: R = 2 against 4 in FP32 0.125 : 0.155 ms
+    // at N = 100k and 1.15 : 1.30 at 400k; R = 1 against 2 in FP64 50 : 56 us at N = 20k
+    // and 261 : 269 at 100k (1e8 terms), but 1.33 : 1.26 ms at N = 70k and omega = 0.05
+    // (7e8 terms), 2.59 : 2.46 at 400k (1.6e9) and 5.08 : 4.73 where N = 70k takes all
     if (!s.tuned && selfOnly_ && self_listless(sets, setOf, P)) {
-        R = fixedR ? fixedR : planPrecision_ == HPHC_PRECISION_FP64 ? 1 : 2;
+        R = fixedR ? fixedR : 2;
+        if (!fixedR && planPrecision_ == HPHC_PRECISION_FP64 &&
+            P * self_terms(sets[setOf[0]], params) < kLongSelfTerms)
+            R = 1;
         itemsPerSM = fixedItems ? fixedItems : 8;
         return HPHC_OK;
     }

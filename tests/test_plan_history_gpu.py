@@ -103,3 +103,18 @@ def test_plan_after_an_event_has_been_far_away(flags, n):
         got, want = _evaluate(e, p), fresh(inward)
         assert got[2] == want[2] == 0.0
         assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("n,omega,R", [(40000, 1.0, 1), (40000, 0.001, 2), (20000, 0.001, 1)])
+def test_strip_height_of_fp64_self_excitation_sweeps(n, omega, R):
+    # two rows a thread where the terms are many (8e8 here), one where the sweep is short
+    # (2e8 and less)
+    loc, t = workloads.uniform(n, 14)
+    p = np.asarray(workloads.BASE_PARAMS) * np.array([1, 1, 1, omega, 1, 1])
+    with hb.CudaHawkes(2, n, FP64, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        assert _evaluate(e, p)[2] == 0.0  # gridded: self-excitation only
+        e.setParameters(p * np.array([1.1, 1, 1, 1, 1, 1]))
+        e.getLogLikelihoodAndGradient()
+        assert e.lastEvaluationPath == hb.PATH_SELF_EXCITATION and e.sweepShape()[0] == R
