@@ -50,8 +50,8 @@ def _exact(loc, t, which):
 @pytest.mark.parametrize("flags,pause", [(FP64, 100.0), (FP32C, 60.0)], ids=["fp64", "fp32c"])
 def test_sums_outside_the_window_are_completed(flags, pause, blocks):
     # The window ends at 40 to 45 (FP32-compensated) or about 60 (FP64) exponents, where
-    # terms reach to 88 or 750: between half and a tenth of the terms remain, 0.75 leaves
-    # room for the strips' heights.  The completed sums are FP64 sums of exp(): the
+    # terms reach to 88 or 750: between half and a tenth of the terms remain, and whole
+    # tiles at the edges, of strips of one height at most 0.75.  The completed sums are FP64 sums of exp(): the
     # exponent's rounding, 100 * 2^-52 = 2e-14, and the sum's; the background sum has the
     # mode's rounding, 2^-24 in the FP32-compensated mode.
     loc, t, low = _events(pause, blocks)
@@ -62,7 +62,7 @@ def test_sums_outside_the_window_are_completed(flags, pause, blocks):
             e.updateLocations(-1, loc)
             e.setParameters(PARAMS)
             ll, g = e.getLogLikelihoodAndGradient()
-            terms = e.lastLaunchStats()[2]
+            terms = e.lastLaunchStats()[2], e.sweepShape()[0]
             got[name] = ll, np.asarray(g), e.getProbsSelfExcite(), terms
             if name == "window":  # the step's window is the same
                 e.setParameters(PARAMS * np.array([1.01, 1, 1, 1, 1, 1]))
@@ -70,8 +70,8 @@ def test_sums_outside_the_window_are_completed(flags, pause, blocks):
                 e.setParameters(PARAMS)
                 e.getLogLikelihoodAndGradient()
                 step = e.getProbsSelfExcite()
-    (lw, gw, pw, nw), (lf, gf, pf, nf) = got["window"], got["full"]
-    assert nw < 0.75 * nf
+    (lw, gw, pw, (nw, rw)), (lf, gf, pf, (nf, rf)) = got["window"], got["full"]
+    assert nw < (0.75 * nf if rw == rf else nf)
     want = _exact(loc, t, low)
     assert np.all(want < (1e-20 if flags == FP32C else 1e-40))
     rtol = 1e-12 if flags == FP64 else 2.0 ** -23
