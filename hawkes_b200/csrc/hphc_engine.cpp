@@ -765,6 +765,7 @@ struct hphc_engine {
         if (st) return st;
         if (rt.ex.selfWindow) set.update_box(hLoc[curLoc].p);
         std::vector<SetView> sets{set.view()};
+        sets[0].hLoc = hLoc[curLoc].p;
         std::vector<int> setOf(K, 0);
         // the evaluation keeps problem 0's sums (a self-excitation-only sweep
         // rewrites rows 3-5 and keeps rows 0-2)
@@ -1549,6 +1550,7 @@ int hphc_multiset_log_likelihood_and_gradient(hphc_multiset* m, const double* pa
             m->dirty[s] = 0;
         }
         views[s] = m->sets[s].view();
+        views[s].hLoc = m->hLoc[s].p;
     }
     std::vector<int> setOf(m->S);
     std::iota(setOf.begin(), setOf.end(), 0);

@@ -328,8 +328,16 @@ constexpr double kSelfCostF64 = 1.9e-6;  // a self-excitation term
 constexpr double kLongSelfTerms = 3e8;   // FP64 sweeps of so many take strips twice as high
 struct GridCost {
     double event, node, fixed;  // fixed: of a group of problems
+    double spread;              // the spread kernel's part of `event`
 };
-constexpr GridCost kGridCost16{3.45e-3, 5.0e-5, 95.0}, kGridCost12{3.2e-3, 5.0e-5, 140.0};
+constexpr GridCost kGridCost16{3.45e-3, 5.0e-5, 95.0, 1.9e-3},
+    kGridCost12{3.2e-3, 5.0e-5, 140.0, 1.3e-3};
+// Where the events crowd: an event of the fullest tile, a pair of events of one bin.  All
+// events in one bin, as at a tenth of the usual precisions: N = 12k, 20k and 30k 0.80,
+// 1.27 and 1.85 ms (0.75, 1.26 and 1.8 with these), 100k 10.7 (11); a fraction c = 0.16,
+// 0.44 and 0.79 on a tile at N = 30k 0.44, 0.72 and 1.12 ms (0.39, 0.74, 1.2).  Without
+// them N = 20k at a tenth of the precisions took 1.18 ms on the grid, 0.66 as pairs.
+constexpr double kGridSerial = 0.03, kGridRank = 0.68e-6;
 constexpr int kGridMinEvents = 1000;
 constexpr double kGridMaxNodes = 4e8;
 constexpr size_t kGridMaxWork = size_t(8) << 30;    // one problem's workspace
@@ -507,6 +515,51 @@ double* Executor::grid_sums(int p) const {
     return p == 0 && sumsOut ? sumsOut : dGridSums_ + gridSumsOff_[p];
 }
 
+// One event of each of kCrowdSample equal parts of the set, the place in the part
+// scattered so that sites taken in turn do not coincide with it.
+Executor::CrowdSample Executor::crowd_sample(const SetView& s) const {
+    CrowdSample c{};
+    const int part = std::max(1, s.N / kCrowdSample);
+    for (int k = 0; k < kCrowdSample; ++k) {
+        const unsigned scatter = (unsigned)k * 2654435761u >> 8;
+        const int i = std::min(s.N - 1, (int)((long long)s.N * k / kCrowdSample) +
+                                            (int)(scatter % (unsigned)part));
+        c.at[0][k] = (float)(s.hTimes[i] - s.hTileMin[0]);
+        c.at[1][k] = (float)(s.hLoc[(size_t)i * D_] - s.locMin[0]);
+        c.at[2][k] = D_ == 2 ? (float)(s.hLoc[(size_t)i * 2 + 1] - s.locMin[1]) : 0.0f;
+    }
+    return c;
+}
+
+// Shares of the events within 12 cells (those that touch a tile of nodes) and 4 cells
+// (a bin) of an event in every coordinate, of the densest part: the second moment of
+// the shares about sampled events over the first, each without bias from counting the
+// event itself.
+Executor::Crowd Executor::crowd(const CrowdSample& c, int order, double a, double b) const {
+    const double unit = (order == 16 ? GridOrder<16>::kInv : GridOrder<12>::kInv) / std::sqrt(2.0);
+    const float tt = (float)(12.0 / (unit * std::fabs(b))), tx = (float)(12.0 / (unit * std::fabs(a)));
+    const float bt = tt / 3.0f, bx = tx / 3.0f;
+    double first[2] = {0.0, 0.0}, second[2] = {0.0, 0.0};
+    for (int i = 0; i < kCrowdSample; ++i) {
+        const float t = c.at[0][i], x = c.at[1][i], y = c.at[2][i];
+        int nt = -1, nb = -1;  // the event itself
+        for (int j = 0; j < kCrowdSample; ++j) {
+            const float dt = std::fabs(c.at[0][j] - t), dx = std::fabs(c.at[1][j] - x),
+                        dy = std::fabs(c.at[2][j] - y);
+            nt += (dt <= tt) & (dx <= tx) & (dy <= tx);
+            nb += (dt <= bt) & (dx <= bx) & (dy <= bx);
+        }
+        first[0] += nt;
+        first[1] += nb;
+        second[0] += nt * (nt - 1.0);
+        second[1] += nb * (nb - 1.0);
+    }
+    Crowd r;
+    if (first[0] > 0.0) r.tile = second[0] / ((kCrowdSample - 2) * first[0]);
+    if (first[1] > 0.0) r.bin = second[1] / ((kCrowdSample - 2) * first[1]);
+    return r;
+}
+
 // Which problems take their background sums from a grid: those whose estimated
 // time on it (fixed, shared by the problems of a launch, per event and per node)
 // is below that of the pairs the sweep would evaluate, counted from sampled tiles
@@ -522,6 +575,8 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
     std::vector<size_t> off(P, 0);
     size_t sums = 0, work = 0;
     bool any = false;
+    CrowdSample sample;
+    int sampled = -1;  // its set
     for (int p = 0; p < P; ++p) {
         const SetView& s = sets[setOf[p]];
         const double* prm = params + (size_t)6 * p;
@@ -549,8 +604,21 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
         const double direct = pairs * (fp32 ? kPairCostF32 : kPairCostF64);
         const int order = fp32 && s.N < kGridHighOrderEvents ? 12 : 16;
         const GridCost& cost = order == 16 ? kGridCost16 : kGridCost12;
-        const double maxNodes =
-            (direct - cost.fixed / std::min(P, kGridMaxJobs) - s.N * cost.event) / cost.node;
+        const double jobs = std::min(P, kGridMaxJobs);
+        double room = direct - cost.fixed / jobs - s.N * cost.event;
+        if (!(room > 0.0)) continue;
+        // A tile's events go through one CTA, a few tiles' through a few, and a bin's are
+        // ranked against each other: wide kernels and clusters.
+        if (s.hLoc) {
+            if (sampled != setOf[p]) {
+                sample = crowd_sample(s);
+                sampled = setOf[p];
+            }
+            const Crowd share = crowd(sample, order, prm[1], prm[2]);
+            room -= std::max(0.0, s.N * (share.tile * kGridSerial / jobs - cost.spread)) +
+                    kGridRank * share.bin * s.N * (double)s.N;
+        }
+        const double maxNodes = room / cost.node;
         if (!(maxNodes > 0.0)) continue;
         const double lo[3] = {tMin, D_ == 2 ? s.locMin[1] : 0.0, s.locMin[0]};
         const double hi[3] = {tMax, D_ == 2 ? s.locMax[1] : 0.0, s.locMax[0]};

@@ -49,7 +49,8 @@ struct SetView {
     bool* packedF64 = nullptr;         // FP32-compensated: whether they hold the present events
     const double* dTileMin = nullptr;  // per-tile time bounds
     const double* dTileMax = nullptr;
-    const double* hTimes = nullptr;    // host copies
+    const double* hLoc = nullptr;      // host copies; hLoc may be missing (shards)
+    const double* hTimes = nullptr;
     const double* hTileMin = nullptr;
     const double* hTileMax = nullptr;
     bool sorted = false;               // times ascending (bands are contiguous)
@@ -257,6 +258,16 @@ private:
     int ensure_buffers();
     void plan_grid(const std::vector<SetView>& sets, const int* setOf, const double* params,
                    int P);
+    // how densely a set's events lie on a problem's grid (plan_grid)
+    struct Crowd {
+        double tile = 0.0, bin = 0.0;  // share of the events that touch a tile, lie in a bin
+    };
+    static constexpr int kCrowdSample = 32;
+    struct CrowdSample {
+        float at[3][kCrowdSample];  // t, x, y of events spread over the set
+    };
+    CrowdSample crowd_sample(const SetView& s) const;
+    Crowd crowd(const CrowdSample& c, int order, double a, double b) const;
     double* grid_sums(int p) const;
     bool release_grid();
     int plan(const std::vector<SetView>& sets, const int* setOf, const double* params, int P,

@@ -118,3 +118,21 @@ def test_strip_height_of_fp64_self_excitation_sweeps(n, omega, R):
         e.setParameters(p * np.array([1.1, 1, 1, 1, 1, 1]))
         e.getLogLikelihoodAndGradient()
         assert e.lastEvaluationPath == hb.PATH_SELF_EXCITATION and e.sweepShape()[0] == R
+
+
+@pytest.mark.parametrize("flags,D,n", [(FP64, 2, 12000), (FP64, 1, 20000), (FP32C, 1, 20000),
+                                       (FP32C, 2, 30000), (FP32C, 2, 70000)])
+def test_crowded_events_keep_the_pair_sweep(flags, D, n):
+    # Kernels ten times as wide put all events into a few bins of the grid, whose CTAs
+    # then take them one after the other: up to 2.6 times the pair sweep's time.  The
+    # larger of these sets are cheaper on the grid at the usual widths.
+    loc, t = workloads.uniform(n, 15, D=D)
+    p = np.asarray(workloads.BASE_PARAMS)
+    wide = p * np.array([1, 0.05, 0.05, 1, 1, 1])
+    with hb.CudaHawkes(D, n, flags, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        assert _evaluate(e, wide)[2] > 0.0
+        if n > 20000:
+            assert _evaluate(e, p)[2] == 0.0
+        assert _evaluate(e, wide * 1.001)[2] > 0.0
