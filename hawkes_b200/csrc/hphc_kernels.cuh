@@ -424,7 +424,10 @@ struct SweepProblem {
     // all problems), there problem (k % slotItems) / strips and its strip, and of
     // that strip's tiles, counted back from its own last one, the chunkTiles of the
     // slot.
+    // slotsUsed: the slots of each strip that may hold terms (the others are neither
+    // written nor read), or null: all of them.
     int slotItems, strips, chunkTiles;
+    const int* slotsUsed;
     int partShift;  // log2 of the items a tile's columns are split over
     // FP32 sweep: event of row r of thread t of a full strip, at
     // [stripBase + r * 128 + t] (launch_strip_order for the sweep's R), or

@@ -666,6 +666,7 @@ sweep_f64_list_kernel(const SweepProblem* problems, const WorkItem* items, const
     for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
          first = false) {
         const SweepProblem& P = problems[w.problem];
+        if (SELF && P.slotsUsed && w.slot >= P.slotsUsed[w.strip]) continue;
         const PairConsts c = P.c;
         const int shift[3] = {P.colShift[0], P.colShift[1], P.colShift[2]};
         f64_item<D, R, SELF, SHORT>(static_cast<const double*>(P.rec), P.tileMin, P.tileMax, P.partials, P.N,
@@ -1319,6 +1320,7 @@ sweep_f32c_list_kernel(const SweepProblem* problems, const WorkItem* items, cons
     for (bool first = true; next_item<SELF, R>(problems, items, n, counter, first, w);
          first = false) {
         const SweepProblem& P = problems[w.problem];
+        if (SELF && P.slotsUsed && w.slot >= P.slotsUsed[w.strip]) continue;
         const PairConsts c = P.c;
         f32c_item<D, R, V, SELF>(static_cast<const float*>(P.rec), P.tileMin, P.tileMax, P.partials,
                            P.colAcc, P.N, P.nTiles, P.Npad, P.symmetric != 0, c, w, P.rowOrder, sTile, sCol);
