@@ -451,6 +451,7 @@ ConstsSpec Executor::consts_spec(const SetView& set, double omega) const {
     ConstsSpec s = consts_spec();
     if (!selfWindow || fixedR || fixedItems || shardWorld > 1 || !set.haveBox) return s;
     const int nTiles = (set.N + kTile - 1) / kTile;
+    if (nTiles < 4) return s;  // a window leaves out whole tiles
     double volume = set.sorted ? set.hTileMax[nTiles - 1] - set.hTileMin[0]
                                : *std::max_element(set.hTileMax, set.hTileMax + nTiles) -
                                      *std::min_element(set.hTileMin, set.hTileMin + nTiles);
@@ -569,6 +570,13 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
                          int P) {
     gridOf_.clear();
     if (!gridSums || keptB || fixedR || fixedItems || shardWorld > 1 || D_ > 2) return;
+    const auto large = [&](int p) {
+        const int N = sets[setOf[p]].N;
+        return N >= kGridMinEvents && N < (1 << 28) && sets[setOf[p]].haveBox;
+    };
+    int first = 0;
+    while (first < P && !large(first)) ++first;
+    if (first == P) return;
     const bool fp32 = precision_ != HPHC_PRECISION_FP64;
     std::vector<char> of(P, 0);
     std::vector<GridShape> shapes(P);
@@ -577,10 +585,10 @@ void Executor::plan_grid(const std::vector<SetView>& sets, const int* setOf, con
     bool any = false;
     CrowdSample sample;
     int sampled = -1;  // its set
-    for (int p = 0; p < P; ++p) {
+    for (int p = first; p < P; ++p) {
+        if (!large(p)) continue;
         const SetView& s = sets[setOf[p]];
         const double* prm = params + (size_t)6 * p;
-        if (!s.haveBox || s.N < kGridMinEvents || s.N >= (1 << 28)) continue;
         const PairConsts c = pair_consts(prm, s);
         const int nTiles = (s.N + kTile - 1) / kTile;
         // pairs the sweep would evaluate (each once)
