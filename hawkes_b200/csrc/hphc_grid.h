@@ -51,11 +51,16 @@ struct GridOrder<12> {
     static constexpr int kInv = 6, kTaps = 32;
 };
 
-// The FP32-compensated mode takes order 12 below this size, where the order's
-// smaller cost shows most in batches of evaluations, and order 16 with FP64
-// self-excitation sums from it on (Executor::enqueue).  A step in sigma or omega,
-// which keeps the background and stays FP32-compensated, then costs below a
-// quarter of a full evaluation, as samplers expect of it.
+// From this size on the FP32-compensated mode takes order 16 with FP64 self-excitation
+// sums (Executor::plan) in place of order 12 with its own, which makes an evaluation as
+// exact as the FP64 mode's for 14 to 17 % of its time: N = 66k 448 -> 524 us, N = 100k 627
+// -> 715, errors of the log-likelihood 4.3e-11 -> below 1e-16 and of the worst gradient
+// component 2.2e-9 -> 5e-16.  Neither cost nor error has an edge there: the line is a
+// choice.  Batches of proposals, where the cost shows most, lie below it, and above it
+// a step in sigma or omega, which keeps the background and stays FP32-compensated (165
+// us at N = 100k), stays below a quarter of a full evaluation, as samplers expect.  A
+// step and a full evaluation of the same parameters differ by the mode's error (4e-11
+// of the log-likelihood).
 constexpr int kGridHighOrderEvents = 1 << 16;
 
 constexpr int kGridBin = 8;   // cells per bin and coordinate

@@ -113,8 +113,8 @@ __device__ __forceinline__ TileMode tile_mode(double tminI, double tmaxI, double
 //     1.93 units, 0.55 in the mean square, and the coefficients are rounded once more
 //     than in natural units; 9 operations.
 //
-// Against exp() at N = 100k with the second form: full sweep 9.63 -> 8.16 ms,
-// self-excitation sweep 1.87 -> 1.37 ms.
+// Against exp() at N = 100k: full pair sweep 9.63 -> 9.14 ms (8.16 with the second form),
+// self-excitation sweep without a window 1.87 -> 1.66 ms (1.37).
 constexpr double kE1 = 0x1.62e42fefa39e4p-6;
 constexpr double kE2 = 0x1.ebfbdff80fb49p-13;
 constexpr double kE3 = 0x1.c6b08d722f8fbp-20;

@@ -60,3 +60,24 @@ def test_more_problems_than_the_workspace_holds():
         want = _single(loc, t, P[k], FP64)
         assert abs(ll[k] - want[0]) <= 1e-13 * abs(want[0])
         np.testing.assert_allclose(g[k], want[1], rtol=1e-10)
+
+
+@pytest.mark.parametrize("n", [65536, 90000])
+def test_steps_agree_with_full_evaluations_of_another_precision(n):
+    # A large FP32-compensated evaluation has FP64 sums, a step in sigma or omega after it
+    # the mode's own: 2e-9 of the log-likelihood and 2e-8 of a gradient component's scale
+    # (some ten times the component at most here), the mode's error.
+    loc, t = workloads.uniform(n, 70)
+    p = np.asarray(workloads.BASE_PARAMS)
+    q = p * np.array([1.1, 1, 1, 0.9, 1, 1])
+    with hb.CudaHawkes(2, n, FP32C, 0) as e:
+        e.setTimesData(t)
+        e.updateLocations(-1, loc)
+        e.setParameters(p)
+        e.getLogLikelihoodAndGradient()
+        e.setParameters(q)
+        step = e.getLogLikelihoodAndGradient()
+        assert e.lastEvaluationPath == hb.PATH_SELF_EXCITATION
+    full = _single(loc, t, q, FP32C)
+    assert abs(step[0] - full[0]) <= 2e-9 * abs(full[0])
+    np.testing.assert_allclose(step[1], full[1], rtol=2e-7)
