@@ -41,6 +41,7 @@ import statistics
 import subprocess
 import sys
 import tempfile
+import threading
 import time
 
 import numpy as np
@@ -116,17 +117,52 @@ def measured_peaks():
 
 # ----------------------------------------------------------- clock sampling --
 
+def nvml_reader(device):
+    """A function returning (SM clock, its maximum, active slowdown reasons) of a CUDA
+    device, read through NVML, or None where that is not to be had."""
+    try:
+        import pynvml
+        import torch
+        pynvml.nvmlInit()
+        uuid = str(torch.cuda.get_device_properties(device).uuid)
+        h = pynvml.nvmlDeviceGetHandleByUUID(uuid if uuid.startswith("GPU-") else "GPU-" + uuid)
+        top = pynvml.nvmlDeviceGetMaxClockInfo(h, pynvml.NVML_CLOCK_SM)
+    except Exception:  # no NVML: nvidia-smi's samples are left
+        return None
+
+    def read():
+        mask = pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(h)
+        return (pynvml.nvmlDeviceGetClockInfo(h, pynvml.NVML_CLOCK_SM), top,
+                [name for name, bit in ClockSampler.REASONS.items() if mask & bit])
+    return read
+
+
 class ClockSampler:
-    """nvidia-smi samples (200 ms) while the timed region runs."""
+    """Clocks and slowdown reasons while the timed region runs: by a thread through NVML
+    every 2 ms (a region of 20 headline steps lasts 14 ms), and by nvidia-smi every
+    200 ms, which counts where NVML is missing."""
 
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,utilization.gpu,"
               "clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
               "clocks_event_reasons.hw_thermal_slowdown,"
               "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
+    REASONS = {"hw_slowdown": 0x8, "hw_thermal_slowdown": 0x40, "sw_thermal_slowdown": 0x20,
+               "sw_power_cap": 0x4}
 
-    def __init__(self):
+    def __init__(self, read=None):
         self.proc = None
         self.tmp = tempfile.NamedTemporaryFile(mode="w+", suffix=".csv", delete=False)
+        self.read, self.samples = read, []
+        self.stop = threading.Event()
+        self.thread = None
+
+    def _poll(self):
+        while not self.stop.is_set():
+            try:
+                self.samples.append(self.read())
+            except Exception:  # a sample that fails is left out
+                pass
+            self.stop.wait(0.002)
 
     def __enter__(self):
         try:
@@ -136,9 +172,15 @@ class ClockSampler:
         except OSError:
             self.proc = None
         time.sleep(0.3)
+        if self.read:
+            self.thread = threading.Thread(target=self._poll, daemon=True)
+            self.thread.start()
         return self
 
     def __exit__(self, *exc):
+        self.stop.set()
+        if self.thread:
+            self.thread.join()
         if self.proc:
             time.sleep(0.3)
             self.proc.terminate()
@@ -152,6 +194,11 @@ class ClockSampler:
         self.tmp.seek(0)
         rows = [r for r in csv.reader(io.StringIO(self.tmp.read())) if len(r) >= 10]
         os.unlink(self.tmp.name)
+        if self.samples:
+            return {"sm_mhz": statistics.median(c for c, _, _ in self.samples),
+                    "sm_max_mhz": max(m for _, m, _ in self.samples),
+                    "reasons": sorted({r for _, _, rs in self.samples for r in rs}),
+                    "samples": len(self.samples)}
         sm, smax, reasons = [], [], set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
         for r in rows:
@@ -564,7 +611,7 @@ def ours_arm(args):
                                        flusher(fp64))
     barrier()
     # FP32-compensated path (the headline), clocks sampled while it runs
-    with ClockSampler() as clocks:
+    with ClockSampler(nvml_reader(torch.cuda.current_device())) as clocks:
         barrier()
         ms32, sweep32, res32 = time_device(fp32, args.steps, args.warmup, flusher(fp32))
         barrier()
@@ -767,7 +814,7 @@ def shard_arm(args):
     res = eng.getLogLikelihoodAndGradient()
     launches = n_sweep + 1 + eng.lastLaunchStats()[0]
     step_ms, sweep_ms = [], []
-    with ClockSampler() as clocks:
+    with ClockSampler(nvml_reader(torch.cuda.current_device())) as clocks:
         barrier()
         for _ in range(args.steps):
             with torch.cuda.stream(ext):
@@ -861,7 +908,7 @@ def sampler_arm(args):
     its = max(3, args.steps // 10)
     init = np.tile(base, (K, 1))
     arms = {}
-    with ClockSampler() as clocks:
+    with ClockSampler(nvml_reader(torch.cuda.current_device())) as clocks:
         for name, flags, device in (("host", hb.CUDA | hb.COMPENSATED, False),
                                     ("device", hb.CUDA | hb.COMPENSATED, True),
                                     ("host_no_reuse",
