@@ -2,7 +2,8 @@
 // parameter vector) with one launch per stage.
 //
 //   stage   what                                          launch
-//   H2D     problem tables, work items, finish tables    one cudaMemcpyAsync from pinned staging
+//   H2D     problem tables, work items, finish tables    from pinned staging: copy_tables_kernel,
+//                                                         above 64 KB one cudaMemcpyAsync
 //   pack    FP32 records scaled per problem (FP32 mode;   pack_f32_jobs_kernel, grid (N, jobs)
 //           one copy per distinct set, tauX, tauT)
 //   grid    background sums of gridded problems           launch_grid_sums (not in the graph)
@@ -10,8 +11,9 @@
 //   finish  per-event contributions, per-CTA sums, and    finish_list_kernel
 //           per-problem totals to pinned host memory
 //
-// The sequence is captured once into a CUDA graph and replayed while buffer
-// capacities and the sweep shape stay the same; only the staged tables change
+// The sequence of each kind of plan is captured into a CUDA graph (a step on kept sums
+// when its layout comes a second time) and replayed while buffer capacities, the
+// sweep shape and the tables' layout stay the same; only the staged tables change
 // between runs.  Work items cover each strip's band of tiles that can hold a
 // non-zero term (found on the host from per-tile time bounds with the same
 // test the kernel applies), split into equal chunks and listed largest first.

@@ -173,11 +173,14 @@ constexpr double kNegligibleLog2F32 = 60.0;
 // in advance, as B_ii does for the background, so the bound is checked
 // afterwards: the sweep leaves out tile pairs more than x / omega apart, and
 // the finish compares each event's sum with what they could hold, at most
-// M e^-x (M x e^-x for the sum weighted by omega dt), M = selfCount.  If that is
-// not below 2^-60 (FP64) or 2^-36 (FP32-compensated) of the event's own sum, the
+// M e^-x (M x e^-x for the sum weighted by omega dt), M = selfCount.  If M x e^-x is
+// not below 2^-60 (FP64) or 2^-36 (FP32-compensated) of the event's own sum s, the
 // finish adds the event's terms of those tile pairs one by one, up to the
-// underflow distance.  Every sum thus holds all its terms to 2^-60 or 2^-36
-// of itself, below the rounding of the mode.
+// underflow distance.  So s lacks less than 2^-60 or 2^-36 of itself, the sum weighted by
+// dt less than that of s / omega, and the one weighted by d^2 (d^2 exp(-sigma^2 d^2 / 2)
+// <= 2 / (e sigma^2)) less than that of s / sigma^2: what they are added to in the
+// gradient.  Of a weighted sum that is itself far below these (neighbours at one
+// place, or at nearly one time) it may be a larger part.
 //
 // x = ln M + ln x + 60 ln 2 + E, where E is the exponent of an event's closest
 // earlier neighbour that all but about exp(-kSelfMisses) of the events stay
@@ -211,8 +214,11 @@ inline double times_32_log2e(double x, double y) {
 // The parameter-dependent constants of one problem: every PairConsts field
 // and every FinishConsts field except T and constant (which depend on the
 // event set only).  Written for host and device alike with products for the
-// integer powers and the correctly rounded sqrt as the only library call, so
-// both give the same bits (the device-resident sampler rewrites them there).
+// integer powers and the correctly rounded sqrt, so both give the same bits (the
+// device-resident sampler rewrites them there), but for the self-excitation window:
+// its x comes from pow, log and exp, whose last bits may differ, and the device
+// loop's ConstsSpec bounds the events for any omega.  The two may leave out other
+// tile pairs, within the window's bound on every sum.
 #ifdef __CUDACC__
 __host__ __device__
 #endif

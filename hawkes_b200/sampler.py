@@ -104,7 +104,8 @@ class Sampler:
         evaluator: a :class:`CudaHawkes` engine (its batched entry point
         evaluates the K proposals in one run) or a callable mapping a K x 6
         array of parameter vectors to K log-likelihoods.  device=True (engine
-        only) runs every iteration on the GPU from one captured CUDA graph."""
+        only) runs every iteration on the GPU with its kernels queued one behind the
+        other."""
         M = int(iterations) - int(burnIn)
         samples = np.zeros((self.numChains, max(M, 0), 6))
         targets = np.zeros((self.numChains, max(M, 0)))
@@ -168,7 +169,7 @@ def sampler(n_iter: int, burnIn: int = 0, locations=None, times=None, radius: fl
     ``createEngine``; ``single`` selects the FP32-compensated mode; ``chains``
     runs that many independent chains from ``params`` (each with its own
     random stream), their proposals evaluated together; ``on_device`` runs the
-    iterations as one replayed CUDA graph (tauX and tauT stay fixed, as in the
+    iterations on the device without the host (tauX and tauT stay fixed, as in the
     reference's sampler)."""
     if locations is None:
         raise HawkesError(3, "No locations found.")
