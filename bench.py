@@ -749,8 +749,10 @@ def ours_arm(args):
         "clocks": clock_summary,
     }
     if gridded:
-        # the engines agree to the bit where both sweep these terms in FP64
-        self64 = np.array_equal(ll32, ll64) and np.array_equal(g32, g64)
+        # where both engines sweep these terms in FP64 they agree to FP64 rounding; FP32-
+        # compensated sums differ by 1e-11 and more in some component
+        self64 = bool(np.all(np.abs(ll32 - ll64) <= 1e-13 * np.abs(ll64)) and
+                      np.all(np.abs(g32 - g64) <= 1e-12 * np.abs(g64)))
         work = (grid_instructions(w["loc"], w["t"], w["params"]) +
                 (FP64_PER_S * ns if self64 else 0.0))
         peak64 = sm_count * FP64_LANES_PER_SM * max_mhz * 1e6 / 1e12
