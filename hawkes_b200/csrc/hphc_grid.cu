@@ -269,8 +269,8 @@ weights_kernel(const __grid_constant__ Batch b, const __grid_constant__ Blocks b
 // stored weights start at a bin's first node, so every slice is a whole aligned
 // 64 bytes), and their tiles are added in warp order.  Events are sorted by t cell
 // inside their bin, so rows that none of the four touches are left out.
-// N = 100k (order 16): 190 us, the tensor pipe busy half of it (90 us of
-// instructions).  Warps that share staged groups, two or four t rows each, took
+// N = 100k (order 16): 190 us, the tensor pipe active 34 % of them; the copies and row
+// reductions of each group lie between.  Warps that share staged groups, two or four t rows each, took
 // 245 and 226 us: the barriers cost more than the sum over the warps' tiles.
 
 constexpr int kSpreadThreads = 128;
@@ -569,7 +569,8 @@ conv_row_kernel(const __grid_constant__ Batch b, const __grid_constant__ Blocks 
 // its share of the P t planes, for the spline and for its second derivative, and
 // the other two coordinates follow on the lane's own sums.  The odd pitch puts the
 // rows of a half warp on distinct banks.  Bound: shared memory, P^3 doubles an event
-// at 16 a clock (N = 100k order 16: 88 us of 174; 270 with the region and the weights
+// at 16 a clock (N = 100k order 16: 37.3e6
+// wavefronts, 128 of 175 us, the pipe 78 % busy; 270 with the region and the weights
 // loaded in step, 200 with the region asynchronous, 174 with the weights too and
 // persistent CTAs).
 
